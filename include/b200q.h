@@ -342,6 +342,18 @@ int b200q_rope_attention(const float *q, const float *k, const float *v, int64_t
                          int table_rows, int batch, int heads, int kv_heads, int head_dim, int horizon, void *k_cache,
                          void *v_cache, int cache_dtype, float scale, void *out, int out_dtype, void *stream);
 
+/* RoPE of a prompt's queries and keys (positions 0..t-1), KV-cache store and causal attention: q [batch * t, heads *
+ * head_dim], k / v [batch * t, kv_heads * head_dim] FP32 rows with their own strides (16-byte aligned), caches
+ * [batch, kv_heads, horizon, head_dim], out [batch * t, heads * head_dim]. FP32 queries and probabilities against the
+ * keys and values as the cache holds them, FP32 softmax and sums (mini_llm/ops/attention_inference.py:255-277).
+ * _supported: head_dim 64, BF16 caches and output, horizon <= 1024 (else return code 3). */
+int b200q_prefill_attention_supported(int heads, int kv_heads, int head_dim, int t, int horizon, int cache_dtype,
+                                      int out_dtype);
+int b200q_prefill_attention(const float *q, const float *k, const float *v, int64_t q_row_stride, int64_t k_row_stride,
+                            int64_t v_row_stride, const float *cos_table, const float *sin_table, int table_rows, int batch,
+                            int t, int heads, int kv_heads, int head_dim, int horizon, void *k_cache, void *v_cache,
+                            int cache_dtype, float scale, void *out, int out_dtype, void *stream);
+
 /* ---- Expert-parallel execution over the GPUs of one node (no counterpart in the reference, which is
  * single-process; semantics = the single-GPU layer, bit for bit). ------------------------------- */
 

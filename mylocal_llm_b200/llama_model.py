@@ -337,9 +337,31 @@ class ExternalLlamaModel:
         _, logits = self._norm_linear(self.final_norm, residual, pending, self.lm_head, torch.float32)
         return logits
 
+    def _prefill_kernel_fits(self, t, horizon):
+        """Whether a prompt of ``t`` tokens from position 0 on runs RoPE, cache store and causal attention as
+        ``b200q_prefill_attention`` (BF16 caches, head_dim 64, horizon up to 1024); else the torch ops do."""
+        cfg = self.config
+        dt = _lib.DTYPE_ID[str(self.dtype).replace("torch.", "")]
+        return t > 1 and bool(_lib.load().b200q_prefill_attention_supported(
+            cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, t, horizon, dt, dt))
+
+    def _prefill_attention(self, q2, k2, v2, b, t, state, layer_index):
+        torch = _torch()
+        cfg = self.config
+        heads, kv_heads, dh = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
+        ptr = lambda x: ctypes.c_void_p(x.data_ptr())
+        dt = _lib.DTYPE_ID[str(self.dtype).replace("torch.", "")]
+        ctx = torch.empty((b * t, heads * dh), dtype=self.dtype, device=q2.device)
+        _lib.call("b200q_prefill_attention", ptr(q2), ptr(k2), ptr(v2), q2.stride(0), k2.stride(0), v2.stride(0),
+                  ptr(self._cos), ptr(self._sin), int(self._cos.shape[0]), b, t, heads, kv_heads, dh, state.horizon,
+                  ptr(state.k[layer_index]), ptr(state.v[layer_index]), dt, float(dh ** -0.5), ptr(ctx), dt,
+                  _lib.current_stream())
+        return ctx
+
     def _forward(self, token_ids, state, positions, mask):
-        """token_ids [B, T]; positions [T] device int64; mask [T, horizon] additive FP32. Returns the
-        final normalised hidden states [B*T, d] in the model dtype."""
+        """token_ids [B, T]; positions [T] device int64; mask [T, horizon] additive FP32, or None for a prompt that
+        starts at position 0 and runs on the prompt-attention kernel. Returns the final normalised hidden states
+        [B*T, d] in the model dtype."""
         torch = _torch()
         cfg = self.config
         b, t = token_ids.shape
@@ -362,6 +384,11 @@ class ExternalLlamaModel:
                 ctx = torch.empty((b, heads * dh), dtype=self.dtype, device=hidden.device)
                 self._rope_attention(q2, k2, v2, positions, state, i, ctx)
                 attn = quantized_linear(ctx, layer["o"])
+                residual, hidden = layer["norm2"].forward_residual_add(residual, attn)
+                hidden, residual = self._ffn(i, layer, hidden, residual)
+                continue
+            if mask is None:
+                attn = self._linear(self._prefill_attention(q2, k2, v2, b, t, state, i), layer["o"])
                 residual, hidden = layer["norm2"].forward_residual_add(residual, attn)
                 hidden, residual = self._ffn(i, layer, hidden, residual)
                 continue
@@ -406,9 +433,11 @@ class ExternalLlamaModel:
         b, t = token_ids.shape
         if b != state.batch or t > state.horizon:
             raise ValueError("prompt does not fit the generation state")
-        positions = torch.arange(t, device=self.device)
-        cols = torch.arange(state.horizon, device=self.device)
-        mask = torch.where(cols[None, :] <= positions[:, None], 0.0, float("-inf")).float()
+        positions = mask = None
+        if not self._prefill_kernel_fits(t, state.horizon):
+            positions = torch.arange(t, device=self.device)
+            cols = torch.arange(state.horizon, device=self.device)
+            mask = torch.where(cols[None, :] <= positions[:, None], 0.0, float("-inf")).float()
         hidden = self._forward(token_ids, state, positions, mask).reshape(b, t, -1)
         state.position.fill_(t)
         state.length = t
