@@ -348,6 +348,33 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const float *gu, int m, i
     }
 }
 
+// The same for rows of whole aligned quads: four columns per thread (two 16-byte loads, one store), rows along grid.y,
+// no division per element. [8192 x 2 * 8192]: 277 us with one element per thread, 0.67 GB moved.
+template <int DT>
+__global__ void __launch_bounds__(256) silu_mul_quad_kernel(const float *gu, int m, int f, void *out) {
+    chain_trigger();
+    chain_wait();
+    const int col = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (col >= f) return;
+    for (int row = blockIdx.y; row < m; row += gridDim.y) {
+        const float *gp = gu + static_cast<size_t>(row) * 2 * f + col;
+        const float4 g = *reinterpret_cast<const float4 *>(gp), u = *reinterpret_cast<const float4 *>(gp + f);
+        const size_t o = static_cast<size_t>(row) * f + col;
+        const float r0 = swiglu_f32(g.x, u.x), r1 = swiglu_f32(g.y, u.y), r2 = swiglu_f32(g.z, u.z), r3 = swiglu_f32(g.w, u.w);
+        if (DT == B200Q_F32) {
+            *reinterpret_cast<float4 *>(static_cast<float *>(out) + o) = make_float4(r0, r1, r2, r3);
+        } else if (DT == B200Q_BF16) {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(r0, r1), b = __floats2bfloat162_rn(r2, r3);
+            *reinterpret_cast<uint2 *>(static_cast<__nv_bfloat16 *>(out) + o) =
+                make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        } else {
+            const __half2 a = __floats2half2_rn(r0, r1), b = __floats2half2_rn(r2, r3);
+            *reinterpret_cast<uint2 *>(static_cast<__half *>(out) + o) =
+                make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        }
+    }
+}
+
 constexpr int ATT_SPLIT = 4;
 
 // B200Q_ATTENTION_SPLIT=0 keeps one CTA per (batch, head) (A/B measurements).
@@ -418,6 +445,13 @@ int b200q_rope_kv_store(float *q, const float *k, const float *v, int64_t q_row_
 int b200q_silu_mul(const float *gate_up, int m, int f, void *out, int out_dtype, void *stream) {
     if (!gate_up || !out) return fail(B200Q_EINVAL, "silu_mul: NULL pointer");
     if (m <= 0 || f <= 0 || !dtype_valid(out_dtype)) return fail(B200Q_EINVAL, "silu_mul: bad argument");
+    if (f % 4 == 0 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+        auto kernel = out_dtype == B200Q_F32 ? silu_mul_quad_kernel<B200Q_F32>
+                    : out_dtype == B200Q_BF16 ? silu_mul_quad_kernel<B200Q_BF16> : silu_mul_quad_kernel<B200Q_F16>;
+        launch_chained(kernel, dim3((f / 4 + 255) / 256, std::min(m, 65535)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                       gate_up, m, f, out);
+        return check_launch("silu_mul");
+    }
     const long long total = static_cast<long long>(m) * f;
     const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 4096));
     launch_chained(silu_mul_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream), gate_up, m, f, out,
