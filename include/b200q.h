@@ -69,6 +69,11 @@ int b200q_device_status_clear(void);
  * (mini_llm/ops/quantized_weight.py:166-250) as a device kernel; bit-exact with it. */
 int b200q_dequantize(const void *w, int fmt, int64_t n, int k, float *out, void *stream);
 
+/* out[i, k] (fp32) = dequantised row ids[i] of W [n, k] (GGUF layouts): a gather of rows and b200q_dequantize of them
+ * as one launch (the token embedding of a packed model). An id outside [0, n) gives zeros and stores 302 in the device
+ * status word. */
+int b200q_embed_rows(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, void *stream);
+
 /* y[m,n] = x[m,k] @ W[n,k]^T, FP32 accumulation; W is read once for up to 8 tokens.
  * Replaces quantized_linear's device branch and its Triton kernel
  * (mini_llm/ops/quantized_linear.py:174-192,272-335) and has the argument order of the

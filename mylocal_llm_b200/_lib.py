@@ -79,6 +79,7 @@ SIGNATURES = {
     "b200q_gemv_silu": [_ptr, _c_int, _c_int, _c_int, _ptr, _c_int, _c_int, _ptr, _c_int, _ptr],
     "b200q_rope_attention": [_ptr, _ptr, _ptr, _c_i64, _c_i64, _c_i64, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int,
                              _c_int, _c_int, _ptr, _ptr, _c_int, _c_f32, _ptr, _c_int, _ptr],
+    "b200q_embed_rows": [_ptr, _c_int, _c_i64, _c_int, _ptr, _c_int, _ptr, _ptr],
     "b200q_prefill_attention_supported": [_c_int] * 7,
     "b200q_prefill_attention": [_ptr, _ptr, _ptr, _c_i64, _c_i64, _c_i64, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
                                 _c_int, _c_int, _ptr, _ptr, _c_int, _c_f32, _ptr, _c_int, _ptr],
@@ -144,6 +145,38 @@ def call(name, *args):
     if rc == 3:
         raise NotImplementedError(message)
     raise B200QError(message)
+
+
+_CALL = call
+_HOST = None
+
+
+def host():
+    """The native host path (``_b200q_host.so``: launch sequences of the operators in C++), or ``None`` while every
+    entry point has to pass through ``call`` - somebody has replaced it to see the calls - or with ``B200Q_HOST=0``."""
+    if call is not _CALL or os.environ.get("B200Q_HOST", "1") == "0":
+        return None
+    return _HOST or _load_host()
+
+
+def _load_host():
+    global _HOST
+    import importlib.util
+    lib = load()
+    with _LOCK:
+        if _HOST is None:
+            from . import build as _build
+            path = _build.HOST_LIB
+            if not path.exists():
+                _build.build_host()
+            import torch  # noqa: F401  (the extension links against its libraries)
+            spec = importlib.util.spec_from_file_location("_b200q_host", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            address = lambda fn: ctypes.cast(fn, _ptr).value
+            module.bind({name: address(getattr(lib, name)) for name in [*SIGNATURES, "b200q_last_error"]}, B200QError)
+            _HOST = module
+    return _HOST
 
 
 def current_stream():

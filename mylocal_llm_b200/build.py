@@ -18,6 +18,8 @@ CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libb200q.so"
 OBJ_DIR = CSRC / "build"
+HOST_SRC = CSRC / "host" / "host_ops.cpp"
+HOST_LIB = PKG / "_b200q_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -47,9 +49,39 @@ def needs_build():
     return any(p.stat().st_mtime > stamp for p in _sources() + _headers())
 
 
+def needs_host_build():
+    """The extension module with the native host path: its source or the C ABI header is newer."""
+    if not HOST_LIB.exists():
+        return True
+    stamp = HOST_LIB.stat().st_mtime
+    return any(p.stat().st_mtime > stamp for p in [HOST_SRC, *INCLUDE.glob("*.h")])
+
+
+def build_host(force=False):
+    """Compile ``_b200q_host.so`` (C++ only, against the installed torch); returns its path."""
+    if not force and not needs_host_build():
+        return HOST_LIB
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    tmp = HOST_LIB.with_suffix(f".{os.getpid()}.tmp.so")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", str(INCLUDE),
+           *[f"-isystem{path}" for path in [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda)]],
+           str(HOST_SRC), "-o", str(tmp), *[f"-L{path}" for path in cpp_extension.library_paths()],
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode:
+        raise RuntimeError(f"host extension build failed:\n{proc.stderr[-4000:]}")
+    os.replace(tmp, HOST_LIB)
+    return HOST_LIB
+
+
 def build(force=False, verbose=False):
-    """Compile and link the in-tree ``libb200q.so``; returns its path."""
+    """Compile and link the in-tree ``libb200q.so`` (and the host extension); returns its path."""
     if not force and not needs_build():
+        build_host(force)
         return LIB
     nvcc = _nvcc()
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
@@ -67,7 +99,9 @@ def build(force=False, verbose=False):
         return obj, proc.stderr
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        host = pool.submit(build_host, force)
         results = list(pool.map(compile_one, _sources()))
+        host.result()
     if verbose:
         for obj, log in results:
             if log:

@@ -1,4 +1,6 @@
 // Small kernels around the streaming GEMV: dequantise, RMSNorm, router, routing plan, combine.
+#include <algorithm>
+
 #include "common.cuh"
 #include "norm_device.cuh"
 
@@ -65,6 +67,23 @@ __global__ void dequantize_kernel(const uint8_t *w, int fmt, long long total, fl
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         const long long b = i / qk;
         out[i] = decode_one(w + b * qb, fmt, static_cast<int>(i - b * qk));
+    }
+}
+
+// Selected rows (token embedding): grid.y = output row, a thread per weight of the row.
+constexpr int STATUS_ROW_RANGE = 302;      // a row index lay outside the matrix
+__global__ void __launch_bounds__(256) embed_rows_kernel(const uint8_t *w, int fmt, long long n, int k, const long long *ids,
+                                                         int count, float *out, int *status) {
+    chain_trigger();
+    chain_wait();         // the ids come from the preceding kernel
+    const int qk = fmt_elems(fmt), qb = fmt_bytes(fmt);
+    const long long row_bytes = static_cast<long long>(k / qk) * qb;
+    for (int i = blockIdx.y; i < count; i += gridDim.y) {
+        const long long row = ids[i];
+        const bool ok = row >= 0 && row < n;
+        if (!ok && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(status, STATUS_ROW_RANGE);
+        for (int e = blockIdx.x * 256 + threadIdx.x; e < k; e += gridDim.x * 256)
+            out[static_cast<size_t>(i) * k + e] = ok ? decode_one(w + row * row_bytes + static_cast<long long>(e / qk) * qb, fmt, e % qk) : 0.f;
     }
 }
 
@@ -500,6 +519,18 @@ int b200q_dequantize(const void *w, int fmt, int64_t n, int k, float *out, void 
     dequantize_kernel<<<static_cast<int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint8_t *>(w), fmt, total, out);
     return check_launch("dequantize");
+}
+
+int b200q_embed_rows(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, void *stream) {
+    if (!w || !ids || !out) return fail(B200Q_EINVAL, "embed_rows: NULL pointer");
+    if (!fmt_valid(fmt)) return fail(B200Q_EINVAL, "embed_rows: unknown format %d", fmt);
+    if (n <= 0 || k <= 0 || k % fmt_elems(fmt) || count <= 0) return fail(B200Q_EINVAL, "embed_rows: bad shape");
+    int *status = device_status_word();
+    if (!status) return fail(B200Q_ECUDA, "embed_rows: no CUDA device");
+    launch_chained(embed_rows_kernel, dim3((k + 255) / 256, std::min(count, 65535)), dim3(256), 0,
+                   static_cast<cudaStream_t>(stream), static_cast<const uint8_t *>(w), fmt, static_cast<long long>(n), k,
+                   reinterpret_cast<const long long *>(ids), count, out, status);
+    return check_launch("embed_rows");
 }
 
 int b200q_rmsnorm(const void *x, int x_dtype, const void *gamma, int gamma_dtype, int rows, int d, float eps,

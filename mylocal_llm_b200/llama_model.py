@@ -87,6 +87,7 @@ class ExternalLlamaModel:
         # launch of its own; the results are the same bits)
         self.fused_norm_linear = os.environ.get("B200Q_NORM_GEMV", "1") != "0"
         self._loaded = False
+        self._host = None              # native host path of the loaded weights (False: they need the Python layers)
 
     def expected_shapes(self):
         cfg = self.config
@@ -197,6 +198,7 @@ class ExternalLlamaModel:
         ang = np.arange(cfg.max_position_embeddings)[:, None] * inv[None, :]
         self._cos = torch.as_tensor(np.cos(ang), dtype=torch.float32).to(self.device)
         self._sin = torch.as_tensor(np.sin(ang), dtype=torch.float32).to(self.device)
+        self._host = None
         self._loaded = True
 
     @property
@@ -425,6 +427,33 @@ class ExternalLlamaModel:
         residual, hidden = nxt.forward_residual_add(residual, ffn)
         return hidden, residual
 
+    def _native(self, token_ids, state):
+        """The model for the native host path (the same launches without an interpreter between them), or ``None``: some
+        layer is not stacked, or the call's tensors are not what it takes."""
+        torch = _torch()
+        host = _lib.host()
+        if (host is None or self._host is False or not self.fused_decode or token_ids.dtype != torch.int64 or not token_ids.is_cuda
+                or not token_ids.numel() or not state.k.is_contiguous() or not state.v.is_contiguous() or state.k.dtype != self.dtype
+                or state.v.dtype != self.dtype):
+            return None
+        if self._host is None:
+            cfg = self.config
+            stacked = all(layer["qkv"] is not None and layer["gate_up"] is not None for layer in self.layers)
+            fits = stacked and cfg.head_dim in (64, 128) and self.embed.quant_type in _lib.FORMAT_ID
+
+            def matrix(w):
+                native = self.native_of.get(id(w))
+                return (w.data, w._format_id, w.shape[0], w.shape[1], None if native is None else native.data,
+                        -1 if native is None else native._format_id)
+
+            self._host = False if not fits else host.Llama(dict(
+                embed=self.embed.data, embed_fmt=self.embed._format_id, final_norm=self.final_norm.gamma, lm_head=matrix(self.lm_head),
+                cos=self._cos, sin=self._sin, d=cfg.hidden_size, f=cfg.intermediate_size, heads=cfg.num_attention_heads,
+                kv_heads=cfg.num_key_value_heads, head_dim=cfg.head_dim, vocab=cfg.vocab_size, eps=cfg.rms_norm_eps,
+                layers=[(layer["norm1"].gamma, layer["norm2"].gamma, matrix(layer["qkv"]), matrix(layer["o"]),
+                         matrix(layer["gate_up"]), matrix(layer["down"])) for layer in self.layers]))
+        return self._host or None
+
     def prefill(self, token_ids, state):
         """token_ids [B, T] int64 CUDA tensor; fills the cache from position 0; returns the logits of
         the last position, FP32 [B, vocab]."""
@@ -434,6 +463,13 @@ class ExternalLlamaModel:
         if b != state.batch or t > state.horizon:
             raise ValueError("prompt does not fit the generation state")
         positions = mask = None
+        if self._prefill_kernel_fits(t, state.horizon):
+            native = self._native(token_ids, state)
+            if native is not None:
+                logits = native.prefill(token_ids.contiguous(), state.k, state.v)
+                state.position.fill_(t)
+                state.length = t
+                return logits
         if not self._prefill_kernel_fits(t, state.horizon):
             positions = torch.arange(t, device=self.device)
             cols = torch.arange(state.horizon, device=self.device)
@@ -451,6 +487,14 @@ class ExternalLlamaModel:
         torch = _torch()
         if state.length >= state.horizon:
             raise ValueError("generation state is full")
+        if (self.fused_norm_linear and os.environ.get("B200Q_SILU_GEMV", "0") != "1"
+                and os.environ.get("B200Q_ROPE_ATTENTION", "1") != "0" and token_ids.numel() == state.batch):
+            native = self._native(token_ids, state)
+            if native is not None:
+                logits = native.decode(token_ids.contiguous(), state.k, state.v, state.position)
+                state.position.add_(1)
+                state.length += 1
+                return logits
         positions = state.position.clone()
         cfg = self.config
         if (self.fused_decode and self.fused_norm_linear and cfg.head_dim in (64, 128)

@@ -133,6 +133,7 @@ class PackedMoELayer:
         # A shared expert with the routed experts' shape and formats runs through the grouped kernels
         # as expert id E (the highest id, hence added last), addressed through pointer tables.
         self._tables = None
+        self._host = (None, None)           # (what it was built from, native layer) - see native()
         # B200Q_FUSE_PLAN=0: separate top-k and plan launches for a one-row step as well
         self.fuse_row_plan = os.environ.get("B200Q_FUSE_PLAN", "1") != "0"
         if shared is not None and all(
@@ -147,12 +148,41 @@ class PackedMoELayer:
         terms = self.router.k + (1 if self._tables is not None else 0)
         return isinstance(self.executor, ResidentExpertExecutor) and terms <= moe_ops.COMBINE_NORM_MAX_K
 
+    def native(self, host):
+        """The layer for the native host path (``_b200q_host.MoeLayer``), or ``None`` when it needs the Python one: another
+        executor, a shared expert that does not fit the grouped kernels, a router without an expert-major weight."""
+        router, bank = self.router, self.bank
+        key = (router._w_expert_major, router.b_router, self.shared_gate, self._tables, self.executor, bank, self.fuse_row_plan,
+               router.normalization_floor, router.k)
+        built, layer = self._host
+        if built is not None and all(a is b for a, b in zip(built, key)):
+            return layer
+        w = router._w_expert_major
+        layer = None
+        if (type(self.executor) is ResidentExpertExecutor and self.executor.banks.get(self.layer_id) is bank and w is not None
+                and w.is_cuda and w.dtype == _torch().float32 and w.is_contiguous() and w.shape[1] % 4 == 0 and w.data_ptr() % 16 == 0
+                and (self._tables is not None or (self.shared is None and self.shared_gate is None))):
+            tables, aligned = self._tables if self._tables is not None else (None, False)
+            layer = host.MoeLayer(w, router.b_router, self.shared_gate, bank.gate, bank.up, bank.down,
+                                  [bank.gate_stride, bank.up_stride, bank.down_stride],
+                                  [_lib.FORMAT_ID[t] for t in (bank.gate_type, bank.up_type, bank.down_type)], tables, aligned,
+                                  self._tables is not None, bank.n_experts, router.k, bank.d_model, bank.d_ff,
+                                  router.normalization_floor, self.fuse_row_plan)
+        self._host = (key, layer)
+        return layer
+
     def forward(self, hidden, residual_norm=None):
         """hidden [B, T, D] -> [B, T, D] in hidden's dtype. With ``residual_norm = (norm, residual)``
         (``RMSNormInference``, FP32 residual stream shaped like ``hidden``) the layer's last kernel also
         adds the branch to the residual and normalises it, and the result is ``(new residual, normalised
         activations)``: the same bits as ``norm.forward_residual_add(residual, self.forward(hidden))``."""
         torch = _torch()
+        host = _lib.host() if residual_norm is None else None
+        if (host is not None and type(hidden) is torch.Tensor and hidden.is_cuda and hidden.ndim == 3 and hidden.is_contiguous()
+                and hidden.numel() and hidden.shape[-1] == self.bank.d_model and str(hidden.dtype)[6:] in _lib.DTYPE_ID):
+            layer = self.native(host)
+            if layer is not None:
+                return layer.forward(hidden)
         if not isinstance(hidden, torch.Tensor) or not hidden.is_cuda:
             raise TypeError("MoE layer requires a CUDA tensor")
         if hidden.ndim != 3 or hidden.shape[0] < 1 or hidden.shape[-1] != self.bank.d_model:

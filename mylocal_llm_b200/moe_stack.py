@@ -35,6 +35,7 @@ class PackedMoEStack:
         # One-token steps run as one persistent kernel over all layers when the stack qualifies
         # (``B200Q_PERSISTENT=0``: always the chain of launches; the results are the same bits).
         self.persistent_step = os.environ.get("B200Q_PERSISTENT", "1") != "0"
+        self._host = (None, None)         # (native layers it was built from, native stack)
         self._persistent = None           # (layer table, workspace, call arguments) or False once found unfit
 
     @property
@@ -105,6 +106,27 @@ class PackedMoEStack:
             return None
         return res, hidden
 
+    def _native(self, residual):
+        """The chain of the layers for the native host path, or ``None`` when a part of it needs the Python layers."""
+        torch = _torch()
+        host = _lib.host()
+        norms = [*self.norms, self.final_norm]
+        gammas = [n.gamma for n in norms]
+        if (host is None or residual.dtype != torch.float32 or not residual.is_cuda or not residual.is_contiguous()
+                or not residual.numel() or residual.shape[-1] != norms[0].d_model):
+            return None
+        layers = [layer.native(host) for layer in self.layers]
+        if (any(layer is None for layer in layers) or len({n.eps for n in norms}) != 1
+                or any(g is None or g.dtype != gammas[0].dtype or g.shape != gammas[0].shape or not g.is_contiguous() for g in gammas)
+                or gammas[0].shape != (residual.shape[-1],)):
+            return None
+        key = (*layers, *gammas)
+        built, stack = self._host
+        if built is None or len(built) != len(key) or any(a is not b for a, b in zip(built, key)):
+            stack = host.MoeStack(layers, gammas, norms[0].eps)
+            self._host = (key, stack)
+        return stack
+
     def stage_times(self):
         """Microseconds the stages of the last layer took in the latest persistent step (router, barrier, top-k +
         plan, gate/up, barrier, down, barrier, combine + norm), as seen by one CTA; needs ``B200Q_STAGE_TIMES=1``
@@ -126,6 +148,10 @@ class PackedMoEStack:
             out = self.forward_one_token(residual)
             if out is not None:
                 return out
+        if trace is None and not self.fuse_residual_norm:
+            native = self._native(residual)
+            if native is not None:
+                return native.forward(residual)
         res = residual
         hidden = self.norms[0].forward_residual(res)
         for i, layer in enumerate(self.layers):

@@ -81,6 +81,7 @@ class DevicePackedGGUFWeight:
         if shape[-1] % qk or int(self.data.numel()) != math.prod(shape) // qk * qb:
             raise ValueError("Invalid packed byte length or K block alignment")
         object.__setattr__(self, "shape", shape)
+        object.__setattr__(self, "_format_id", _lib.FORMAT_ID[self.quant_type])
 
     @property
     def nbytes(self):
@@ -207,6 +208,12 @@ def quantized_linear(x, weight, *, block_k=512, cpu_packed_backend="reference", 
     by default the output has the activation dtype, as in the reference. ``allow_gemm=False`` keeps the call on
     the GEMV kernels (exact products) whatever the number of tokens: for callers whose result must not depend on
     how a batch is split."""
+    if type(weight) is DevicePackedGGUFWeight and block_k in _BLOCK_K:
+        host = _lib.host()
+        if host is not None:
+            y = host.linear(x, weight.data, weight._format_id, weight.shape[0], weight.shape[1], out_dtype, allow_gemm)
+            if y is not None:
+                return y
     _check_activation(x)
     if x.ndim not in (2, 3):
         raise ValueError("Expected x as [M, K] or [B, T, K]")

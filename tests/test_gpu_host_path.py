@@ -1,0 +1,123 @@
+"""The native host path (``_b200q_host.so``) against the Python layers (``B200Q_HOST=0``): the same entry points in the
+same order, so every result has to be the same bits - linears on both sides of the GEMM rule, MoE layers with and
+without pointer tables and token images, a stack, a Llama prompt and its decode steps."""
+
+import numpy as np
+import pytest
+
+from mylocal_llm_b200 import (DevicePackedGGUFWeight, PackedMoELayer, _lib, packed_to_device, quantized_linear, synthetic_bank)
+from mylocal_llm_b200.llama_model import ExternalLlamaConfig, ExternalLlamaModel
+from mylocal_llm_b200.moe_stack import PackedMoEStack
+from mylocal_llm_b200.quantize import random_packed
+from mylocal_llm_b200.quantized_linear import dequantize_device, retile_weight
+
+pytestmark = pytest.mark.gpu
+
+
+def both(monkeypatch, run):
+    """(native path, Python layers); the native path must be there."""
+    assert _lib.host() is not None
+    native = run()
+    monkeypatch.setenv("B200Q_HOST", "0")
+    assert _lib.host() is None
+    python = run()
+    monkeypatch.delenv("B200Q_HOST")
+    return native, python
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 33])
+@pytest.mark.parametrize("fmt,dtype,tiled", [("Q4_K", "bfloat16", True), ("Q6_K", "bfloat16", False), ("Q8_0", "float32", True)])
+def test_linear(cuda, monkeypatch, fmt, dtype, tiled, m):
+    torch = cuda
+    w = packed_to_device(random_packed(fmt, (80, 512), seed=m, d=0.01, dmin=0.005))
+    w = retile_weight(w) if tiled else w
+    x = torch.randn((1, m, 512), device="cuda").to(getattr(torch, dtype))
+    for kwargs in ({}, {"out_dtype": torch.float32}, {"allow_gemm": False}):
+        a, b = both(monkeypatch, lambda: quantized_linear(x, w, **kwargs))
+        assert a.shape == b.shape == (1, m, 80) and a.dtype == b.dtype and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("t", [1, 5, 40])
+@pytest.mark.parametrize("shared", [True, False])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_moe_layer(cuda, monkeypatch, t, shared, dtype):
+    torch = cuda
+    types, d, f, e = ("Q4_K", "Q4_K", "Q6_K"), 512, 256, 16
+    bank = synthetic_bank(e, d, f, types, seed=3)
+    triple = tuple(packed_to_device(random_packed(q, s, seed=i, d=1 / 2048, dmin=1 / 4096))
+                   for i, (q, s) in enumerate(zip(types, ((f, d), (f, d), (d, f))))) if shared else None
+    gate = torch.randn(d, device="cuda") if shared else None
+    layer = PackedMoELayer(bank, 0.05 * torch.randn((d, e), device="cuda"), 4, shared=triple, shared_gate=gate)
+    x = torch.randn((1, t, d), device="cuda").to(getattr(torch, dtype))
+    a, b = both(monkeypatch, lambda: layer.forward(x))
+    assert a.dtype == b.dtype and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("t", [2, 33])
+def test_moe_stack(cuda, monkeypatch, t):
+    torch = cuda
+    stack = PackedMoEStack.synthetic(3, d_model=512, d_ff=256, n_experts=16, top_k=4, shared_d_ff=256, seed=5)
+    x = torch.randn((t, 1, 512), device="cuda")
+    kept = x.clone()
+    a, b = both(monkeypatch, lambda: stack.forward(x))
+    assert torch.equal(x, kept) and torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("batch", [1, 3, 17])
+def test_llama_prompt_and_steps(cuda, monkeypatch, batch):
+    torch = cuda
+    cfg = ExternalLlamaConfig(vocab_size=512, hidden_size=512, intermediate_size=768, num_hidden_layers=3, num_attention_heads=8,
+                              num_key_value_heads=2, head_dim=64, max_position_embeddings=128)
+    model = ExternalLlamaModel.synthetic(cfg, seed=batch)
+    ids = torch.randint(0, 512, (batch, 23), device="cuda")
+
+    def run():
+        state = model.create_generation_state(batch, 64)
+        out = [model.prefill(ids[:, :20].contiguous(), state)] + [model.decode_one(ids[:, 20 + i].contiguous(), state) for i in range(3)]
+        assert int(state.position) == state.length == 23
+        return out + [state.k, state.v]
+
+    for a, b in zip(*both(monkeypatch, run)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("fmt", ["Q8_0", "Q4_K", "Q6_K"])
+def test_embed_rows_is_the_gather_of_dequantised_rows(cuda, fmt):
+    torch = cuda
+    import ctypes
+    w = packed_to_device(random_packed(fmt, (37, 512), seed=1, d=0.01, dmin=0.005))
+    ids = torch.tensor([36, 0, 5, 5, 17], device="cuda")
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    out = torch.full((6, 512), float("nan"), device="cuda")
+    _lib.call("b200q_embed_rows", ptr(w.data), _lib.FORMAT_ID[fmt], 37, 512, ptr(ids), 5, ptr(out), _lib.current_stream())
+    assert torch.equal(out[:5], dequantize_device(w.data, 37, 512, fmt)[ids]) and torch.isnan(out[5]).all()
+    assert _lib.device_status() == 0
+    bad = torch.tensor([37, 3], device="cuda")
+    _lib.call("b200q_embed_rows", ptr(w.data), _lib.FORMAT_ID[fmt], 37, 512, ptr(bad), 2, ptr(out), _lib.current_stream())
+    assert _lib.device_status() == 302 and (out[0] == 0).all()          # refused by the kernel's own bounds check
+    _lib.clear_device_status()
+
+
+def test_calls_stay_visible_when_they_are_intercepted(cuda):
+    torch = cuda
+    w = packed_to_device(random_packed("Q8_0", (64, 256), seed=2, d=0.01))
+    real, calls = _lib.call, []
+    _lib.call = lambda name, *a: (calls.append(name), real(name, *a))[1]
+    try:
+        quantized_linear(torch.zeros((1, 256), device="cuda"), w)
+    finally:
+        _lib.call = real
+    assert calls == ["b200q_gemv"]
+
+
+def test_errors_are_those_of_the_python_layer(cuda):
+    torch = cuda
+    w = DevicePackedGGUFWeight(torch.zeros(64 * 34, dtype=torch.uint8, device="cuda"), (64, 32), "Q8_0")
+    with pytest.raises(ValueError, match="K does not match"):
+        quantized_linear(torch.zeros((1, 64), device="cuda"), w)
+    with pytest.raises(ValueError, match="contiguous"):
+        quantized_linear(torch.zeros((32, 2), device="cuda").t(), w)
+    with pytest.raises(TypeError):
+        quantized_linear(np.zeros((1, 32), np.float32), w)
+    with pytest.raises(TypeError, match="FP16, BF16, or FP32"):
+        quantized_linear(torch.zeros((1, 32), dtype=torch.float64, device="cuda"), w)
