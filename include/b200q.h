@@ -257,6 +257,19 @@ int b200q_moe_down(const void *down_base, int64_t down_stride, int down_fmt, con
                    const int32_t *seg_expert, const int32_t *seg_begin, const int32_t *seg_count,
                    const int32_t *num_segments, int max_segments, float *terms, void *stream);
 
+/* The same launch fed with images of the hidden activations: b200q_moe_hidden_images converts every row of hbuf [rows, f]
+ * once into the form the tile-layout kernels consume (two FP16 planes after a power-of-two scale), and every row group of
+ * an expert reads the images of its segment instead of converting them again. Same bits as b200q_moe_down; `images` holds
+ * rows * b200q_moe_hidden_image_bytes(f) bytes, 16-byte aligned (0: this f has no images); kernels that do not use images
+ * ignore the buffer. */
+int b200q_moe_hidden_image_bytes(int f);
+int b200q_moe_hidden_images(const float *hbuf, int rows, int f, void *images, void *stream);
+int b200q_moe_down_images(const void *down_base, int64_t down_stride, int down_fmt, const uint64_t *down_table,
+                          int tables_aligned16, int flat_rows, int d, int f, const float *hbuf, const void *images,
+                          const float *route, const int32_t *order, const int32_t *seg_expert, const int32_t *seg_begin,
+                          const int32_t *seg_count, const int32_t *num_segments, int max_segments, float *terms,
+                          void *stream);
+
 /* out[row, d] = sum over the row's k assignments of terms[pos], added one by one in
  * ascending expert id starting from zero (plain FP32 adds, no FMA, no tree), plus an optional
  * extra[row,d]*extra_scale[row] term added last (the shared expert). `inv` maps the flat

@@ -97,6 +97,10 @@ SIGNATURES = {
     "b200q_peer_push_rows": [_ptr, ctypes.c_size_t, _ptr, ctypes.c_size_t, _c_int, _ptr],
     "b200q_moe_down": [_ptr, _c_i64, _c_int, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr,
                        _c_int, _ptr, _ptr],
+    "b200q_moe_hidden_image_bytes": [_c_int],
+    "b200q_moe_hidden_images": [_ptr, _c_int, _c_int, _ptr, _ptr],
+    "b200q_moe_down_images": [_ptr, _c_i64, _c_int, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr,
+                              _ptr, _ptr, _c_int, _ptr, _ptr],
     "b200q_moe_combine": [_ptr, _ptr, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr],
     "b200q_moe_combine_norm": [_ptr, _ptr, _c_int, _c_int, _c_int, _ptr, _ptr, _c_int, _ptr, _c_f32, _ptr, _c_int,
                                _c_f32, _ptr, _ptr, _c_int, _ptr],

@@ -1,0 +1,284 @@
+// Grouped gate/up and down projections over token images (grouped_stream.cuh): kernels, the hidden-activation images and
+// the launches.
+#include <cstdlib>
+#include <cstring>
+
+#include "grouped_stream.cuh"
+#include "mma_host.h"
+
+namespace b200q {
+
+// Sums the K parts of a team's row group in ascending order: every warp but the first stores its eight sums, the team
+// meets, the first warp adds. Two buffers in turn: a warp stores into a buffer again only after the team's next meeting,
+// which the first warp reaches with its reads of that buffer done. Returns true in the warp that holds the total.
+template <int COUNT>
+__device__ __forceinline__ bool add_parts(float (&v)[COUNT], float *partial, int &pbuf, int kp, int team, int kpi, int warp, int lane) {
+    if (kp == 1) return true;
+    float *buf = partial + pbuf * (GS_WARPS * 32 * 8);
+    pbuf ^= 1;
+    if (kpi) {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) buf[(warp * 8 + i) * 32 + lane] = v[i];
+    }
+    named_barrier_sync(1 + team, kp * 32);
+    if (kpi) return false;
+    for (int q = 1; q < kp; ++q)
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) v[i] += buf[((warp + q) * 8 + i) * 32 + lane];
+    return true;
+}
+
+// Gate/up + SwiGLU over Q4_K / Q5_K tiles: hbuf[sorted assignment, row].
+template <bool Q5, int NTERMS>
+__global__ void __launch_bounds__(GS_THREADS, 1) grouped_gate_up_kernel(const GroupedArgs a) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    chain_trigger();
+    chain_wait();                 // plan and images come from preceding kernels
+    constexpr int TILE = direct_tile_bytes<Q5>();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int team = warp / a.kp, kpi = warp - team * a.kp;
+    float *partial = reinterpret_cast<float *>(smem + GS_CTRL_BYTES);
+    const int plane = a.nsb * 512, sums_off = NTERMS * plane, scale_off = sums_off + a.nsb * 32;
+    int pbuf = 0;
+    auto work = [&](int seg, int group, const uint8_t *buf, TileStream<TILE, true> &stream) -> bool {
+        const int begin = a.seg_begin[seg], count = min(a.seg_count[seg], 8);
+        const uint8_t *image = buf + g * a.smem_stride;
+        const uint8_t *fp = image + tig * 16 + kpi * 512, *xp = image + sums_off + tig * 4 + kpi * 32;
+        float tg[1][4] = {{0.f, 0.f, 0.f, 0.f}}, tu[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+        auto frag = [&](int, int s, int p) { return *reinterpret_cast<const uint4 *>(fp + s * 64 + p * plane); };
+        auto sums = [&](int, int term) { return *reinterpret_cast<const uint32_t *>(xp + term * 16); };
+        for (int sb = kpi; sb < a.nsb; sb += a.kp) {
+            SuperBlockRegs<Q5> r;
+            const uint8_t *tile;
+            if (!stream.next(tile)) return false;
+            read_superblock_tile<Q5>(r, tile, lane);
+            stream.refill(lane);
+            superblock_mma<Q5, NTERMS, 1>(r, frag, sums, tig, tg);
+            if (!stream.next(tile)) return false;
+            read_superblock_tile<Q5>(r, tile, lane);
+            stream.refill(lane);
+            superblock_mma<Q5, NTERMS, 1>(r, frag, sums, tig, tu);
+            fp += a.kp * 512;
+            xp += a.kp * 32;
+        }
+        float v[8] = {tg[0][0], tg[0][1], tg[0][2], tg[0][3], tu[0][0], tu[0][1], tu[0][2], tu[0][3]};
+        if (!add_parts(v, partial, pbuf, a.kp, team, kpi, warp, lane)) return true;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int t = 2 * tig + e;
+            if (t < count) {
+                const float inv = *reinterpret_cast<const float *>(buf + t * a.smem_stride + scale_off + 4);
+                float *dst = a.y + static_cast<size_t>(begin + t) * a.n + group * 16 + g;
+                dst[0] = swiglu_f32(v[e] * inv, v[4 + e] * inv);
+                dst[8] = swiglu_f32(v[2 + e] * inv, v[6 + e] * inv);
+            }
+        }
+        return true;
+    };
+    grouped_walk<false, TILE, true>(a, smem, work);
+}
+
+// Down projection over Q6_K / Q8_0 tiles of FP32 hidden activations (two FP16 planes), times the route weight.
+template <typename T>
+__global__ void __launch_bounds__(GS_THREADS, 1) grouped_down_kernel(const GroupedArgs a) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    chain_trigger();
+    chain_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int team = warp / a.kp, kpi = warp - team * a.kp;
+    float *partial = reinterpret_cast<float *>(smem + GS_CTRL_BYTES);
+    const int plane = a.nsb * 512, scale_off = 2 * plane;
+    int pbuf = 0;
+    auto work = [&](int seg, int group, const uint8_t *buf, TileStream<T::BYTES, false> &stream) -> bool {
+        const int begin = a.seg_begin[seg], count = min(a.seg_count[seg], 8);
+        // the lane's two tokens: route weight and output row (used at the end)
+        float route[2] = {0.f, 0.f};
+        float *out[2] = {nullptr, nullptr};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int t = 2 * tig + e;
+            if (t < count) {
+                const int flat = a.order[begin + t];
+                route[e] = a.route[flat];
+                out[e] = term_row_pointer(a.y, a.y_table, a.rows_per_rank, a.n, a.flat_rows ? flat : begin + t);
+            }
+        }
+        const uint8_t *fp = buf + g * a.smem_stride + tig * 16 + kpi * 512;
+        float tot[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+        auto frag = [&](int, int pair, int p) { return fp + pair * 64 + p * plane; };
+        for (int sb = kpi; sb < a.nsb; sb += a.kp) {
+            typename T::Regs r;
+            const uint8_t *tile;
+            if (!stream.next(tile)) return false;
+            T::read(r, tile, lane);
+            stream.refill(lane);
+            T::template mma<2, 1>(r, frag, tot);
+            fp += a.kp * 512;
+        }
+        if (!add_parts(tot[0], partial, pbuf, a.kp, team, kpi, warp, lane)) return true;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int t = 2 * tig + e;
+            if (t < count) {
+                const float inv = *reinterpret_cast<const float *>(buf + t * a.smem_stride + scale_off + 4);
+                float *dst = out[e] + group * 16 + g;
+                dst[0] = tot[0][e] * inv * route[e];
+                dst[8] = tot[0][2 + e] * inv * route[e];
+            }
+        }
+        return true;
+    };
+    grouped_walk<true, T::BYTES, false>(a, smem, work);
+}
+
+// Image of one row of FP32 hidden activations, a warp per row: the power-of-two scale and the two FP16 planes of
+// prepare_fragments, pairs of fragments of the four lanes of a quad side by side (64 bytes), then scale and inverse.
+__global__ void __launch_bounds__(256) hidden_image_kernel(const float *h, int rows, int k, uint8_t *images, int image_bytes) {
+    chain_trigger();
+    chain_wait();
+    const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const float *src = h + static_cast<size_t>(row) * k;
+    uint8_t *dst = images + static_cast<size_t>(row) * image_bytes;
+    constexpr int KEEP = 8;                              // chunks of four values per lane kept between the passes
+    float4 kept[KEEP];
+    float amax = 0.f;
+    const int chunks = k >> 2;
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) {
+        const int c = lane + 32 * i;
+        kept[i] = c < chunks ? *reinterpret_cast<const float4 *>(src + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    auto grow = [&](const float4 &v) {
+        // integer maxima of the magnitudes' bits: a NaN stays the largest, as in prepare_fragments
+        const uint32_t m = max(max(__float_as_uint(fabsf(v.x)), __float_as_uint(fabsf(v.y))), max(__float_as_uint(fabsf(v.z)), __float_as_uint(fabsf(v.w))));
+        amax = __uint_as_float(max(__float_as_uint(amax), m));
+    };
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) grow(kept[i]);
+    for (int c = lane + 32 * KEEP; c < chunks; c += 32) grow(*reinterpret_cast<const float4 *>(src + 4 * c));
+    amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+    float s = 1.0f;
+    if (amax > 0.f && amax < __int_as_float(0x7f800000)) {
+        int e;
+        frexpf(amax, &e);
+        s = ldexpf(1.0f, min(14 - e, 100));
+    }
+    const int plane = k * 2;
+    auto put = [&](int c, const float4 &v4) {
+        const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+        unsigned short hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float sv = v[i] * s;
+            const __half hv = __float2half_rn(sv);
+            hi[i] = __half_as_ushort(hv);
+            lo[i] = __half_as_ushort(__float2half_rn(sv - __half2float(hv)));
+        }
+        // positions 4c..: pair c >> 3, quad lane c & 3, fragment (c >> 2) & 1
+        uint8_t *at = dst + (c >> 3) * 64 + (c & 3) * 16 + ((c >> 2) & 1) * 8;
+        *reinterpret_cast<uint2 *>(at) = make_uint2(hi[0] | (static_cast<uint32_t>(hi[2]) << 16), hi[1] | (static_cast<uint32_t>(hi[3]) << 16));
+        *reinterpret_cast<uint2 *>(at + plane) = make_uint2(lo[0] | (static_cast<uint32_t>(lo[2]) << 16), lo[1] | (static_cast<uint32_t>(lo[3]) << 16));
+    };
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+        if (lane + 32 * i < chunks) put(lane + 32 * i, kept[i]);
+    for (int c = lane + 32 * KEEP; c < chunks; c += 32) put(c, *reinterpret_cast<const float4 *>(src + 4 * c));
+    if (lane == 0) *reinterpret_cast<float4 *>(dst + 2 * plane) = make_float4(s, 1.0f / s, 0.f, 0.f);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------------------------
+// Warps per 16-row group (parts of K) for a grouped launch over tile-layout weights with more than a few segments; a
+// function of the plan's bound only, so that every caller with that bound adds in the same order. A CTA deals its row
+// groups to 16 / kp teams: the last round is on average half empty, which costs 1 / (2 kp) of a round, while every
+// doubling of kp adds a meeting of the team per group (about 2 % of a group of eight super-blocks). About 65 % of the
+// bound are segments that exist (measured 62-73 % for 16 to 256 tokens over 512 experts).
+int grouped_kp(int n, int nsb, int max_segments) {
+    const double groups = 0.65 * max_segments * (n / 16) / sm_count();
+    int best = 1;
+    double cost = 1e30;
+    for (int kp = 1; kp <= 8 && kp <= nsb; kp *= 2) {
+        const double c = (groups * kp / GS_WARPS + 0.5) / kp * (1.0 + 0.16 * (kp - 1) / nsb);
+        if (c < cost) {
+            cost = c;
+            best = kp;
+        }
+    }
+    return best;
+}
+
+int hidden_image_bytes(int k) { return k > 0 && k % 256 == 0 && k <= 8192 ? k * 4 + 16 : 0; }
+
+int hidden_images(const float *h, int rows, int k, void *images, cudaStream_t stream) {
+    if (hidden_image_bytes(k) == 0 || ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(images)) & 15))
+        return fail(B200Q_EUNSUPPORTED, "hidden images: f must be a multiple of 256, buffers 16-byte aligned");
+    launch_chained(hidden_image_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, h, rows, k, static_cast<uint8_t *>(images),
+                   hidden_image_bytes(k));
+    return check_launch("hidden images");
+}
+
+// Fills the shared part of the arguments; false when two segment buffers do not fit in shared memory.
+static bool grouped_args(const MmaRequest &q, int image_bytes, int tile_bytes, GroupedArgs &a, size_t &smem) {
+    a.wa = q.wa; a.wb = q.wb; a.stride_a = q.stride_a; a.stride_b = q.stride_b;
+    a.table_a = q.table_a; a.table_b = q.table_b;
+    a.n = q.n; a.nsb = q.k / 256; a.kp = grouped_kp(q.n, a.nsb, q.max_segments);
+    a.images = static_cast<const uint8_t *>(q.images);
+    a.image_bytes = image_bytes;
+    a.smem_stride = (image_bytes + 63) / 128 * 128 + 64;
+    // two segment buffers and two tiles per warp at least; what is left goes to the tile rings first
+    a.off_ring = GS_CTRL_BYTES + (a.kp > 1 ? GS_PART_BYTES : 0);
+    const int room = MM_SMEM_LIMIT - a.off_ring, buf_bytes = 8 * a.smem_stride, ring_bytes = GS_WARPS * tile_bytes;
+    a.bufs = 2;
+    a.ring = (room - 2 * buf_bytes) / ring_bytes;
+    if (a.ring > GS_MAX_RING) a.ring = GS_MAX_RING;
+    if (room < 2 * buf_bytes || a.ring < 2) return false;
+    a.bufs = (room - a.ring * ring_bytes) / buf_bytes;
+    if (a.bufs > GS_MAX_BUFS) a.bufs = GS_MAX_BUFS;
+    a.off_bufs = a.off_ring + a.ring * ring_bytes;
+    a.topk = q.topk; a.order = q.order; a.seg_expert = q.seg_expert; a.seg_begin = q.seg_begin; a.seg_count = q.seg_count;
+    a.num_segments = q.num_segments; a.max_segments = q.max_segments; a.y = static_cast<float *>(q.y); a.route = q.route;
+    a.flat_rows = q.flat_rows; a.y_table = q.y_table; a.rows_per_rank = q.rows_per_rank;
+    a.status = device_status_word();
+    smem = a.off_bufs + static_cast<size_t>(a.bufs) * 8 * a.smem_stride;
+    return a.status != nullptr;
+}
+
+static int launch_grouped(void (*fn)(const GroupedArgs), const GroupedArgs &a, size_t smem, cudaStream_t stream, const char *what) {
+    if (cudaFuncSetAttribute(reinterpret_cast<const void *>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM_LIMIT) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(B200Q_ECUDA, "%s: shared memory opt-in failed", what);
+    }
+    launch_chained(fn, dim3(sm_count()), dim3(GS_THREADS), smem, stream, a);
+    return check_launch(what);
+}
+
+int grouped_gate_up_launch(const MmaRequest &q, cudaStream_t stream, bool *launched) {
+    *launched = false;
+    GroupedArgs a{};
+    size_t smem = 0;
+    const int image_bytes = direct_token_image_bytes(q.k, q.x_dtype);
+    if (!q.images || !q.tiled || image_bytes == 0 || (reinterpret_cast<uintptr_t>(q.images) & 15) || q.max_segments <= GROUPED_FEW_SEGMENTS)
+        return B200Q_OK;
+    if (!grouped_args(q, image_bytes, q.fmt_a == B200Q_Q5_K ? Q5T_TILE_BYTES : Q4T_TILE_BYTES, a, smem)) return B200Q_OK;
+    const bool two = q.x_dtype == B200Q_F32, q5 = q.fmt_a == B200Q_Q5_K;
+    auto fn = q5 ? (two ? grouped_gate_up_kernel<true, 2> : grouped_gate_up_kernel<true, 1>)
+                 : (two ? grouped_gate_up_kernel<false, 2> : grouped_gate_up_kernel<false, 1>);
+    *launched = true;
+    return launch_grouped(fn, a, smem, stream, "grouped gate/up");
+}
+
+int grouped_down_launch(const MmaRequest &q, cudaStream_t stream, bool *launched) {
+    *launched = false;
+    GroupedArgs a{};
+    size_t smem = 0;
+    if (!q.images || hidden_image_bytes(q.k) == 0 || (reinterpret_cast<uintptr_t>(q.images) & 15) || q.max_segments <= GROUPED_FEW_SEGMENTS)
+        return B200Q_OK;
+    if (!grouped_args(q, hidden_image_bytes(q.k), q.fmt_a == B200Q_Q8_0_TILED ? Q8T_TILE_BYTES : Q6T_TILE_BYTES, a, smem)) return B200Q_OK;
+    *launched = true;
+    return launch_grouped(q.fmt_a == B200Q_Q8_0_TILED ? grouped_down_kernel<Q8Tile> : grouped_down_kernel<Q6Tile>, a, smem, stream,
+                          "grouped down");
+}
+
+}  // namespace b200q

@@ -32,7 +32,7 @@ struct Api {
     FN(last_error); FN(gemv); FN(gemm); FN(gemm_ws); FN(gemm_workspace_bytes); FN(gemm_supported); FN(rmsnorm);
     FN(residual_rmsnorm); FN(gemv_norm); FN(gemv_norm_supported); FN(router_logits_t); FN(router_topk_ex);
     FN(router_topk_plan_row); FN(shared_gate); FN(moe_plan_ex); FN(moe_token_image_bytes); FN(moe_token_images);
-    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_combine); FN(silu_mul); FN(rope_attention);
+    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
     FN(prefill_attention); FN(embed_rows);
 #undef FN
 } api;
@@ -43,7 +43,7 @@ void bind(const py::dict &addresses, py::object error_type) {
     FN(last_error); FN(gemv); FN(gemm); FN(gemm_ws); FN(gemm_workspace_bytes); FN(gemm_supported); FN(rmsnorm);
     FN(residual_rmsnorm); FN(gemv_norm); FN(gemv_norm_supported); FN(router_logits_t); FN(router_topk_ex);
     FN(router_topk_plan_row); FN(shared_gate); FN(moe_plan_ex); FN(moe_token_image_bytes); FN(moe_token_images);
-    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_combine); FN(silu_mul); FN(rope_attention);
+    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
     FN(prefill_attention); FN(embed_rows);
 #undef FN
     b200q_error = error_type.release().ptr();
@@ -137,7 +137,7 @@ struct Carver {
 };
 
 constexpr int SEGMENT_CAP = 8;          // tokens of one expert per pass of the grouped kernels
-constexpr int TOKEN_IMAGE_MIN_ROWS = 32;
+constexpr int TOKEN_IMAGE_MIN_ROWS = 2;
 
 struct MoeLayer {
     at::Tensor router, bias, gate_vector;               // [E, D] FP32; bias / shared-expert gate may be undefined
@@ -155,15 +155,16 @@ struct MoeLayer {
         const int max_segments = std::min(plan_experts, total) + total / SEGMENT_CAP;
         const bool q45 = gate_fmt == up_fmt && (gate_fmt == B200Q_Q4_K || gate_fmt == B200Q_Q5_K ||
                                                 gate_fmt == B200Q_Q4_K_TILED || gate_fmt == B200Q_Q5_K_TILED);
-        const int image_bytes = q45 && t >= TOKEN_IMAGE_MIN_ROWS && !env_is("B200Q_TOKEN_IMAGES", "0")
-                                    ? std::max(0, api.moe_token_image_bytes(d, xdt)) : 0;
+        const bool images = t >= TOKEN_IMAGE_MIN_ROWS && !env_is("B200Q_TOKEN_IMAGES", "0");
+        const int image_bytes = q45 && images ? std::max(0, api.moe_token_image_bytes(d, xdt)) : 0;
+        const int hidden_bytes = images && (down_fmt == B200Q_Q6_K_TILED || down_fmt == B200Q_Q8_0_TILED) ? api.moe_hidden_image_bytes(f) : 0;
         Carver c;
         const size_t o_logits = c.take(sizeof(float) * t * experts), o_weights = c.take(sizeof(float) * total),
                      o_ids = c.take(sizeof(int64_t) * total), o_scale = c.take(sizeof(float) * t),
                      o_counts = c.take(4 * plan_experts), o_offsets = c.take(4 * (plan_experts + 1)), o_order = c.take(4 * total),
                      o_inv = c.take(4 * total), o_seg = c.take(12 * static_cast<size_t>(max_segments)), o_misc = c.take(8),
                      o_hbuf = c.take(sizeof(float) * total * f), o_terms = c.take(sizeof(float) * total * d),
-                     o_images = c.take(static_cast<size_t>(image_bytes) * t);
+                     o_images = c.take(static_cast<size_t>(image_bytes) * t), o_hidden = c.take(static_cast<size_t>(hidden_bytes) * total);
         const at::Tensor scratch = empty({static_cast<int64_t>(c.used)}, at::kByte, x.device());
         uint8_t *base = static_cast<uint8_t *>(scratch.data_ptr());
         auto f32 = [&](size_t o) { return reinterpret_cast<float *>(base + o); };
@@ -203,7 +204,12 @@ struct MoeLayer {
             CALL(moe_gate_up, bank(gate), gs, gate_fmt, bank(up), us, up_fmt, table(gate_table), table(up_table), aligned16, f, d,
                  x.data_ptr(), xdt, k, order, seg_expert, seg_begin, seg_count, num_segments, max_segments, hbuf, s);
         }
-        CALL(moe_down, bank(down), ds, down_fmt, table(down_table), aligned16, 0, d, f, hbuf, weights, order, seg_expert, seg_begin,
+        if (hidden_bytes) {
+            CALL(moe_hidden_images, hbuf, total, f, base + o_hidden, s);
+            CALL(moe_down_images, bank(down), ds, down_fmt, table(down_table), aligned16, 0, d, f, hbuf, base + o_hidden, weights, order,
+                 seg_expert, seg_begin, seg_count, num_segments, max_segments, terms, s);
+        } else
+            CALL(moe_down, bank(down), ds, down_fmt, table(down_table), aligned16, 0, d, f, hbuf, weights, order, seg_expert, seg_begin,
              seg_count, num_segments, max_segments, terms, s);
         CALL(moe_combine, terms, inv, t, k, d, nullptr, nullptr, out.data_ptr(), odt, s);
     }

@@ -76,6 +76,7 @@ bool direct_plan_args(const MmaRequest &q, DirectArgs *out, long long *smem_out)
         if (most(kp) > sm_count() && most(kp) <= 2LL * sm_count())
             while (kp > 1 && most(kp) > sm_count()) kp /= 2;
     }
+    if (grouped && q.max_segments > GROUPED_FEW_SEGMENTS) kp = grouped_kp(q.n, nsb, q.max_segments);
     a.kp = kp;
     a.rg = MD_WARPS / kp;
     a.off_bfrag = MD_CTRL_BYTES + token_tiles * MD_PART_BYTES;
@@ -102,6 +103,10 @@ int direct_try_launch(const MmaRequest &q, cudaStream_t stream, bool *launched) 
     DirectArgs a{};
     long long smem = 0;
     if (!direct_plan_args(q, &a, &smem)) return B200Q_OK;
+    if (q.mode == 2) {
+        const int rc = grouped_gate_up_launch(q, stream, launched);
+        if (rc || *launched) return rc;
+    }
     const bool q5 = q.fmt_a == B200Q_Q5_K;
     DirectFn fn = q5 ? (a.nterms == 2 ? pick_mode<true, 2>(q.mode, token_tiles) : pick_mode<true, 1>(q.mode, token_tiles))
                      : (a.nterms == 2 ? pick_mode<false, 2>(q.mode, token_tiles)

@@ -86,15 +86,12 @@ __device__ __forceinline__ uint4 ldg128(const uint8_t *p) {
     return v;
 }
 
-__device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
+// The first product of a chain: no accumulator to clear and read.
+__device__ __forceinline__ void mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                              uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // Packed bytes of two rows' (g, g + 8) super-block as seen by one lane. q[0..1] / q[2..3]: the code words of row g /
@@ -179,6 +176,21 @@ __device__ __forceinline__ void load_superblock_tiled(SuperBlockRegs<Q5> &r, con
     }
 }
 
+// The same from a tile in shared memory.
+template <bool Q5>
+__device__ __forceinline__ void read_superblock_tile(SuperBlockRegs<Q5> &r, const uint8_t *tile, int lane) {
+    constexpr int CODES = Q5 ? 768 : 256;
+    const int g = lane >> 2;
+    r.hd[0] = *reinterpret_cast<const uint4 *>(tile + 16 * g);
+    r.hd[1] = *reinterpret_cast<const uint4 *>(tile + 16 * (g + 8));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.q[i] = *reinterpret_cast<const uint4 *>(tile + CODES + 512 * i + lane * 16);
+    if (Q5) {
+        r.h[0] = *reinterpret_cast<const uint2 *>(tile + 256 + lane * 8);
+        r.h[1] = *reinterpret_cast<const uint2 *>(tile + 512 + lane * 8);
+    }
+}
+
 // Scales of one row: the eight 6-bit sub-block scales as FP16 subnormal pairs widened to FP32 (sc * 2^-24), the lane's
 // pair of minima as FP16 subnormals (A operand of the min product), d and dmin with the powers of two that undo both
 // subnormal forms (2^24 of the codes, 2^24 of the scales; 2^24 of the minima and the 64 of MD_XS_SCALE).
@@ -190,15 +202,17 @@ struct RowScales {
 
 __device__ __forceinline__ RowScales decode_scales(const uint4 &hd, int tig) {
     RowScales s;
-    s.d = half_bits_to_float(hd.x & 0xffffu) * 281474976710656.0f;       // 2^48
-    s.dmin = half_bits_to_float(hd.x >> 16) * 1073741824.0f;             // 2^30
+    const __half2 dd = *reinterpret_cast<const __half2 *>(&hd.x);
+    s.d = __low2float(dd) * 281474976710656.0f;       // 2^48
+    s.dmin = __high2float(dd) * 1073741824.0f;        // 2^30
     const uint32_t sc_lo = hd.y & 0x3f3f3f3fu;                                       // sub-blocks 0..3
     const uint32_t sc_hi = (hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u);        // sub-blocks 4..7
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const uint32_t pair = __byte_perm(i < 2 ? sc_lo : sc_hi, 0u, (i & 1) ? 0x4342 : 0x4140);
-        s.sc[2 * i] = half_bits_to_float(pair & 0xffffu);
-        s.sc[2 * i + 1] = half_bits_to_float(pair >> 16);
+        const __half2 h = *reinterpret_cast<const __half2 *>(&pair);
+        s.sc[2 * i] = __low2float(h);
+        s.sc[2 * i + 1] = __high2float(h);
     }
     const uint32_t mn = (tig & 2) ? ((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u) : hd.z & 0x3f3f3f3fu;
     s.mins = __byte_perm(mn, 0u, (tig & 1) ? 0x4342 : 0x4140);
@@ -419,10 +433,11 @@ __device__ __forceinline__ void gather_token_images(const uint8_t *images, int i
 // With NT token tiles (8 tokens each; their fragments `btile` / `xtile` entries apart) every decoded
 // A operand is multiplied into each tile, so the decode cost is paid once per 8*NT tokens; the
 // arithmetic of one token does not depend on NT.
-template <bool Q5, int NTERMS, int NT>
-__device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &r, const uint2 *bfrag, int btile, int nfrag,
-                                               const uint32_t *xsfrag, int xtile, int sb, int lane, float (&tot)[NT][4]) {
-    const int tig = lane & 3;
+// frag(nt, s, plane): the lane's 16 bytes of sub-block s (its two fragments) in plane 0 (FP16 high parts) or 1
+// (remainders) of token tile nt; sums(nt, term): the lane's word of the activation sums.
+template <bool Q5, int NTERMS, int NT, typename FragFn, typename SumFn>
+__device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &r, const FragFn frag, const SumFn sums, int tig,
+                                               float (&tot)[NT][4]) {
     const RowScales sa = decode_scales(r.hd[0], tig), sbk = decode_scales(r.hd[1], tig);
     // even sub-blocks (low nibbles) and odd ones (high nibbles, 16 times the code) in accumulators of their own
     float even[NT][4], odd[NT][4];
@@ -464,13 +479,12 @@ __device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &r, cons
             }
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                const uint4 *bf = reinterpret_cast<const uint4 *>(bfrag + nt * btile) + (sb * 8 + s) * 32 + lane;
-                const uint4 v = *bf;
-                mma_f16(acc, f[0][0], f[0][1], f[0][2], f[0][3], v.x, v.y);
+                float acc[4];
+                const uint4 v = frag(nt, s, 0);
+                mma_f16_first(acc, f[0][0], f[0][1], f[0][2], f[0][3], v.x, v.y);
                 mma_f16(acc, f[1][0], f[1][1], f[1][2], f[1][3], v.z, v.w);
                 if (NTERMS == 2) {
-                    const uint4 u = bf[nfrag * 16];
+                    const uint4 u = frag(nt, s, 1);
                     mma_f16(acc, f[0][0], f[0][1], f[0][2], f[0][3], u.x, u.y);
                     mma_f16(acc, f[1][0], f[1][1], f[1][2], f[1][3], u.z, u.w);
                 }
@@ -484,9 +498,9 @@ __device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &r, cons
     }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        float accm[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_f16(accm, sa.mins, sbk.mins, 0u, 0u, xsfrag[nt * xtile + (sb * 2 + 0) * 32 + lane], 0u);
-        mma_f16(accm, sa.mins, sbk.mins, 0u, 0u, xsfrag[nt * xtile + (sb * 2 + 1) * 32 + lane], 0u);
+        float accm[4];
+        mma_f16_first(accm, sa.mins, sbk.mins, 0u, 0u, sums(nt, 0), 0u);
+        mma_f16(accm, sa.mins, sbk.mins, 0u, 0u, sums(nt, 1), 0u);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float sum = fmaf(0.0625f, odd[nt][i], even[nt][i]);
@@ -671,10 +685,12 @@ __device__ __forceinline__ void mma_direct_body(const DirectArgs &a, const Stage
             if (!a.tiled) transpose_native<Q5>(cur, tig);
             const int stream = DUAL ? (item & 1) : 0;
             const int sb = kpi + (DUAL ? (item >> 1) : item) * a.kp;
-            if (stream == 0)
-                superblock_mma<Q5, NTERMS, NT>(cur, bfrag, btile, nfrag, xsfrag, xtile, sb, lane, tot_a);
-            else
-                superblock_mma<Q5, NTERMS, NT>(cur, bfrag, btile, nfrag, xsfrag, xtile, sb, lane, tot_b);
+            const uint4 *bf = reinterpret_cast<const uint4 *>(bfrag) + sb * 256 + lane;
+            const uint32_t *xf = xsfrag + sb * 64 + lane;
+            auto frag = [&](int nt, int s, int plane) { return bf[nt * (btile >> 1) + plane * nfrag * 16 + s * 32]; };
+            auto sums = [&](int nt, int term) { return xf[nt * xtile + term * 32]; };
+            if (stream == 0) superblock_mma<Q5, NTERMS, NT>(cur, frag, sums, tig, tot_a);
+            else superblock_mma<Q5, NTERMS, NT>(cur, frag, sums, tig, tot_b);
         }
 
         // combine the kp partial sums of each row group in fixed order:

@@ -31,7 +31,9 @@ struct MmaRequest {
     const uint64_t *y_table;
     int rows_per_rank;
     int *status;
-    const void *images;   // mode 2, optional: per-token activation images (direct_token_images) of the rows of x
+    // optional: mode 2: per-token activation images (direct_token_images) of the rows of x; mode 3: images of the hidden
+    // activations (hidden_images), one per sorted assignment
+    const void *images;
 };
 
 // Launches the tensor-core kernel when the request fits it (alignment, K multiple of 256, shared
@@ -53,6 +55,15 @@ int direct_tokens_per_pass(int fmt, int mode, int k, int x_dtype);
 // launch that fills `images` [rows x bytes] from x [rows x k].
 int direct_token_image_bytes(int k, int x_dtype);
 int direct_token_images(const void *x, int x_dtype, int rows, int k, void *images, cudaStream_t stream);
+
+// Grouped launches over images (grouped_stream.cu): plans of more segments than a single decoded row's; *launched stays
+// false where they do not apply and the block-structured kernels take the request.
+constexpr int GROUPED_FEW_SEGMENTS = 16;
+int grouped_kp(int n, int nsb, int max_segments);
+int grouped_gate_up_launch(const MmaRequest &q, cudaStream_t stream, bool *launched);
+int grouped_down_launch(const MmaRequest &q, cudaStream_t stream, bool *launched);
+int hidden_image_bytes(int k);
+int hidden_images(const float *h, int rows, int k, void *images, cudaStream_t stream);
 
 // Weights in the Q6_K / Q8_0 tile layouts (mode 0 or 3, at most tiled_tokens_per_pass() tokens):
 // there is no other kernel for these layouts, so a request that does not fit returns an error

@@ -189,6 +189,7 @@ int tiled_plan_args(const MmaRequest &q, Q6TiledArgs *out, long long *smem_out) 
         };
         if (most(kp) > sm_count() && most(kp) <= 2LL * sm_count())
             while (kp > 1 && most(kp) > sm_count()) kp /= 2;
+        if (q.max_segments > GROUPED_FEW_SEGMENTS) kp = grouped_kp(q.n, nsb, q.max_segments);
     }
     a.kp = kp;
     a.rg = Q6T_WARPS / kp;
@@ -211,6 +212,11 @@ int q6k_tiled_launch(const MmaRequest &q, cudaStream_t stream) {
     long long smem = 0;
     const int rc = tiled_plan_args(q, &a, &smem);
     if (rc) return rc;
+    if (grouped) {
+        bool launched = false;
+        const int grc = grouped_down_launch(q, stream, &launched);
+        if (grc || launched) return grc;
+    }
     Q6Fn fn;
     if (q.fmt_a == B200Q_Q8_0_TILED) {
         if (grouped) fn = a.nterms == 2 ? tiled_kernel<Q8Tile, 3, 2, 1> : tiled_kernel<Q8Tile, 3, 1, 1>;

@@ -131,12 +131,11 @@ __device__ __forceinline__ float biased_byte_to_float(uint32_t word, int b) {
     return __uint_as_float(bits) - 8388736.0f;
 }
 
-// One tile: 16 scale groups = 16 mma steps; tot += d * sum_s scale_s * (codes_s . x_s). With NT
-// token tiles (8 tokens each, their fragments `tile_stride` entries apart) every decoded A operand
-// is multiplied into each of them, so the decode cost is paid once per 8*NT tokens.
-template <int NTERMS, int NT>
-__device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const uint2 *bfrag, int tile_stride, int nfrag, int sb,
-                                            int lane, float (&tot)[NT][4]) {
+// One tile: 16 scale groups = 16 mma steps; tot += d * sum_s scale_s * (codes_s . x_s). frag(nt, pair, plane) points to the
+// lane's 16 bytes of fragments 2 pair, 2 pair + 1 of the tile (plane 0: FP16 high parts, 1: remainders) of token tile nt:
+// every decoded A operand is multiplied into each token tile, so the decode cost is paid once per 8*NT tokens.
+template <int NTERMS, int NT, typename FragFn>
+__device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const FragFn frag, float (&tot)[NT][4]) {
     const uint32_t magic = 0x64006400u, neg = 0xe420e420u;       // 1024 | code ; -(1024 + 32)
     const uint32_t wa[12] = {r.c[0].x, r.c[0].y, r.c[0].z, r.c[0].w, r.c[1].x, r.c[1].y,
                              r.c[1].z, r.c[1].w, r.c[2].x, r.c[2].y, r.c[2].z, r.c[2].w};
@@ -154,6 +153,7 @@ __device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const uint2 *bf
         const uint32_t b0w = wb[3 * c], b1w = wb[3 * c + 1], b2w = wb[3 * c + 2];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
+            const int s = 8 * (c >> 1) + 2 * j + (c & 1);
             uint32_t p0a, p1a, p0b, p1b;
             if (j < 3) {
                 const uint32_t va = j == 0 ? a0w : (j == 1 ? a1w : a2w);
@@ -168,15 +168,18 @@ __device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const uint2 *bf
                 p0b = and_or(b2w >> 8, 0x00300030u, and_or(b0w >> 12, 0x000f000fu, magic));
                 p1b = and_or(b2w >> 10, 0x00300030u, and_or(b1w >> 12, 0x000f000fu, magic));
             }
-            const int s = 8 * (c >> 1) + 2 * j + (c & 1);
             const uint32_t a0 = hadd2_u32(p0a, neg), a1 = hadd2_u32(p0b, neg), a2 = hadd2_u32(p1a, neg),
                            a3 = hadd2_u32(p1b, neg);
             const float fa = biased_byte_to_float(sa[s >> 2], s & 3), fb = biased_byte_to_float(sb4[s >> 2], s & 3);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                const BFrag b = load_bfrag<NTERMS>(bfrag + nt * tile_stride, nfrag, sb * 16 + s, lane);
-                mma_terms<NTERMS>(acc, a0, a1, a2, a3, b);
+                float acc[4];
+                const uint2 bh = *reinterpret_cast<const uint2 *>(frag(nt, s >> 1, 0) + 8 * (s & 1));
+                mma_f16_first(acc, a0, a1, a2, a3, bh.x, bh.y);
+                if (NTERMS == 2) {
+                    const uint2 bl = *reinterpret_cast<const uint2 *>(frag(nt, s >> 1, 1) + 8 * (s & 1));
+                    mma_f16(acc, a0, a1, a2, a3, bl.x, bl.y);
+                }
                 blk[nt][0] = fmaf(fa, acc[0], blk[nt][0]);
                 blk[nt][1] = fmaf(fa, acc[1], blk[nt][1]);
                 blk[nt][2] = fmaf(fb, acc[2], blk[nt][2]);
@@ -200,10 +203,18 @@ struct Q6Tile {
     static constexpr int BYTES = Q6T_TILE_BYTES;
     using Regs = Q6TileRegs;
     static __device__ __forceinline__ void load(Regs &r, const uint8_t *tile, int lane) { load_q6_tile(r, tile, lane); }
-    template <int NTERMS, int NT>
-    static __device__ __forceinline__ void mma(const Regs &r, const uint2 *bfrag, int tile_stride, int nfrag, int sb,
-                                               int lane, float (&tot)[NT][4]) {
-        q6_tile_mma<NTERMS, NT>(r, bfrag, tile_stride, nfrag, sb, lane, tot);
+    static __device__ __forceinline__ void read(Regs &r, const uint8_t *tile, int lane) {       // from shared memory
+        const int g = lane >> 2;
+#pragma unroll
+        for (int p = 0; p < 6; ++p) r.c[p] = *reinterpret_cast<const uint4 *>(tile + p * 512 + lane * 16);
+        r.sa = *reinterpret_cast<const uint4 *>(tile + Q6T_SCALES_OFF + 16 * g);
+        r.sb = *reinterpret_cast<const uint4 *>(tile + Q6T_SCALES_OFF + 16 * (g + 8));
+        const uint16_t *d = reinterpret_cast<const uint16_t *>(tile + Q6T_D_OFF);
+        r.dd = d[g] | (static_cast<uint32_t>(d[g + 8]) << 16);
+    }
+    template <int NTERMS, int NT, typename FragFn>
+    static __device__ __forceinline__ void mma(const Regs &r, const FragFn frag, float (&tot)[NT][4]) {
+        q6_tile_mma<NTERMS, NT>(r, frag, tot);
     }
 };
 
@@ -228,9 +239,15 @@ struct Q8Tile {
         r.da = ldg128(tile + Q8T_SCALES_OFF + 16 * g);
         r.db = ldg128(tile + Q8T_SCALES_OFF + 16 * (g + 8));
     }
-    template <int NTERMS, int NT>
-    static __device__ __forceinline__ void mma(const Regs &r, const uint2 *bfrag, int tile_stride, int nfrag, int sb,
-                                               int lane, float (&tot)[NT][4]) {
+    static __device__ __forceinline__ void read(Regs &r, const uint8_t *tile, int lane) {       // from shared memory
+        const int g = lane >> 2;
+#pragma unroll
+        for (int p = 0; p < 8; ++p) r.c[p] = *reinterpret_cast<const uint4 *>(tile + p * 512 + lane * 16);
+        r.da = *reinterpret_cast<const uint4 *>(tile + Q8T_SCALES_OFF + 16 * g);
+        r.db = *reinterpret_cast<const uint4 *>(tile + Q8T_SCALES_OFF + 16 * (g + 8));
+    }
+    template <int NTERMS, int NT, typename FragFn>
+    static __device__ __forceinline__ void mma(const Regs &r, const FragFn frag, float (&tot)[NT][4]) {
         const uint32_t neg = 0xe480e480u;                       // -(1024 + 128)
         const uint32_t wa[16] = {r.c[0].x, r.c[0].y, r.c[0].z, r.c[0].w, r.c[1].x, r.c[1].y, r.c[1].z, r.c[1].w,
                                  r.c[2].x, r.c[2].y, r.c[2].z, r.c[2].w, r.c[3].x, r.c[3].y, r.c[3].z, r.c[3].w};
@@ -240,10 +257,12 @@ struct Q8Tile {
 #pragma unroll
         for (int blk = 0; blk < 8; ++blk) {
             float acc[NT][4];
+            uint4 bh[NT], bl[NT];
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
+            for (int nt = 0; nt < NT; ++nt) {
+                bh[nt] = *reinterpret_cast<const uint4 *>(frag(nt, blk, 0));
+                if (NTERMS == 2) bl[nt] = *reinterpret_cast<const uint4 *>(frag(nt, blk, 1));
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int s = 2 * blk + h;
@@ -254,8 +273,9 @@ struct Q8Tile {
                                a3 = hadd2_u32(__byte_perm(vb, 0x64646464u, 0x4341), neg);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    const BFrag b = load_bfrag<NTERMS>(bfrag + nt * tile_stride, nfrag, sb * 16 + s, lane);
-                    mma_terms<NTERMS>(acc[nt], a0, a1, a2, a3, b);
+                    if (h == 0) mma_f16_first(acc[nt], a0, a1, a2, a3, bh[nt].x, bh[nt].y);
+                    else mma_f16(acc[nt], a0, a1, a2, a3, bh[nt].z, bh[nt].w);
+                    if (NTERMS == 2) mma_f16(acc[nt], a0, a1, a2, a3, h ? bl[nt].z : bl[nt].x, h ? bl[nt].w : bl[nt].y);
                 }
             }
             const float fa = half_bits_to_float((da[blk >> 1] >> (16 * (blk & 1))) & 0xffffu);
@@ -272,7 +292,8 @@ struct Q8Tile {
 };
 
 // Activation fragments in natural order: fragment f (16 positions 16f..16f+15), lane (g, tig):
-// token g, positions 16f + 4tig + {0,2} -> b0, {1,3} -> b1; FP16 high part (+ remainder plane for
+// token g, positions 16f + 4tig + {0,2} -> b0, {1,3} -> b1, the two fragments of a pair side by side as in
+// prepare_direct (uint2 entry ((f >> 1) * 32 + lane) * 2 + (f & 1)); FP16 high part (+ remainder plane for
 // FP32 inputs) after a per-token power-of-two scaling. All Q6T_THREADS threads take part.
 template <int NTERMS, int KEEP, typename RowFn>
 __device__ __forceinline__ void prepare_fragments(RowFn row_of, int m_tokens, int k, const void *x, int x_dtype,
@@ -333,11 +354,11 @@ __device__ __forceinline__ void prepare_fragments(RowFn row_of, int m_tokens, in
             hi[i] = __half_as_ushort(h);
             lo[i] = __half_as_ushort(__float2half_rn(sv - __half2float(h)));
         }
-        const int f = p >> 4, dst = 4 * t + ((p >> 2) & 3);
-        bfrag[f * 32 + dst] = make_uint2(hi[0] | (static_cast<uint32_t>(hi[2]) << 16),
+        const int entry = ((p >> 5) * 32 + 4 * t + ((p >> 2) & 3)) * 2 + ((p >> 4) & 1);
+        bfrag[entry] = make_uint2(hi[0] | (static_cast<uint32_t>(hi[2]) << 16),
                                          hi[1] | (static_cast<uint32_t>(hi[3]) << 16));
         if (NTERMS == 2)
-            bfrag[(nfrag + f) * 32 + dst] = make_uint2(lo[0] | (static_cast<uint32_t>(lo[2]) << 16),
+            bfrag[nfrag * 32 + entry] = make_uint2(lo[0] | (static_cast<uint32_t>(lo[2]) << 16),
                                                        lo[1] | (static_cast<uint32_t>(lo[3]) << 16));
     };
 #pragma unroll
@@ -460,7 +481,10 @@ __device__ __forceinline__ void tiled_body(const Q6TiledArgs &a, const StagePoin
             cur = nxt;
             if (item + 1 < items_per_block) TILE::load(nxt, cur_p + (item + 1) * item_step, lane);
             else if (has_next) TILE::load(nxt, nxt_p, lane);
-            TILE::template mma<NTERMS, NT>(cur, bfrag, tile_stride, nfrag, kpi + item * a.kp, lane, tot);
+            const uint4 *bf = reinterpret_cast<const uint4 *>(bfrag) + (kpi + item * a.kp) * 256 + lane;
+            TILE::template mma<NTERMS, NT>(cur, [&](int nt, int pair, int plane) {
+                return reinterpret_cast<const uint8_t *>(bf + nt * (tile_stride >> 1) + plane * nfrag * 16 + pair * 32);
+            }, tot);
         }
 
         const int group = group0 + rgi;

@@ -355,7 +355,7 @@ static int moe_down_impl(const void *down_base, int64_t down_stride, int down_fm
                          int tables_aligned16, int flat_rows, int d, int f, const float *hbuf, const float *route,
                          const int32_t *order, const int32_t *seg_expert, const int32_t *seg_begin,
                          const int32_t *seg_count, const int32_t *num_segments, int max_segments, float *terms,
-                         const uint64_t *y_table, int rows_per_rank, void *stream) {
+                         const uint64_t *y_table, int rows_per_rank, const void *images, void *stream) {
     if ((!down_base && !down_table) || !hbuf || !route || !order || !seg_expert || !seg_begin || !seg_count ||
         !num_segments || (!terms && !y_table))
         return fail(B200Q_EINVAL, "moe_down: NULL pointer");
@@ -370,6 +370,7 @@ static int moe_down_impl(const void *down_base, int64_t down_stride, int down_fm
         q.seg_begin = seg_begin; q.seg_count = seg_count; q.num_segments = num_segments; q.max_segments = max_segments;
         q.route = route; q.flat_rows = (flat_rows || y_table) ? 1 : 0; q.y_table = y_table;
         q.rows_per_rank = rows_per_rank;
+        q.images = images;
         return q6k_tiled_launch(q, static_cast<cudaStream_t>(stream));
     }
     const bool tiled = direct_tiled_base(down_fmt) >= 0;
@@ -430,7 +431,26 @@ int b200q_moe_down(const void *down_base, int64_t down_stride, int down_fmt, con
                    const int32_t *seg_count, const int32_t *num_segments, int max_segments, float *terms,
                    void *stream) {
     return moe_down_impl(down_base, down_stride, down_fmt, down_table, tables_aligned16, flat_rows, d, f, hbuf, route,
-                         order, seg_expert, seg_begin, seg_count, num_segments, max_segments, terms, nullptr, 0,
+                         order, seg_expert, seg_begin, seg_count, num_segments, max_segments, terms, nullptr, 0, nullptr,
+                         stream);
+}
+
+int b200q_moe_hidden_image_bytes(int f) { return hidden_image_bytes(f); }
+
+int b200q_moe_hidden_images(const float *hbuf, int rows, int f, void *images, void *stream) {
+    if (!hbuf || !images) return fail(B200Q_EINVAL, "moe_hidden_images: NULL pointer");
+    if (rows <= 0 || f <= 0) return fail(B200Q_EINVAL, "moe_hidden_images: bad shape rows=%d f=%d", rows, f);
+    return hidden_images(hbuf, rows, f, images, static_cast<cudaStream_t>(stream));
+}
+
+int b200q_moe_down_images(const void *down_base, int64_t down_stride, int down_fmt, const uint64_t *down_table,
+                          int tables_aligned16, int flat_rows, int d, int f, const float *hbuf, const void *images,
+                          const float *route, const int32_t *order, const int32_t *seg_expert, const int32_t *seg_begin,
+                          const int32_t *seg_count, const int32_t *num_segments, int max_segments, float *terms,
+                          void *stream) {
+    if (!images) return fail(B200Q_EINVAL, "moe_down_images: NULL image buffer");
+    return moe_down_impl(down_base, down_stride, down_fmt, down_table, tables_aligned16, flat_rows, d, f, hbuf, route,
+                         order, seg_expert, seg_begin, seg_count, num_segments, max_segments, terms, nullptr, 0, images,
                          stream);
 }
 
@@ -442,7 +462,7 @@ int b200q_moe_down_peer(const void *down_base, int64_t down_stride, int down_fmt
     if (!term_tables) return fail(B200Q_EINVAL, "moe_down_peer: NULL term table");
     return moe_down_impl(down_base, down_stride, down_fmt, down_table, tables_aligned16, 1, d, f, hbuf, route, order,
                          seg_expert, seg_begin, seg_count, num_segments, max_segments, nullptr, term_tables,
-                         rows_per_rank, stream);
+                         rows_per_rank, nullptr, stream);
 }
 
 }  // extern "C"

@@ -155,9 +155,9 @@ def router_topk_plan_row(logits2d, k, n_experts, *, renormalize=True, floor=2.0 
     return weights, ids, plan
 
 
-# Rows of activations from which the grouped gate/up launch is fed with per-token images (one extra small
-# launch that converts every row once; below this the segments convert their few tokens themselves).
-TOKEN_IMAGE_MIN_ROWS = 32
+# Rows of activations from which the grouped launches are fed with images (one small launch before each that converts
+# every row once; a single row's plan of a few one-token segments converts its row itself).
+TOKEN_IMAGE_MIN_ROWS = 2
 
 
 def token_images(x2d):
@@ -214,6 +214,17 @@ def moe_down(hbuf, route_weights, plan, down_bank, down_fmt, d, f, down_stride, 
         raise ValueError("routing weights must be a contiguous FP32 tensor")
     terms = out if out is not None else torch.empty((plan.rows * plan.k, d), dtype=torch.float32,
                                                      device=hbuf.device)
+    # the tile-layout kernels of larger plans read images of the hidden rows (made here; the same bits either way)
+    if plan.rows >= TOKEN_IMAGE_MIN_ROWS and down_fmt in ("Q6_K_TILED", "Q8_0_TILED") and os.environ.get("B200Q_TOKEN_IMAGES", "1") != "0":
+        per_row = _lib.load().b200q_moe_hidden_image_bytes(int(f))
+        if per_row:
+            images = torch.empty((plan.rows * plan.k, per_row), dtype=torch.uint8, device=hbuf.device)
+            _lib.call("b200q_moe_hidden_images", _ptr(hbuf), plan.rows * plan.k, f, _ptr(images), _lib.current_stream())
+            _lib.call("b200q_moe_down_images", _ptr(down_bank), int(down_stride), _lib.FORMAT_ID[down_fmt], _ptr(down_table),
+                      1 if tables_aligned16 else 0, 1 if flat_rows else 0, d, f, _ptr(hbuf), _ptr(images), _ptr(route_weights),
+                      _ptr(plan.order), _ptr(plan.seg_expert), _ptr(plan.seg_begin), _ptr(plan.seg_count),
+                      _ptr(plan.num_segments), plan.max_segments, _ptr(terms), _lib.current_stream())
+            return terms
     _lib.call("b200q_moe_down", _ptr(down_bank), int(down_stride), _lib.FORMAT_ID[down_fmt], _ptr(down_table),
               1 if tables_aligned16 else 0, 1 if flat_rows else 0, d, f, _ptr(hbuf),
               _ptr(route_weights), _ptr(plan.order), _ptr(plan.seg_expert), _ptr(plan.seg_begin),
