@@ -369,11 +369,188 @@ __device__ __forceinline__ void prepare_direct(RowFn row_of, int m_tokens, int k
     named_barrier_sync(BARRIER, THREADS);
 }
 
+// Four consecutive activations as they lie in memory: FP32 inputs (NTERMS = 2) or 16-bit ones.
+template <int NTERMS>
+struct RawChunk {
+    uint32_t w[NTERMS == 2 ? 4 : 2];
+};
+// The chunk at element index e (a multiple of 4); `vec_ok` tells whether the tensor allows aligned vector loads.
+template <int NTERMS>
+__device__ __forceinline__ void load_chunk(const void *x, size_t e, bool vec_ok, RawChunk<NTERMS> &r) {
+    if constexpr (NTERMS == 2) {
+        const float *p = static_cast<const float *>(x) + e;
+        if (vec_ok) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(p);
+            r.w[0] = v.x; r.w[1] = v.y; r.w[2] = v.z; r.w[3] = v.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r.w[i] = __float_as_uint(p[i]);
+        }
+    } else {
+        const uint16_t *p = static_cast<const uint16_t *>(x) + e;
+        if (vec_ok) {
+            const uint2 v = *reinterpret_cast<const uint2 *>(p);
+            r.w[0] = v.x; r.w[1] = v.y;
+        } else {
+            r.w[0] = p[0] | (static_cast<uint32_t>(p[1]) << 16);
+            r.w[1] = p[2] | (static_cast<uint32_t>(p[3]) << 16);
+        }
+    }
+}
+// Bits of the largest magnitude of a chunk, in the type's own width: magnitudes order like their bits, Inf and NaN last.
+template <int NTERMS>
+__device__ __forceinline__ uint32_t chunk_amax(const RawChunk<NTERMS> &r) {
+    if constexpr (NTERMS == 2) {
+        return max(max(r.w[0] & 0x7fffffffu, r.w[1] & 0x7fffffffu), max(r.w[2] & 0x7fffffffu, r.w[3] & 0x7fffffffu));
+    } else {
+        const uint32_t m = __vmaxu2(r.w[0] & 0x7fff7fffu, r.w[1] & 0x7fff7fffu);
+        return max(m & 0xffffu, m >> 16);
+    }
+}
+template <int NTERMS>
+__device__ __forceinline__ void chunk_values(const RawChunk<NTERMS> &r, bool f16, float (&v)[4]) {
+    if constexpr (NTERMS == 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r.w[i]);
+    } else if (f16) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            v[2 * i] = __half2float(__ushort_as_half(static_cast<unsigned short>(r.w[i] & 0xffffu)));
+            v[2 * i + 1] = __half2float(__ushort_as_half(static_cast<unsigned short>(r.w[i] >> 16)));
+        }
+    } else {  // bf16: the upper 16 bits of an FP32
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            v[2 * i] = __uint_as_float(r.w[i] << 16);
+            v[2 * i + 1] = __uint_as_float(r.w[i] & 0xffff0000u);
+        }
+    }
+}
+
+// The same preparation, the same bits, for many chunks per thread (dense launches of several tokens). What bounds it is
+// the latency of the reads - every CTA reads all of x from L2 - so BATCH chunks are requested before the first is looked
+// at, and the second pass starts with the batch that the first left in registers; above, the conversion behind every load
+// waits for it. Launches of 8 tokens: Q4_K [8192 x 2048] 11.7 -> 8.7 us, Q8_0 [2048 x 8192] 27.7 -> 14.6 us; 16 tokens,
+// Q8_0 [2048 x 2048] 14.6 -> 8.8 us. Up to MD_FEW_CHUNKS chunks per thread the short code above is the faster one: these copies of a chunk's
+// code cost about 1 us of instruction fetch in a launch that uses one or two of them.
+// SUMS: also the activation sums of the sub-blocks.
+constexpr int MD_FEW_CHUNKS = 4;
+template <int NTERMS, int BATCH, bool SUMS, int THREADS, int BARRIER, typename RowFn>
+__device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k, const void *x, int x_dtype,
+                                               uint2 *bfrag, uint32_t *xsfrag, float *tok_scale, int tid) {
+    const int lane = tid & 31;
+    const int nfrag = k >> 4;
+    const bool vec_ok = (reinterpret_cast<uintptr_t>(x) % (NTERMS == 2 ? 16 : 8)) == 0;   // rows are multiples of 256 elements
+    const bool f16 = x_dtype == B200Q_F16;
+    unsigned int *amax_bits = reinterpret_cast<unsigned int *>(tok_scale + 16);   // [8]
+    if (tid < 8) amax_bits[tid] = 0u;
+    named_barrier_sync(BARRIER, THREADS);
+    const int chunks_per_token = k >> 2;            // a multiple of 64: a warp's 32 chunks share one token
+    const int total = m_tokens * chunks_per_token, first = tid & ~31;
+    // c / chunks_per_token for c <= 8 * chunks_per_token < 2^17 by a multiplication: the error of the rounded-up
+    // reciprocal, c / 2^32 at most, is below the distance 1 / chunks_per_token to the next whole number
+    const uint32_t recip = 0xffffffffu / static_cast<uint32_t>(chunks_per_token) + 1u;
+    auto token_of = [&](int c) { return static_cast<int>(__umulhi(static_cast<uint32_t>(c), recip)); };
+    RawChunk<NTERMS> raw[BATCH];
+    auto load_batch = [&](int base) {
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            const int c0 = base + i * THREADS;
+            if (c0 >= total) break;
+            const int t = token_of(c0);
+            load_chunk<NTERMS>(x, static_cast<size_t>(row_of(t)) * k + static_cast<size_t>(c0 + lane - t * chunks_per_token) * 4,
+                               vec_ok, raw[i]);
+        }
+    };
+    // 1. per-token maximum magnitude
+    int kept = first;                               // base of the batch in registers
+    for (int base = first; base < total; base += BATCH * THREADS) {
+        kept = base;
+        load_batch(base);
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            const int c0 = base + i * THREADS;
+            if (c0 >= total) break;
+            const uint32_t m = __reduce_max_sync(0xffffffffu, chunk_amax<NTERMS>(raw[i]));
+            if (lane == 0) atomicMax(&amax_bits[token_of(c0)], m);
+        }
+    }
+    named_barrier_sync(BARRIER, THREADS);
+    if (tid < 8) {
+        const uint32_t bits = amax_bits[tid];
+        float amax;
+        if (NTERMS == 2) amax = __uint_as_float(bits);
+        else amax = f16 ? __half2float(__ushort_as_half(static_cast<unsigned short>(bits))) : __uint_as_float(bits << 16);
+        float s = 1.0f;                             // (stays 1 where the maximum is Inf or NaN)
+        if (amax > 0.f && amax < __int_as_float(0x7f800000)) {
+            int e;
+            frexpf(amax, &e);
+            s = ldexpf(1.0f, min(14 - e, 100));   // scaled maximum in [2^13, 2^14)
+        }
+        tok_scale[tid] = s;
+        tok_scale[8 + tid] = 1.0f / s;
+    }
+    named_barrier_sync(BARRIER, THREADS);
+    // 2. scale, split, store: the chunk at position p of token t is the entry of fragment f = p>>4, lane 4t + ((p>>2)&3)
+    auto store_chunk = [&](int c0, const RawChunk<NTERMS> &r) {
+        const int t = token_of(c0);
+        const int p = (c0 + lane - t * chunks_per_token) * 4;
+        const float s = tok_scale[t];
+        float v[4];
+        chunk_values<NTERMS>(r, f16, v);
+        unsigned short hi[4], lo[4];
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float sv = v[i] * s;
+            const __half h = __float2half_rn(sv);
+            hi[i] = __half_as_ushort(h);
+            if (SUMS) sum += __half2float(h);
+            if (NTERMS == 2) {
+                const __half l = __float2half_rn(sv - __half2float(h));
+                lo[i] = __half_as_ushort(l);
+                if (SUMS) sum += __half2float(l);
+            }
+        }
+        const int entry = ((p >> 5) * 32 + 4 * t + ((p >> 2) & 3)) * 2 + ((p >> 4) & 1);
+        bfrag[entry] = make_uint2(hi[0] | (static_cast<uint32_t>(hi[2]) << 16), hi[1] | (static_cast<uint32_t>(hi[3]) << 16));
+        if (NTERMS == 2)
+            bfrag[nfrag * 32 + entry] = make_uint2(lo[0] | (static_cast<uint32_t>(lo[2]) << 16), lo[1] | (static_cast<uint32_t>(lo[3]) << 16));
+        if (SUMS) {
+            // sub-block sum: its eight chunks sit in eight consecutive lanes
+            const int sb = p >> 8, sub = (p >> 5) & 7;
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            if ((lane & 7) == 0) {
+                const float scaled = sum * MD_XS_SCALE;
+                const __half h = __float2half_rn(scaled);
+                const __half l = __float2half_rn(scaled - __half2float(h));
+                // operand of the min product: lane 4*t + (sub>>1) holds sub-blocks (sub & ~1, sub | 1)
+                const int lane_t = 4 * t + (sub >> 1);
+                reinterpret_cast<unsigned short *>(xsfrag + (sb * 2 + 0) * 32 + lane_t)[sub & 1] = __half_as_ushort(h);
+                reinterpret_cast<unsigned short *>(xsfrag + (sb * 2 + 1) * 32 + lane_t)[sub & 1] = __half_as_ushort(l);
+            }
+        }
+    };
+    for (int base = kept;;) {
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+            if (base + i * THREADS >= total) break;
+            store_chunk(base + i * THREADS, raw[i]);
+        }
+        base = base == kept ? first : base + BATCH * THREADS;       // the batches before the kept one, again from memory
+        if (base >= kept) break;
+        load_batch(base);
+    }
+    named_barrier_sync(BARRIER, THREADS);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Token images. In the grouped gate/up launch every expert segment needs the fragments of its tokens, and
 // a token routed to k experts would be converted k times (at 64 tokens: 704 conversions of 64 distinct
 // rows, each a chain of dependent loads, a reduction and three barriers). token_image_kernel runs
-// prepare_direct once per token - same code, so the same bits - and stores what it wrote for token slot 0:
+// prepare_tokens once per token - same code, so the same bits - and stores what it wrote for token slot 0:
 //   [NTERMS * nfrag * 32 bytes]  the slot's four lanes (tig 0..3, 16 bytes each) of every pair of fragments
 //   [nsb * 2 * 16 bytes]         the slot's four words of every activation-sum row
 //   [16 bytes]                   scale, inverse scale
@@ -628,10 +805,16 @@ __device__ __forceinline__ void mma_direct_body(const DirectArgs &a, const Stage
     int seg_begin = 0, cur_unit = -1, last_single = (MODE == 2) ? gp.prepared_row : -1;
     if (!GROUPED) {
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-            prepare_direct<NTERMS, (NT == 1 ? 4 : 2)>([nt](int t) { return 8 * nt + t; }, max(min(a.m - 8 * nt, 8), 0),
-                                                      a.k, gp.x, a.x_dtype, bfrag + nt * btile, xsfrag + nt * xtile,
-                                                      tok_scale + nt * MD_TOK_STRIDE, tid);
+        for (int nt = 0; nt < NT; ++nt) {
+            const auto row_of = [nt](int t) { return 8 * nt + t; };
+            const int tokens = max(min(a.m - 8 * nt, 8), 0);
+            if (NT == 2 || tokens * (a.k >> 2) > MD_FEW_CHUNKS * MD_THREADS)
+                prepare_tokens<NTERMS, 8, true, MD_THREADS, 1>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * btile,
+                                                               xsfrag + nt * xtile, tok_scale + nt * MD_TOK_STRIDE, tid);
+            else
+                prepare_direct<NTERMS, MD_FEW_CHUNKS>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * btile,
+                                                      xsfrag + nt * xtile, tok_scale + nt * MD_TOK_STRIDE, tid);
+        }
     }
 
     int pbuf = 0;

@@ -442,10 +442,16 @@ __device__ __forceinline__ void tiled_body(const Q6TiledArgs &a, const StagePoin
     int seg_begin = 0, cur_unit = -1;
     if (!GROUPED) {
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-            prepare_fragments<NTERMS, (NT == 1 ? 4 : 2)>([nt](int t) { return 8 * nt + t; }, max(min(a.m - 8 * nt, 8), 0),
-                                                         a.k, gp.x, a.x_dtype, bfrag + nt * tile_stride,
+        for (int nt = 0; nt < NT; ++nt) {
+            const auto row_of = [nt](int t) { return 8 * nt + t; };
+            const int tokens = max(min(a.m - 8 * nt, 8), 0);
+            if (NT == 2 || tokens * (a.k >> 2) > MD_FEW_CHUNKS * Q6T_THREADS)
+                prepare_tokens<NTERMS, 8, false, Q6T_THREADS, 1>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * tile_stride,
+                                                                 nullptr, tok_scale + nt * Q6T_TOK_STRIDE, tid);
+            else
+                prepare_fragments<NTERMS, MD_FEW_CHUNKS>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * tile_stride,
                                                          tok_scale + nt * Q6T_TOK_STRIDE, tid);
+        }
     }
 
     int pbuf = 0;
