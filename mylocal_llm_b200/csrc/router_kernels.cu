@@ -92,6 +92,95 @@ __global__ void __launch_bounds__(256) router_logits_t_kernel(const void *x, int
     }
 }
 
+// The same logits from register tiles: a warp holds R expert rows x TOK tokens (a lane the columns 4 lane.. of every 128),
+// so a 16-byte read of x from shared memory feeds 4 R FMAs and one of the weight 4 TOK; the kernel above reads a row of x
+// per expert row and waits for shared memory. The sums are that kernel's, bit for bit: per lane one chain of FMAs in
+// column order (columns past d are zeros on both sides), lanes added in warp_sum's order - each butterfly step here hands
+// half of the values to the partner lane, which ends with one of the 32 per lane. A warp has 32 chains, enough to fill the FMA pipe
+// (R = 8, 64 chains: as fast at 256 tokens, twice as long below 64, where too few CTAs are left).
+template <int R, int TOK>
+__global__ void __launch_bounds__(256, 2) router_logits_tile_kernel(const void *x, int x_dtype, int t, int d, const float *wt,
+                                                                    const float *bias, int e, float *logits) {
+    constexpr int V = R * TOK;
+    static_assert(V % 32 == 0 && TOK % (V / 32) == 0, "whole values per lane");
+    chain_trigger();
+    extern __shared__ float xs[];   // [TOK][dpad]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int dpad = (d + 127) & ~127, t0 = blockIdx.y * TOK;
+    const int row0 = (blockIdx.x * 8 + warp) * R;
+    const float *wp[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) wp[r] = wt + static_cast<size_t>(min(row0 + r, e - 1)) * d + lane * 4;
+    chain_wait();                   // x comes from preceding kernels
+    {
+        const size_t esize = x_dtype == B200Q_F32 ? 4 : 2;
+        const bool vec_ok = (reinterpret_cast<uintptr_t>(x) % (4 * esize)) == 0;
+        for (int i = tid * 4; i < TOK * dpad; i += 256 * 4) {
+            const int tt = i / dpad, col = i - tt * dpad;
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (t0 + tt < t && col < d) {
+                const size_t at = static_cast<size_t>(t0 + tt) * d + col;
+                if (vec_ok && x_dtype == B200Q_F32) {
+                    q = *reinterpret_cast<const float4 *>(static_cast<const float *>(x) + at);
+                } else if (vec_ok) {
+                    const uint2 raw = *reinterpret_cast<const uint2 *>(static_cast<const uint16_t *>(x) + at);
+                    q = x_dtype == B200Q_F16
+                            ? make_float4(half_bits_to_float(raw.x & 0xffffu), half_bits_to_float(raw.x >> 16),
+                                          half_bits_to_float(raw.y & 0xffffu), half_bits_to_float(raw.y >> 16))
+                            : make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
+                                          __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
+                } else {
+                    q = make_float4(load_as_float(x, x_dtype, at), load_as_float(x, x_dtype, at + 1),
+                                    load_as_float(x, x_dtype, at + 2), load_as_float(x, x_dtype, at + 3));
+                }
+            }
+            *reinterpret_cast<float4 *>(xs + i) = q;
+        }
+    }
+    __syncthreads();
+    if (row0 >= e) return;
+    float acc[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] = 0.f;
+    const float *xp = xs + lane * 4;
+    for (int col = lane * 4; col < dpad; col += 128, xp += 128) {
+        float4 w[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            w[r] = col < d ? *reinterpret_cast<const float4 *>(wp[r]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            wp[r] += 128;
+        }
+#pragma unroll
+        for (int tt = 0; tt < TOK; ++tt) {
+            const float4 xv = *reinterpret_cast<const float4 *>(xp + tt * dpad);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                float s = acc[r * TOK + tt];
+                s = fmaf(w[r].x, xv.x, s);
+                s = fmaf(w[r].y, xv.y, s);
+                s = fmaf(w[r].z, xv.z, s);
+                acc[r * TOK + tt] = fmaf(w[r].w, xv.w, s);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] = 0.f + acc[i];          // (a chain that ends in -0 counts as +0 there)
+#pragma unroll
+    for (int o = 16, n = V / 2; o; o >>= 1, n >>= 1) {
+        const bool upper = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float keep = upper ? acc[n + i] : acc[i], give = upper ? acc[i] : acc[n + i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < V / 32; ++i) {
+        const int v = lane * (V / 32) + i, row = row0 + v / TOK, tok = t0 + v % TOK;
+        if (row < e && tok < t) logits[static_cast<size_t>(tok) * e + row] = acc[i] + (bias ? bias[row] : 0.f);
+    }
+}
+
 // Ordered combine, one thread per output column: the k terms are loaded first (independent
 // loads), then added one by one in ascending position order with plain FP32 adds.
 template <int KMAX>
@@ -218,6 +307,21 @@ extern "C" int b200q_router_logits_t(const void *x, int x_dtype, int t, int d, c
     if (!dtype_valid(x_dtype)) return fail(B200Q_EINVAL, "router_logits_t: bad dtype");
     if (t <= 0 || d <= 0 || e <= 0 || d % 4) return fail(B200Q_EINVAL, "router_logits_t: bad shape (d %% 4 == 0)");
     if (reinterpret_cast<uintptr_t>(wt) & 15) return fail(B200Q_EINVAL, "router_logits_t: weight must be 16-byte aligned");
+    // Register tiles from 40960 logits on (d = 2048: 96 tokens x 512 experts 26.0 -> 12.8 us, 256 66.6 -> 24.3, 512 124 ->
+    // 43; 256 tokens x 128 experts, below the line, 19.0 against 12.3). 64 x 512 is 15.3 against 12.4 alone, but an 8-layer
+    // step of that size took 1962 us with the kernel above and 1980 with the tiles; 32 x 512 8.4 against 10.6.
+    if (static_cast<long long>(t) * e >= 40960 && d <= RT_CHUNK) {
+        constexpr int R = 4, TOK = 8;
+        auto fn = router_logits_tile_kernel<R, TOK>;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, TOK * RT_CHUNK * 4) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(B200Q_ECUDA, "router_logits_t: shared memory opt-in failed");
+        }
+        launch_chained(fn, dim3((e + 8 * R - 1) / (8 * R), (t + TOK - 1) / TOK), dim3(256),
+                       static_cast<size_t>(TOK) * ((d + 127) & ~127) * sizeof(float), static_cast<cudaStream_t>(stream), x, x_dtype,
+                       t, d, wt, bias, e, logits);
+        return check_launch("router_logits_t");
+    }
     // 8 tokens per CTA (three CTAs per SM at d = 2048) up to 128 rows, 16 beyond
     const int tok = t <= 128 ? 8 : 16;
     const size_t smem = static_cast<size_t>(tok) * d * sizeof(float);
