@@ -844,35 +844,51 @@ static int gemm_pair_mode() {          // read at every call, so a test can comp
 }
 
 // y[t, col] = partial[0][t, col] + partial[1][t, col] + ... in ascending split order (deterministic), rounded once.
+template <int VEC>      // outputs per thread: 4 where m * n is a multiple of 4 (16-byte aligned parts), else 1
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *partial, int splits, long long count, void *y,
                                                             int y_dtype) {
     chain_trigger();
     chain_wait();
-    const long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 4;
-    if (i >= count) return;                           // count is a multiple of 4 (n is)
-    float4 acc = *reinterpret_cast<const float4 *>(partial + i);
-    for (int z = 1; z < splits; ++z) {
-        const float4 v = *reinterpret_cast<const float4 *>(partial + static_cast<size_t>(z) * count + i);
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    const long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * VEC;
+    if (i >= count) return;
+    float acc[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
+    for (int z = 0; z < splits; ++z) {
+        float v[VEC];
+        const float *src = partial + static_cast<size_t>(z) * count + i;
+        if constexpr (VEC == 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(src);
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        } else {
+            v[0] = src[0];
+        }
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] = z ? acc[e] + v[e] : v[e];
     }
-    store_out(y, y_dtype, i, __float_as_uint(acc.x));
-    store_out(y, y_dtype, i + 1, __float_as_uint(acc.y));
-    store_out(y, y_dtype, i + 2, __float_as_uint(acc.z));
-    store_out(y, y_dtype, i + 3, __float_as_uint(acc.w));
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) store_out(y, y_dtype, i + e, __float_as_uint(acc[e]));
 }
 
-// Split of K over grid.z for shapes with too few (weight-row tile x token tile) CTAs to fill the SMs: a power
-// of two, at least 4 groups (16 slabs) of K per CTA, no more CTAs than SMs; 1 = no split.
+// Split of K over grid.z for shapes with too few (weight-row tile x token tile) CTAs to fill the SMs: at least 4 groups
+// (16 slabs) of K per CTA (rounded up: the longest part is what counts), no more CTAs than SMs; 1 = no split. Where the
+// groups are a power of two, so is the split: equal parts, and the sums of those shapes keep their order. Other K have
+// uneven parts anyway and take the split with the shortest longest part ([5003 x 2816] x 77, Q6_K: 40 CTAs of 11 groups
+// 26.7 us, 120 CTAs of 4, 4 and 3 with the sum 17.6 us).
 static int gemm_splits(int n, int k, int m) {
-    if (n % 4 != 0) return 1;
     const int ntok = m >= 256 ? 256 : (m + 15) / 16 * 16;
     const int token_tiles = (m + ntok - 1) / ntok;
     const int n_tiles = (n + UG_BM - 1) / UG_BM;
     const int mt = (token_tiles >= 2 && static_cast<long long>(n_tiles) * ((token_tiles + 1) / 2) >= sm_count()) ? 2 : 1;
     const long long ctas = static_cast<long long>(n_tiles) * ((token_tiles + mt - 1) / mt);
     int splits = 1;
-    while (splits < 8 && ctas * splits * 2 <= sm_count() && (k / 256) / (splits * 2) >= 4) splits *= 2;
-    return splits;
+    const int groups = k / 256;
+    while (splits < 8 && ctas * splits * 2 <= sm_count() && groups / (splits * 2) >= 4) splits *= 2;
+    auto part = [groups](int s) { return (groups + s - 1) / s; };
+    if (groups & (groups - 1))
+        for (int s = splits + 1; s <= 8 && ctas * s <= sm_count() && part(s) >= 4; ++s)
+            if (part(s) < part(splits)) splits = s;
+    return part(part(splits));                         // (33 groups in 8 parts are 5 each: seven parts, none empty)
 }
 
 }  // namespace b200q
@@ -979,8 +995,10 @@ static int gemm_impl(const void *w, int fmt, int n, int k, const void *x, int x_
     int rc = check_launch("gemm");
     if (rc || splits == 1) return rc;
     const long long count = static_cast<long long>(m) * n;
-    launch_chained(splitk_reduce_kernel, dim3(static_cast<unsigned>((count / 4 + 255) / 256)), dim3(256), 0,
-                   static_cast<cudaStream_t>(stream), static_cast<const float *>(workspace), splits, count, y, y_dtype);
+    const int vec = count % 4 == 0 ? 4 : 1;
+    launch_chained(vec == 4 ? splitk_reduce_kernel<4> : splitk_reduce_kernel<1>,
+                   dim3(static_cast<unsigned>((count / vec + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                   static_cast<const float *>(workspace), splits, count, y, y_dtype);
     return check_launch("gemm (split-K sum)");
 }
 
