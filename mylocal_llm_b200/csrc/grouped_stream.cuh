@@ -15,6 +15,9 @@
 // Image rows lie behind one another in shared memory, 64 bytes more than a multiple of 128 apart, so the eight lanes of a
 // quarter warp (two tokens x 64 bytes) read eight different 16-byte banks groups.
 // The sums are those of the block-structured kernels with the same kp, bit for bit.
+// Bound by instruction issue (256 tokens, 512 experts: 0.63-0.68 of the slots, ALU pipe 0.54, DRAM 0.53 / 0.40): positions
+// in the run of row groups are kept by steps instead of divisions, and the copies are predicated, not branched around
+// (8-layer step of 64 tokens 1962 -> 1902 us, 16-token layer 133 -> 128).
 #pragma once
 
 #include "q6k_tiled.cuh"
@@ -77,6 +80,32 @@ __device__ __forceinline__ bool request_segment(const GroupedArgs &a, SegmentRin
     return true;
 }
 
+// Position in the CTA's run of row groups, advanced a round of teams at a time (a division per item costs as much as a
+// tile's loads).
+struct GroupCursor {
+    int item, seg, group;
+    __device__ __forceinline__ void step(int teams, int groups_per_seg) {
+        item += teams;
+        group += teams;
+        while (group >= groups_per_seg) {
+            group -= groups_per_seg;
+            ++seg;
+        }
+    }
+};
+
+// One bulk copy into the ring, announced on its barrier; issued by the lane that `issue` names, without a branch.
+__device__ __forceinline__ void request_tile(bool issue, uint64_t *bar, uint8_t *dst, const uint8_t *src, uint32_t bytes) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %0, 0;\n\t"
+        "@p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %4;\n\t"
+        "@p cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%2], [%3], %4, [%1];\n\t}" ::"r"(
+            static_cast<int>(issue)),
+        "r"(smem_u32(bar)), "r"(smem_u32(dst)), "l"(src), "r"(bytes)
+        : "memory");
+}
+
 // A warp's stream of weight tiles: the tiles of its row groups in order (DUAL: gate and up alternating), fetched by bulk
 // copies a ring ahead of their use. All lanes keep the cursor, lane 0 issues.
 template <int TILE, bool DUAL>
@@ -86,35 +115,33 @@ struct TileStream {
     uint64_t *full;                // its mbarriers
     int slot, phase;               // next tile to consume
     int item, end, teams, kpi;     // fetch cursor: row group, its tile, stream; end of the CTA's range
+    GroupCursor ahead;             // the row group after that: na, nb are its matrices
     int groups_per_seg, sb, upper;
     const uint8_t *wa, *wb, *na, *nb;
 
-    __device__ __forceinline__ void bases(int it, const uint8_t *&pa, const uint8_t *&pb) const {
-        if (it >= end) return;
-        const int seg = it / groups_per_seg, group = it - seg * groups_per_seg;
-        const int expert = a.seg_expert[seg];
-        const size_t off = (static_cast<size_t>(group) * a.nsb + kpi) * TILE;
+    __device__ __forceinline__ void bases(const GroupCursor &at, const uint8_t *&pa, const uint8_t *&pb) const {
+        if (at.item >= end) return;
+        const int expert = a.seg_expert[at.seg];
+        const size_t off = (static_cast<size_t>(at.group) * a.nsb + kpi) * TILE;
         pa = expert_matrix(a.wa, a.stride_a, a.table_a, expert) + off;
         if (DUAL) pb = expert_matrix(a.wb, a.stride_b, a.table_b, expert) + off;
     }
-    __device__ __forceinline__ void start(int first, int lane) {
-        item = first;
+    __device__ __forceinline__ void start(const GroupCursor &first, int lane) {
+        item = first.item;
+        ahead = first;
         sb = kpi;
         upper = 0;
         slot = phase = 0;
         wa = wb = na = nb = nullptr;
-        bases(item, wa, wb);
-        bases(item + teams, na, nb);
+        bases(first, wa, wb);
+        ahead.step(teams, groups_per_seg);
+        bases(ahead, na, nb);
         for (int i = 0; i < a.ring; ++i) fetch(i, lane);
     }
     // requests the tile at the cursor into slot `into` and moves on
     __device__ __forceinline__ void fetch(int into, int lane) {
         if (item >= end) return;
-        const uint8_t *src = (DUAL && upper) ? wb : wa;
-        if (lane == 0) {
-            mbar_arrive_expect_tx(&full[into], TILE);
-            bulk_copy_g2s(slots + into * TILE, src, TILE, &full[into]);
-        }
+        request_tile(lane == 0, &full[into], slots + into * TILE, (DUAL && upper) ? wb : wa, TILE);
         if (DUAL) {
             upper ^= 1;
             if (upper) return;
@@ -127,7 +154,8 @@ struct TileStream {
             sb = kpi;
             wa = na;
             wb = nb;
-            bases(item + teams, na, nb);
+            ahead.step(teams, groups_per_seg);
+            bases(ahead, na, nb);
         }
     }
     // the next tile in shared memory (false: gave up); after its last read the caller calls refill()
@@ -171,13 +199,15 @@ __device__ __forceinline__ void grouped_walk(const GroupedArgs &a, uint8_t *smem
     fence_barrier_init();
     __syncthreads();
     const int teams = GS_WARPS / a.kp, team = warp / a.kp, kpi = warp - team * a.kp;
-    int item = begin + team, seg = ring.first;
+    GroupCursor at{begin, ring.first, begin - ring.first * groups_per_seg};     // this warp's row group
+    at.step(team, groups_per_seg);
+    int seg = ring.first, buf = 0, phase = 0;              // segment this warp is in, its buffer and that buffer's round
     TileStream<TILE, DUAL> stream{a, smem + a.off_ring + static_cast<size_t>(warp) * a.ring * TILE, tile_bars};
     stream.end = end;
     stream.teams = teams;
     stream.kpi = kpi;
     stream.groups_per_seg = groups_per_seg;
-    stream.start(item, lane);
+    stream.start(at, lane);
     ring.issued = ring.first;
     bool ok = true;
     const int ahead = a.bufs - 1;
@@ -185,33 +215,35 @@ __device__ __forceinline__ void grouped_walk(const GroupedArgs &a, uint8_t *smem
         while (ok && ring.issued <= min(ring.first + ahead, ring.last)) ok = request_segment<SORTED>(a, ring, ring.issued++, bufs, lane);
 
     bool entered = false;                                  // this warp has waited for segment `seg`
-    auto wait_full = [&](int s) {
-        const int at = s - ring.first;
-        return __all_sync(0xffffffffu, mbar_wait_bounded(&full[at % a.bufs], (at / a.bufs) & 1, a.status, STATUS_GROUPED_WAIT)) != 0;
+    auto wait_full = [&](int b, int ph) {
+        return __all_sync(0xffffffffu, mbar_wait_bounded(&full[b], ph, a.status, STATUS_GROUPED_WAIT)) != 0;
     };
     // Leaves the segments before `upto` in order, each after its activations have landed (also those this warp has no
     // group in: a buffer's next round can then not be released before this one). The producer requests the segments that
     // now fit only on its next entry (below): it would wait here for warps that are still in the segment it left.
     auto advance = [&](int upto) {
         while (ok && seg < upto) {
-            if (!entered) ok = wait_full(seg);
-            if (ok && lane == 0) mbar_arrive(&empty[(seg - ring.first) % a.bufs]);
+            if (!entered) ok = wait_full(buf, phase);
+            if (ok && lane == 0) mbar_arrive(&empty[buf]);
             ++seg;
+            if (++buf == a.bufs) {
+                buf = 0;
+                phase ^= 1;
+            }
             entered = false;
             if (warp == 0)
                 while (ok && ring.issued <= min(seg + ahead - 1, ring.last)) ok = request_segment<SORTED>(a, ring, ring.issued++, bufs, lane);
         }
     };
-    while (ok && item < end) {
-        const int now = item / groups_per_seg;
-        advance(now);
+    while (ok && at.item < end) {
+        advance(at.seg);
         if (ok && !entered) {
-            ok = wait_full(now);
+            ok = wait_full(buf, phase);
             entered = true;
         }
         if (!ok) break;
-        ok = work(now, item - now * groups_per_seg, bufs + static_cast<size_t>((now - ring.first) % a.bufs) * 8 * a.smem_stride, stream);
-        item += teams;
+        ok = work(seg, at.group, bufs + static_cast<size_t>(buf) * 8 * a.smem_stride, stream);
+        at.step(teams, groups_per_seg);
         // after its first group of a segment the producer asks for the one whose buffer the others have left by now
         if (warp == 0 && ok && ring.issued <= min(seg + ahead, ring.last)) ok = request_segment<SORTED>(a, ring, ring.issued++, bufs, lane);
     }
@@ -219,7 +251,8 @@ __device__ __forceinline__ void grouped_walk(const GroupedArgs &a, uint8_t *smem
     if (!ok) {
         // gave up: copies may still be on their way into this CTA's shared memory - let each of them land (bounded)
         if (warp == 0)
-            for (int s = max(ring.first, ring.issued - a.bufs); s < ring.issued; ++s) wait_full(s);
+            for (int s = max(ring.first, ring.issued - a.bufs); s < ring.issued; ++s)
+                wait_full((s - ring.first) % a.bufs, ((s - ring.first) / a.bufs) & 1);
         for (int i = 0; i < a.ring; ++i) {
             mbar_wait_bounded(&tile_bars[stream.slot], stream.phase, a.status, STATUS_GROUPED_TILE);
             if (++stream.slot == a.ring) {

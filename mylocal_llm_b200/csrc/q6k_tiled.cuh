@@ -125,10 +125,14 @@ __device__ __forceinline__ uint32_t hadd2_u32(uint32_t a, uint32_t b) {
     return d;
 }
 
-// Scale byte b of `word` (stored +128) as an exact float.
-__device__ __forceinline__ float biased_byte_to_float(uint32_t word, int b) {
-    const uint32_t bits = __byte_perm(word, 0x4b000000u, 0x7650 + b);     // 8388608 + byte
-    return __uint_as_float(bits) - 8388736.0f;
+// Scale byte b of two words (stored +128) as exact floats, one packed subtraction for both.
+__device__ __forceinline__ void biased_bytes_to_float2(uint32_t wa, uint32_t wb, int b, float &fa, float &fb) {
+    const uint32_t va = __byte_perm(wa, 0x4b000000u, 0x7650 + b), vb = __byte_perm(wb, 0x4b000000u, 0x7650 + b);  // 8388608 + byte
+    uint64_t v, bias;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(va), "r"(vb));
+    asm("mov.b64 %0, {%1, %1};" : "=l"(bias) : "f"(-8388736.0f));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(bias));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(fa), "=f"(fb) : "l"(v));
 }
 
 // One tile: 16 scale groups = 16 mma steps; tot += d * sum_s scale_s * (codes_s . x_s). frag(nt, pair, plane) points to the
@@ -170,7 +174,8 @@ __device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const FragFn fr
             }
             const uint32_t a0 = hadd2_u32(p0a, neg), a1 = hadd2_u32(p0b, neg), a2 = hadd2_u32(p1a, neg),
                            a3 = hadd2_u32(p1b, neg);
-            const float fa = biased_byte_to_float(sa[s >> 2], s & 3), fb = biased_byte_to_float(sb4[s >> 2], s & 3);
+            float fa, fb;
+            biased_bytes_to_float2(sa[s >> 2], sb4[s >> 2], s & 3, fa, fb);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 float acc[4];
