@@ -274,6 +274,9 @@ __host__ __device__ constexpr int fmt_group_bytes(int fmt) {        // packed by
     return fmt == B200Q_Q8_0 ? 8 * 34 : fmt == B200Q_Q4_K ? 144 : fmt == B200Q_Q5_K ? 176 : 210;
 }
 
+// bytes between the L2 requests of a row's four threads for one group (see decode_group)
+__host__ __device__ constexpr int fmt_prefetch_step(int fmt) { return fmt == B200Q_Q8_0 ? fmt_group_bytes(fmt) / 4 : 0; }
+
 struct RawGroup {
     uint4 q[4];   // slab SL's 16 code bytes (Q4_K / Q5_K: nibble bytes; Q6_K: low-nibble bytes; Q8_0: codes)
     uint4 h[2];   // Q5_K: h[0] = high-bit bytes; Q6_K: h[half] = bytes holding the upper two bits
@@ -514,7 +517,9 @@ __device__ __forceinline__ bool decode_store_two(const RawGroup (&grp)[PIECES], 
 
 // The four slabs of group g from `cur`; after the first two of them (when cur's bytes have arrived and no other
 // load of this thread is in flight) the packed bytes of group g + 1 are requested into `nxt`, and L2 is asked
-// for group g + 3. The request sits after a slab and not at the end of the previous group on purpose: the
+// for group g + 3: each of a row's four threads for its own quarter of the 272 bytes of Q8_0 (one request brings 128 bytes
+// at most; 24-layer prompt of 512 tokens 5566 -> 5448 us), all four for the start of a K-quant block, which is most of it
+// (quarters measured 1 % slower there: Q5_K [8192 x 2048] x 512 23.3 -> 23.6 us). The request sits after a slab and not at the end of the previous group on purpose: the
 // hardware waits for "all loads issued so far under this dependency counter", and with the loads of both
 // register sets in flight at the first use of one of them a decoder waited out the full memory latency of
 // the set it had just requested (2.6 stalled warps per issue at [8192 x 2048] x 512).
@@ -522,12 +527,13 @@ template <int FMT, int PIECES>
 __device__ __forceinline__ bool decode_group(const RawGroup (&cur)[PIECES], RawGroup (&nxt)[PIECES],
                                              const uint8_t *const (&row_ptr)[PIECES], const int (&prow)[PIECES],
                                              const int (&pquart)[PIECES], int g, int ngroups, DecoderRing &ring, int lane) {
-    constexpr int GB = fmt_group_bytes(FMT);
+    constexpr int GB = fmt_group_bytes(FMT), ASK = fmt_prefetch_step(FMT);
     if (!decode_store_two<FMT, 0, PIECES>(cur, prow, pquart, ring, lane)) return false;
 #pragma unroll
     for (int j = 0; j < PIECES; ++j) {
         fetch_group<FMT>(row_ptr[j] + static_cast<size_t>(min(g + 1, ngroups - 1)) * GB, pquart[j], nxt[j]);
-        if (g + 3 < ngroups) asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr[j] + static_cast<size_t>(g + 3) * GB));
+        if (g + 3 < ngroups)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr[j] + static_cast<size_t>(g + 3) * GB + pquart[j] * ASK));
     }
     return decode_store_two<FMT, 2, PIECES>(cur, prow, pquart, ring, lane);
 }
@@ -613,7 +619,7 @@ __global__ void __launch_bounds__(UG_THREADS, 1) umma_gemm_kernel(const __grid_c
         // packed bytes (requested two slabs before their first use; two groups further ahead the lines are
         // only asked into L2). Weights are read-only: no dependency wait. The loop is unrolled by two so the
         // sets are named statically and nothing is copied.
-        constexpr int GB = fmt_group_bytes(FMT);
+        constexpr int GB = fmt_group_bytes(FMT), ASK = fmt_prefetch_step(FMT);
         DecoderRing ring{smem, free_bar, full_bar, &abort_flag, a.status, stage_bytes, S, 0, 0,
                          (PAIR && rank == 1) ? cluster_map(smem_u32(&full_bar[0]), 0) : 0u};
         RawGroup set0[UG_PIECES], set1[UG_PIECES];
@@ -621,7 +627,8 @@ __global__ void __launch_bounds__(UG_THREADS, 1) umma_gemm_kernel(const __grid_c
         for (int j = 0; j < UG_PIECES; ++j) {
             fetch_group<FMT>(row_ptr[j], pquart[j], set0[j]);
             for (int ahead = 1; ahead <= 2; ++ahead)
-                if (ahead < ngroups) asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr[j] + static_cast<size_t>(ahead) * GB));
+                if (ahead < ngroups)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(row_ptr[j] + static_cast<size_t>(ahead) * GB + pquart[j] * ASK));
         }
         for (int g = 0; g < ngroups; g += 2) {
             if (!decode_group<FMT, UG_PIECES>(set0, set1, row_ptr, prow, pquart, g, ngroups, ring, lane)) break;
