@@ -180,16 +180,29 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) decode_attention_kernel(const 
         long long hint = position[0];
         if (hint >= horizon) hint = horizon - 1;
         const int esize = cache_dtype == B200Q_F32 ? 4 : 2;
+        const int lines = DH * esize / 128;               // of a cache row (1, 2 or 4)
         const size_t row0 = (static_cast<size_t>(bb) * hkv + kvh) * horizon;
         for (int gi = 0; gi < 16; ++gi) {
             const long long j0 = (static_cast<long long>(gi) * SPLIT * ATT_WARPS + part * ATT_WARPS + warp) * ATT_U;
             if (j0 > hint) break;
+            if constexpr (ATT_WARPS == 8) {
+                // many groups per warp: one request per 128-byte line, lane i takes line i of the group's key rows, then
+                // of its value rows (24-layer step of 16 sequences at position 512 2.39 -> 2.35 ms; with 32 warps and a
+                // group or two each the rows' own lanes are as good: one sequence 1.077 against 1.080 ms)
+                for (int i = lane; i < 2 * ATT_U * lines; i += 32) {
+                    const int u = (i / lines) % ATT_U;
+                    if (j0 + u > hint) continue;
+                    const size_t off = (row0 + j0 + u) * DH * esize + (i % lines) * 128;
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(i < ATT_U * lines ? k_cache : v_cache) + off));
+                }
+            } else {
 #pragma unroll
-            for (int u = 0; u < ATT_U; ++u) {
-                if (j0 + u > hint) break;
-                const size_t off = ((row0 + j0 + u) * DH + lane * EPL) * esize;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(k_cache) + off));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(v_cache) + off));
+                for (int u = 0; u < ATT_U; ++u) {
+                    if (j0 + u > hint) break;
+                    const size_t off = ((row0 + j0 + u) * DH + lane * EPL) * esize;
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(k_cache) + off));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(v_cache) + off));
+                }
             }
         }
     }
