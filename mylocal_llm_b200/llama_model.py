@@ -301,6 +301,8 @@ class ExternalLlamaModel:
         ptr = lambda x: ctypes.c_void_p(x.data_ptr())
         cache_id = _lib.DTYPE_ID[str(self.dtype).replace("torch.", "")]
         kc, vc = state.k[layer_index], state.v[layer_index]
+        if not (self._cache_fits(kc, b, state.horizon) and self._cache_fits(vc, b, state.horizon)):
+            raise ValueError("the KV cache does not fit the model")
         if os.environ.get("B200Q_ROPE_ATTENTION", "1") != "0":
             _lib.call("b200q_rope_attention", ptr(q2), ptr(k2), ptr(v2), q2.stride(0), k2.stride(0), v2.stride(0),
                       ptr(positions), ptr(self._cos), ptr(self._sin), int(self._cos.shape[0]), b, heads, kv_heads, dh,
@@ -339,13 +341,30 @@ class ExternalLlamaModel:
         _, logits = self._norm_linear(self.final_norm, residual, pending, self.lm_head, torch.float32)
         return logits
 
-    def _prefill_kernel_fits(self, t, horizon):
+    def _cache_fits(self, cache, b, horizon):
+        """Whether ``cache`` is one layer's keys or values as the kernels address them: ``[>= b, kv_heads, horizon,
+        head_dim]`` in the model's type, contiguous, on the model's device. They take a pointer and compute the rest from
+        the model's configuration, so a cache made for another model would be written past its end."""
+        cfg = self.config
+        return (cache.ndim == 4 and cache.shape[0] >= b
+                and tuple(cache.shape[1:]) == (cfg.num_key_value_heads, horizon, cfg.head_dim)
+                and cache.dtype == self.dtype and cache.is_contiguous() and cache.device == self.embed.data.device)
+
+    def _stacked_cache_fits(self, cache, b, horizon):
+        """The same for all layers in one allocation, of which the first ones are this model's."""
+        return (isinstance(cache, _torch().Tensor) and cache.ndim == 5 and cache.shape[0] >= self.config.num_hidden_layers
+                and cache.is_contiguous() and self._cache_fits(cache[0], b, horizon))
+
+    def _prefill_kernel_fits(self, b, t, state):
         """Whether a prompt of ``t`` tokens from position 0 on runs RoPE, cache store and causal attention as
         ``b200q_prefill_attention`` (BF16 caches, head_dim 64, horizon up to 1024); else the torch ops do."""
         cfg = self.config
         dt = _lib.DTYPE_ID[str(self.dtype).replace("torch.", "")]
-        return t > 1 and bool(_lib.load().b200q_prefill_attention_supported(
-            cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, t, horizon, dt, dt))
+        return (t > 1 and bool(_lib.load().b200q_prefill_attention_supported(
+            cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, t, state.horizon, dt, dt))
+            and all(self._stacked_cache_fits(part, b, state.horizon)
+                    or all(self._cache_fits(part[i], b, state.horizon) for i in range(cfg.num_hidden_layers))
+                    for part in (state.k, state.v)))
 
     def _prefill_attention(self, q2, k2, v2, b, t, state, layer_index):
         torch = _torch()
@@ -432,9 +451,11 @@ class ExternalLlamaModel:
         layer is not stacked, or the call's tensors are not what it takes."""
         torch = _torch()
         host = _lib.host()
-        if (host is None or self._host is False or not self.fused_decode or token_ids.dtype != torch.int64 or not token_ids.is_cuda
-                or not token_ids.numel() or not state.k.is_contiguous() or not state.v.is_contiguous() or state.k.dtype != self.dtype
-                or state.v.dtype != self.dtype):
+        device = self.embed.data.device
+        fits = lambda cache: self._stacked_cache_fits(cache, state.batch, state.horizon)
+        if (host is None or self._host is False or not self.fused_decode or token_ids.dtype != torch.int64
+                or token_ids.device != device or not token_ids.numel() or not fits(state.k) or not fits(state.v)
+                or state.position.dtype != torch.int64 or state.position.device != device):
             return None
         if self._host is None:
             cfg = self.config
@@ -463,14 +484,14 @@ class ExternalLlamaModel:
         if b != state.batch or t > state.horizon:
             raise ValueError("prompt does not fit the generation state")
         positions = mask = None
-        if self._prefill_kernel_fits(t, state.horizon):
+        if self._prefill_kernel_fits(b, t, state):
             native = self._native(token_ids, state)
             if native is not None:
                 logits = native.prefill(token_ids.contiguous(), state.k, state.v)
                 state.position.fill_(t)
                 state.length = t
                 return logits
-        if not self._prefill_kernel_fits(t, state.horizon):
+        else:
             positions = torch.arange(t, device=self.device)
             cols = torch.arange(state.horizon, device=self.device)
             mask = torch.where(cols[None, :] <= positions[:, None], 0.0, float("-inf")).float()

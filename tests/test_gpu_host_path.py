@@ -81,6 +81,39 @@ def test_llama_prompt_and_steps(cuda, monkeypatch, batch):
         assert torch.equal(a, b)
 
 
+def small_llama(layers=2, kv_heads=4, heads=4, seed=1):
+    return ExternalLlamaModel.synthetic(ExternalLlamaConfig(
+        vocab_size=512, hidden_size=256, intermediate_size=512, num_hidden_layers=layers, num_attention_heads=heads,
+        num_key_value_heads=kv_heads, head_dim=64, max_position_embeddings=64), seed=seed)
+
+
+@pytest.mark.parametrize("host", ["1", "0"])
+def test_caches_of_another_model_are_refused(cuda, monkeypatch, host):
+    torch = cuda
+    monkeypatch.setenv("B200Q_HOST", host)
+    model, ids = small_llama(), torch.randint(0, 512, (2, 5), device="cuda")
+    for other in (small_llama(layers=1), small_llama(kv_heads=1)):
+        state = other.create_generation_state(2, 32)
+        with pytest.raises((IndexError, RuntimeError)):
+            model.prefill(ids, state)
+        with pytest.raises((IndexError, ValueError)):
+            model.decode_one(ids[:, 0].contiguous(), state)
+    state = model.create_generation_state(2, 32)
+    state.k = state.k.half()
+    with pytest.raises(RuntimeError):
+        model.prefill(ids, state)
+    with pytest.raises(ValueError, match="KV cache"):
+        model.decode_one(ids[:, 0].contiguous(), state)
+    # more layers than the model has, or a strided cache in a prompt, stay what they were: fine
+    state, plain = small_llama(layers=3).create_generation_state(2, 32), model.create_generation_state(2, 32)
+    assert torch.equal(model.prefill(ids, state), model.prefill(ids, plain))
+    assert torch.equal(state.k[:2], plain.k) and not state.k[2].any()
+    strided = model.create_generation_state(2, 32)
+    strided.k, strided.v = (torch.zeros((2, 2, 4, 32, 128), dtype=torch.bfloat16, device="cuda")[..., :64] for _ in range(2))
+    model.prefill(ids, strided)
+    assert torch.equal(strided.v[0], plain.v[0]) and torch.equal(strided.k[0], plain.k[0])
+
+
 @pytest.mark.parametrize("fmt", ["Q8_0", "Q4_K", "Q6_K"])
 def test_embed_rows_is_the_gather_of_dequantised_rows(cuda, fmt):
     torch = cuda
