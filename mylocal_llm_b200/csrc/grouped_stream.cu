@@ -48,16 +48,16 @@ __global__ void __launch_bounds__(GS_THREADS, 1) grouped_gate_up_kernel(const Gr
         auto frag = [&](int, int s, int p) { return *reinterpret_cast<const uint4 *>(fp + s * 64 + p * plane); };
         auto sums = [&](int, int term) { return *reinterpret_cast<const uint32_t *>(xp + term * 16); };
         for (int sb = kpi; sb < a.nsb; sb += a.kp) {
-            SuperBlockRegs<Q5> r;
+            SuperBlockRegs<Q5> ra, rb;
             const uint8_t *tile;
             if (!stream.next(tile)) return false;
-            read_superblock_tile<Q5>(r, tile, lane);
+            read_superblock_tile<Q5>(ra, rb, tile, lane);
             stream.refill(lane);
-            superblock_mma<Q5, NTERMS, 1>(r, frag, sums, tig, tg);
+            superblock_mma<Q5, NTERMS, 1>(ra, rb, frag, sums, tig, tg);
             if (!stream.next(tile)) return false;
-            read_superblock_tile<Q5>(r, tile, lane);
+            read_superblock_tile<Q5>(ra, rb, tile, lane);
             stream.refill(lane);
-            superblock_mma<Q5, NTERMS, 1>(r, frag, sums, tig, tu);
+            superblock_mma<Q5, NTERMS, 1>(ra, rb, frag, sums, tig, tu);
             fp += a.kp * 512;
             xp += a.kp * 32;
         }

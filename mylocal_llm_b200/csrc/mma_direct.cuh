@@ -8,18 +8,14 @@
 // 48 KB of loads outstanding per SM.
 //
 // Arithmetic per super-block (256 weights of one row):
-//   * the lanes of a quad hold interleaved 4-byte words of a row's codes (word w of a 32-byte chunk belongs to lane
-//     w & 3), so the sixteen codes of one mma step come from one sub-block in every lane;
-//   * a masked nibble pair is used as it stands: 0..15 in the low (or bits 4..7 of the) mantissa bits of an FP16 is the
-//     subnormal q * 2^-24 (16 q * 2^-24), which the tensor cores multiply exactly - one AND per pair (plus one shift per
-//     word) instead of a byte permute and a packed FMA (Q5_K ORs the fifth bit in above the nibble);
-//   * two mma.m16n8k16 per sub-block, then one FP32 FMA per accumulator with the sub-block's 6-bit scale;
+//   * 4- or 5-bit codes -> FP16 pairs by byte permute; one packed FMA turns (1024+q) into sc*q
+//     exactly (sc*q <= 63*31 < 2048 is an integer FP16 holds exactly), so the 6-bit sub-block
+//     scales ride inside the A fragments and one accumulator serves the whole super-block;
+//   * 16 mma.m16n8k16 steps accumulate sum(sc*q*x) in FP32 for 16 rows x 8 tokens;
 //   * the minima go through one more mma: A = the eight 6-bit mins, B = per-sub-block activation
 //     sums (FP16 high + remainder), giving sum(mn * sum_x);
-//   * y += d * acc - dmin * acc_min in FP32, the powers of two folded into d and dmin.
+//   * y += d * acc - dmin * acc_min in FP32.
 // Every product is exact; roundings are the FP32 accumulations, as in the FP32-lane kernels.
-// What bounds it: instruction issue (about 230 per 16 x 256 tile of Q4_K, 394 with the packed FMA form; at HBM speed a
-// tile may take 400 issue slots of its scheduler).
 //
 // Activations are prepared once per CTA (or per expert segment) exactly as in mma_gemv.cuh:
 // power-of-two scaling per token, FP16 high (+ remainder for FP32 inputs), stored as B fragments.
@@ -86,6 +82,17 @@ __device__ __forceinline__ uint4 ldg128(const uint8_t *p) {
     return v;
 }
 
+__device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
 // The first product of a chain: no accumulator to clear and read.
 __device__ __forceinline__ void mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                               uint32_t b0, uint32_t b1) {
@@ -94,139 +101,130 @@ __device__ __forceinline__ void mma_f16_first(float (&d)[4], uint32_t a0, uint32
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// Packed bytes of two rows' (g, g + 8) super-block as seen by one lane. q[0..1] / q[2..3]: the code words of row g /
-// g + 8, word (c, j) of chunk c = bytes [32c + 16j + 4tig, +4) of the row's 128 code bytes, two chunks per uint4 in the
-// order (c, 0), (c, 1), (c + 1, 0), (c + 1, 1). h: Q5_K's fifth-bit bytes [16j + 4tig, +4), j = 0, 1, of the two rows.
+// Packed bytes of one row's super-block as seen by one lane.
 template <bool Q5>
 struct SuperBlockRegs {
-    uint4 hd[2];    // d, dmin, 12 scale/min bytes of each row
-    uint4 q[4];
-    uint2 h[2];
+    uint4 hd;   // d, dmin, 12 scale/min bytes
+    uint4 qa;   // quants bytes [16*tig, +16)        -> sub-blocks 2*(tig>>1), +1
+    uint4 qb;   // quants bytes [64 + 16*tig, +16)   -> sub-blocks 4 + 2*(tig>>1), +1
+    uint4 qh;   // Q5_K: high-bit bytes of elements [16*(tig&1), +16)
 };
 
-// In GGUF rows a lane's words lie 16 bytes apart: four lanes load 64 contiguous bytes (16 each) and exchange words, a
-// 4 x 4 transpose inside the quad.
-__device__ __forceinline__ void quad_exchange(uint32_t &lo, uint32_t &hi, bool upper, int mask) {
-    const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? lo : hi, mask);
-    if (upper) lo = got;
-    else hi = got;
-}
-__device__ __forceinline__ uint4 quad_transpose(uint4 v, int tig) {
-    quad_exchange(v.x, v.y, tig & 1, 1);
-    quad_exchange(v.z, v.w, tig & 1, 1);
-    quad_exchange(v.x, v.z, tig & 2, 2);
-    quad_exchange(v.y, v.w, tig & 2, 2);
-    return v;
-}
-
-// The transpose of a native block's words is left to the consumer (transpose_native): the shuffles would wait for the
-// loads here.
 template <bool Q5>
-__device__ __forceinline__ void load_superblock(SuperBlockRegs<Q5> &r, const uint8_t *row_a, const uint8_t *row_b, int tig) {
-    constexpr int CODES = Q5 ? 48 : 16;
-    r.hd[0] = ldg128(row_a);
-    r.hd[1] = ldg128(row_b);
-    r.q[0] = ldg128(row_a + CODES + 16 * tig);
-    r.q[1] = ldg128(row_a + CODES + 64 + 16 * tig);
-    r.q[2] = ldg128(row_b + CODES + 16 * tig);
-    r.q[3] = ldg128(row_b + CODES + 64 + 16 * tig);
+__device__ __forceinline__ void load_superblock(SuperBlockRegs<Q5> &r, const uint8_t *blk, int tig) {
+    r.hd = ldg128(blk);
     if (Q5) {
-        const uint32_t *ha = reinterpret_cast<const uint32_t *>(row_a + 16 + 4 * tig), *hb = reinterpret_cast<const uint32_t *>(row_b + 16 + 4 * tig);
-        r.h[0] = make_uint2(__ldg(ha), __ldg(ha + 4));
-        r.h[1] = make_uint2(__ldg(hb), __ldg(hb + 4));
+        r.qh = ldg128(blk + 16 + 16 * (tig & 1));
+        r.qa = ldg128(blk + 48 + 16 * tig);
+        r.qb = ldg128(blk + 112 + 16 * tig);
+    } else {
+        r.qh = make_uint4(0u, 0u, 0u, 0u);
+        r.qa = ldg128(blk + 16 + 16 * tig);
+        r.qb = ldg128(blk + 80 + 16 * tig);
     }
-}
-template <bool Q5>
-__device__ __forceinline__ void transpose_native(SuperBlockRegs<Q5> &r, int tig) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r.q[i] = quad_transpose(r.q[i], tig);
 }
 
 // Q4_K tile layout (device-side re-ordering of the GGUF bytes, same size): a tile holds the 16
 // super-blocks of 16 consecutive rows at one K position (2304 bytes):
 //   [0, 256)     the 16 rows' first 16 bytes (d, dmin, scales/mins), row r at 16*r
-//   [256, 2304)  four planes of 512 bytes with one 16-byte piece per lane (lane*16): planes 0/1 = the words q[0] / q[1]
-//                above of row g, planes 2/3 those of row g+8: what a lane of the native layout holds after its exchange
+//   [256, 2304)  four planes of 512 bytes with one 16-byte piece per lane (lane*16): planes 0/1 =
+//                bytes [16+16tig, +16) and [80+16tig, +16) of row g's block, planes 2/3 the same of
+//                row g+8 - exactly the pieces load_superblock() fetches, so the arithmetic is shared.
 // Tiles are ordered (row group, super-block): a warp instruction reads 512 contiguous bytes.
 constexpr int Q4T_TILE_BYTES = 2304;
-// Q5_K the same way (2816 bytes, the size of 16 native blocks): the 16 headers, then two planes of 256 bytes with the
-// rows' fifth-bit words (lane*8: words j = 0, 1 of row g, then of row g + 8), then the four quant planes:
+// Q5_K the same way (2816 bytes, the size of 16 native blocks): the 16 headers, then the rows' 32 bytes of
+// fifth bits (row r at 256 + 32 r; a lane reads the half its elements need, lanes tig and tig + 2 the same
+// one), then the four quant planes:
 //   [0, 256) headers | [256, 768) fifth bits | [768, 2816) planes 0/1 (row g), 2/3 (row g + 8), lane * 16 each
 constexpr int Q5T_TILE_BYTES = 2816;
 template <bool Q5>
 __host__ __device__ constexpr int direct_tile_bytes() { return Q5 ? Q5T_TILE_BYTES : Q4T_TILE_BYTES; }
 
-__device__ __forceinline__ uint2 ldg64(const uint8_t *p) {
-    uint2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
-
 template <bool Q5>
-__device__ __forceinline__ void load_superblock_tiled(SuperBlockRegs<Q5> &r, const uint8_t *tile, int lane) {
-    constexpr int CODES = Q5 ? 768 : 256;
-    const int g = lane >> 2;
-    r.hd[0] = ldg128(tile + 16 * g);
-    r.hd[1] = ldg128(tile + 16 * (g + 8));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r.q[i] = ldg128(tile + CODES + 512 * i + lane * 16);
+__device__ __forceinline__ void load_superblock_tiled(SuperBlockRegs<Q5> &ra, SuperBlockRegs<Q5> &rb,
+                                                      const uint8_t *tile, int lane) {
+    const int g = lane >> 2, tig = lane & 3;
+    ra.hd = ldg128(tile + 16 * g);
+    rb.hd = ldg128(tile + 16 * (g + 8));
     if (Q5) {
-        r.h[0] = ldg64(tile + 256 + lane * 8);
-        r.h[1] = ldg64(tile + 512 + lane * 8);
+        ra.qh = ldg128(tile + 256 + 32 * g + 16 * (tig & 1));
+        rb.qh = ldg128(tile + 256 + 32 * (g + 8) + 16 * (tig & 1));
+        ra.qa = ldg128(tile + 768 + lane * 16);
+        ra.qb = ldg128(tile + 1280 + lane * 16);
+        rb.qa = ldg128(tile + 1792 + lane * 16);
+        rb.qb = ldg128(tile + 2304 + lane * 16);
+    } else {
+        ra.qa = ldg128(tile + 256 + lane * 16);
+        ra.qb = ldg128(tile + 768 + lane * 16);
+        rb.qa = ldg128(tile + 1280 + lane * 16);
+        rb.qb = ldg128(tile + 1792 + lane * 16);
+        ra.qh = rb.qh = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
 // The same from a tile in shared memory.
 template <bool Q5>
-__device__ __forceinline__ void read_superblock_tile(SuperBlockRegs<Q5> &r, const uint8_t *tile, int lane) {
+__device__ __forceinline__ void read_superblock_tile(SuperBlockRegs<Q5> &ra, SuperBlockRegs<Q5> &rb, const uint8_t *tile,
+                                                     int lane) {
     constexpr int CODES = Q5 ? 768 : 256;
-    const int g = lane >> 2;
-    r.hd[0] = *reinterpret_cast<const uint4 *>(tile + 16 * g);
-    r.hd[1] = *reinterpret_cast<const uint4 *>(tile + 16 * (g + 8));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r.q[i] = *reinterpret_cast<const uint4 *>(tile + CODES + 512 * i + lane * 16);
-    if (Q5) {
-        r.h[0] = *reinterpret_cast<const uint2 *>(tile + 256 + lane * 8);
-        r.h[1] = *reinterpret_cast<const uint2 *>(tile + 512 + lane * 8);
-    }
+    const int g = lane >> 2, tig = lane & 3;
+    auto at = [&](int byte) { return *reinterpret_cast<const uint4 *>(tile + byte); };
+    ra.hd = at(16 * g);
+    rb.hd = at(16 * (g + 8));
+    ra.qh = Q5 ? at(256 + 32 * g + 16 * (tig & 1)) : make_uint4(0u, 0u, 0u, 0u);
+    rb.qh = Q5 ? at(256 + 32 * (g + 8) + 16 * (tig & 1)) : make_uint4(0u, 0u, 0u, 0u);
+    ra.qa = at(CODES + lane * 16);
+    ra.qb = at(CODES + 512 + lane * 16);
+    rb.qa = at(CODES + 1024 + lane * 16);
+    rb.qb = at(CODES + 1536 + lane * 16);
 }
 
-// Scales of one row: the eight 6-bit sub-block scales as FP16 subnormal pairs widened to FP32 (sc * 2^-24), the lane's
-// pair of minima as FP16 subnormals (A operand of the min product), d and dmin with the powers of two that undo both
-// subnormal forms (2^24 of the codes, 2^24 of the scales; 2^24 of the minima and the 64 of MD_XS_SCALE).
+// Scales of one row for this lane: the four sub-blocks its quant bytes belong to, as FP16 pairs
+// (sc, sc) and (-1024*sc, -1024*sc); plus the A operand of the min product and d, dmin.
 struct RowScales {
-    float sc[8];
-    uint32_t mins;      // (mn[2*tig], mn[2*tig+1])
+    uint32_t sc[4];     // [span A low, span A high, span B low, span B high]
+    uint32_t nsc[4];
+    uint32_t mins;      // (mn[2*tig], mn[2*tig+1]) as exact FP16 pair
     float d, dmin;
 };
 
 __device__ __forceinline__ RowScales decode_scales(const uint4 &hd, int tig) {
     RowScales s;
-    const __half2 dd = *reinterpret_cast<const __half2 *>(&hd.x);
-    s.d = __low2float(dd) * 281474976710656.0f;       // 2^48
-    s.dmin = __high2float(dd) * 1073741824.0f;        // 2^30
+    s.d = half_bits_to_float(hd.x & 0xffffu);
+    s.dmin = half_bits_to_float(hd.x >> 16);
     const uint32_t sc_lo = hd.y & 0x3f3f3f3fu;                                       // sub-blocks 0..3
     const uint32_t sc_hi = (hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u);        // sub-blocks 4..7
+    const uint32_t mn_lo = hd.z & 0x3f3f3f3fu;
+    const uint32_t mn_hi = ((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u);
+    const int sh = (tig >> 1) * 16;   // sub-block pair 2*(tig>>1) inside each word
+    const uint32_t a2 = sc_lo >> sh, b2 = sc_hi >> sh;   // low two bytes: the lane's two sub-blocks
+    const uint32_t bias = 0x64006400u, k1024 = 0xe400e400u;   // 1024, -1024 as FP16 pairs
+    s.sc[0] = hsub2_u32(__byte_perm(a2, 0x64646464u, 0x4040), bias);
+    s.sc[1] = hsub2_u32(__byte_perm(a2, 0x64646464u, 0x4141), bias);
+    s.sc[2] = hsub2_u32(__byte_perm(b2, 0x64646464u, 0x4040), bias);
+    s.sc[3] = hsub2_u32(__byte_perm(b2, 0x64646464u, 0x4141), bias);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t pair = __byte_perm(i < 2 ? sc_lo : sc_hi, 0u, (i & 1) ? 0x4342 : 0x4140);
-        const __half2 h = *reinterpret_cast<const __half2 *>(&pair);
-        s.sc[2 * i] = __low2float(h);
-        s.sc[2 * i + 1] = __high2float(h);
-    }
-    const uint32_t mn = (tig & 2) ? ((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u) : hd.z & 0x3f3f3f3fu;
-    s.mins = __byte_perm(mn, 0u, (tig & 1) ? 0x4342 : 0x4140);
+    for (int i = 0; i < 4; ++i) s.nsc[i] = hmul2_u32(s.sc[i], k1024);
+    const uint32_t mw = ((tig & 2) ? mn_hi : mn_lo) >> ((tig & 1) * 16);
+    s.mins = hsub2_u32(__byte_perm(mw, 0x64646464u, 0x4140), bias);
     return s;
 }
 
 
 // ---------------------------------------------------------------------------------------------
-// Activation fragments for the direct kernel, in natural order: fragment f holds positions 16f .. 16f + 15; for lane
-// (g = lane>>2, tig = lane&3) token g at positions 16f + 4 tig + {0,2 -> b0 ; 1,3 -> b1}, the positions of the codes in
-// that lane's word. The two fragments of a sub-block lie side by side (one 16-byte load): uint2 entry
-// ((f >> 1) * 32 + lane) * 2 + (f & 1).
+// Activation fragments for the direct kernel. Fragment (sb, fi) with fi = (X*2 + nib)*4 + j holds,
+// for lane (g = lane>>2, tig = lane&3), token g at positions
+//   256*sb + 32*(4*X + 2*(tig>>1) + nib) + 16*(tig&1) + 4*j + {0,2 -> b0 ; 1,3 -> b1}
+// which are exactly the positions of the codes that lane extracts from word j of its quant bytes. Fragments f = sb*16 + fi
+// lie in pairs (one 16-byte load): uint2 entry ((f >> 1) * 32 + lane) * 2 + (f & 1), direct_entry().
 // xsfrag (sb, term) holds (sum_x[sub 2*tig], sum_x[sub 2*tig+1]) / 64 for token g.
 // ---------------------------------------------------------------------------------------------
+// Entry of the chunk of four positions that starts at p, token slot t.
+__device__ __forceinline__ int direct_entry(int p, int t) {
+    const int sub = (p >> 5) & 7, tig = 2 * ((sub >> 1) & 1) + ((p >> 4) & 1);
+    const int f = (p >> 8) * 16 + ((sub >> 2) * 2 + (sub & 1)) * 4 + ((p >> 2) & 3);
+    return ((f >> 1) * 32 + 4 * t + tig) * 2 + (f & 1);
+}
 // Four consecutive activations starting at element index e (a multiple of 4) as floats.
 // `vec_ok` tells whether the tensor allows aligned vector loads.
 __device__ __forceinline__ void load4(const void *x, int x_dtype, size_t e, bool vec_ok, float (&v)[4]) {
@@ -314,7 +312,8 @@ __device__ __forceinline__ void prepare_direct(RowFn row_of, int m_tokens, int k
         tok_scale[8 + tid] = 1.0f / s;
     }
     named_barrier_sync(BARRIER, THREADS);
-    // 2. scale, split, store: the chunk at position p of token t is the entry of fragment f = p>>4, lane 4t + ((p>>2)&3)
+    // 2. scale, split, store: the chunk at position p of token t is fragment entry (f, lane 4t+tig) with
+    //    sb = p>>8, sub = (p>>5)&7, X = sub>>2, nib = sub&1, tig = 2*((sub>>1)&1) + ((p>>4)&1), j = (p>>2)&3
     auto store_chunk = [&](int c0, const float (&v)[4]) {
         const int t = c0 / chunks_per_token;
         const int p = (c0 + lane - t * chunks_per_token) * 4;
@@ -332,7 +331,7 @@ __device__ __forceinline__ void prepare_direct(RowFn row_of, int m_tokens, int k
             }
         }
         const int sb = p >> 8, sub = (p >> 5) & 7;
-        const int entry = ((p >> 5) * 32 + 4 * t + ((p >> 2) & 3)) * 2 + ((p >> 4) & 1);
+        const int entry = direct_entry(p, t);
         uint2 out;
         out.x = static_cast<uint32_t>(__half_as_ushort(hi[0])) | (static_cast<uint32_t>(__half_as_ushort(hi[2])) << 16);
         out.y = static_cast<uint32_t>(__half_as_ushort(hi[1])) | (static_cast<uint32_t>(__half_as_ushort(hi[3])) << 16);
@@ -491,7 +490,8 @@ __device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k
         tok_scale[8 + tid] = 1.0f / s;
     }
     named_barrier_sync(BARRIER, THREADS);
-    // 2. scale, split, store: the chunk at position p of token t is the entry of fragment f = p>>4, lane 4t + ((p>>2)&3)
+    // 2. scale, split, store: with the sums in this kernel's order, else in the natural one of q6k_tiled.cuh (fragment
+    //    f = p>>4, lane 4t + ((p>>2)&3))
     auto store_chunk = [&](int c0, const RawChunk<NTERMS> &r) {
         const int t = token_of(c0);
         const int p = (c0 + lane - t * chunks_per_token) * 4;
@@ -512,7 +512,7 @@ __device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k
                 if (SUMS) sum += __half2float(l);
             }
         }
-        const int entry = ((p >> 5) * 32 + 4 * t + ((p >> 2) & 3)) * 2 + ((p >> 4) & 1);
+        const int entry = SUMS ? direct_entry(p, t) : ((p >> 5) * 32 + 4 * t + ((p >> 2) & 3)) * 2 + ((p >> 4) & 1);
         bfrag[entry] = make_uint2(hi[0] | (static_cast<uint32_t>(hi[2]) << 16), hi[1] | (static_cast<uint32_t>(hi[3]) << 16));
         if (NTERMS == 2)
             bfrag[nfrag * 32 + entry] = make_uint2(lo[0] | (static_cast<uint32_t>(lo[2]) << 16), lo[1] | (static_cast<uint32_t>(lo[3]) << 16));
@@ -550,7 +550,7 @@ __device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k
 // Token images. In the grouped gate/up launch every expert segment needs the fragments of its tokens, and
 // a token routed to k experts would be converted k times (at 64 tokens: 704 conversions of 64 distinct
 // rows, each a chain of dependent loads, a reduction and three barriers). token_image_kernel runs
-// prepare_tokens once per token - same code, so the same bits - and stores what it wrote for token slot 0:
+// prepare_direct once per token - same code, so the same bits - and stores what it wrote for token slot 0:
 //   [NTERMS * nfrag * 32 bytes]  the slot's four lanes (tig 0..3, 16 bytes each) of every pair of fragments
 //   [nsb * 2 * 16 bytes]         the slot's four words of every activation-sum row
 //   [16 bytes]                   scale, inverse scale
@@ -606,83 +606,76 @@ __device__ __forceinline__ void gather_token_images(const uint8_t *images, int i
     }
 }
 
-// One super-block of rows (g, g+8): tot += d * sum_s sc_s * (codes_s . x_s) - dmin * sum_s mn_s * sum_x_s.
+// 16 mma steps of one super-block for rows (g, g+8): acc += sum(sc*q*x); accm += sum(mn * sum_x/64).
 // With NT token tiles (8 tokens each; their fragments `btile` / `xtile` entries apart) every decoded
 // A operand is multiplied into each tile, so the decode cost is paid once per 8*NT tokens; the
 // arithmetic of one token does not depend on NT.
-// frag(nt, s, plane): the lane's 16 bytes of sub-block s (its two fragments) in plane 0 (FP16 high parts) or 1
-// (remainders) of token tile nt; sums(nt, term): the lane's word of the activation sums.
+// frag(nt, pair, plane): the lane's 16 bytes of fragments 2 pair, 2 pair + 1 of the super-block in plane 0 (FP16 high
+// parts) or 1 (remainders) of token tile nt; sums(nt, term): the lane's word of the activation sums.
 template <bool Q5, int NTERMS, int NT, typename FragFn, typename SumFn>
-__device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &r, const FragFn frag, const SumFn sums, int tig,
-                                               float (&tot)[NT][4]) {
-    const RowScales sa = decode_scales(r.hd[0], tig), sbk = decode_scales(r.hd[1], tig);
-    // even sub-blocks (low nibbles) and odd ones (high nibbles, 16 times the code) in accumulators of their own
-    float even[NT][4], odd[NT][4];
+__device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &ra, const SuperBlockRegs<Q5> &rb, const FragFn frag,
+                                               const SumFn sums, int tig, float (&tot)[NT][4]) {
+    const RowScales sa = decode_scales(ra.hd, tig), sbk = decode_scales(rb.hd, tig);
+    float acc[NT][4], acc2[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) even[nt][i] = odd[nt][i] = 0.f;
-    const uint32_t wa[8] = {r.q[0].x, r.q[0].y, r.q[0].z, r.q[0].w, r.q[1].x, r.q[1].y, r.q[1].z, r.q[1].w};
-    const uint32_t wb[8] = {r.q[2].x, r.q[2].y, r.q[2].z, r.q[2].w, r.q[3].x, r.q[3].y, r.q[3].z, r.q[3].w};
-    const uint32_t ha[2] = {r.h[0].x, r.h[0].y}, hb[2] = {r.h[1].x, r.h[1].y};
-    // fifth bits of sub-block s, bytes 0 and 2 (byte = 0) or 1 and 3 (byte = 1) of a high-bit word, at bit 4 (odd
-    // sub-blocks: bit 8, above a nibble in bits 4..7)
-    auto fifth = [](uint32_t h, int s, int byte) {
-        const int to = (s & 1) ? 8 : 4, from = s + 8 * byte;
-        const uint32_t v = from >= to ? h >> (from - to) : h << (to - from);
-        return v & ((s & 1) ? 0x01000100u : 0x00100010u);
-    };
+        for (int i = 0; i < 4; ++i) acc[nt][i] = acc2[nt][i] = 0.f;
+    const uint32_t qa_a[4] = {ra.qa.x, ra.qa.y, ra.qa.z, ra.qa.w}, qb_a[4] = {ra.qb.x, ra.qb.y, ra.qb.z, ra.qb.w};
+    const uint32_t qa_b[4] = {rb.qa.x, rb.qa.y, rb.qa.z, rb.qa.w}, qb_b[4] = {rb.qb.x, rb.qb.y, rb.qb.z, rb.qb.w};
+    const uint32_t qh_a[4] = {ra.qh.x, ra.qh.y, ra.qh.z, ra.qh.w}, qh_b[4] = {rb.qh.x, rb.qh.y, rb.qh.z, rb.qh.w};
+    const int pair = tig >> 1;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const uint32_t a[2] = {wa[2 * c], wa[2 * c + 1]}, b[2] = {wb[2 * c], wb[2 * c + 1]};
-        const uint32_t a8[2] = {a[0] >> 8, a[1] >> 8}, b8[2] = {b[0] >> 8, b[1] >> 8};
+    for (int X = 0; X < 2; ++X) {
 #pragma unroll
         for (int nib = 0; nib < 2; ++nib) {
-            const int s = 2 * c + nib;
-            const uint32_t mask = nib ? 0x00f000f0u : 0x000f000fu;
-            uint32_t f[2][4];
+            const int si = X * 2 + nib;
+            // Q5_K: bit (sub-block index) of the high-bit byte, moved to bit 4 of the code
+            const int sub = 4 * X + 2 * pair + nib;
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                f[j][0] = a[j] & mask;
-                f[j][1] = b[j] & mask;
-                f[j][2] = a8[j] & mask;
-                f[j][3] = b8[j] & mask;
-                if (Q5) {
-                    f[j][0] |= fifth(ha[j], s, 0);
-                    f[j][1] |= fifth(hb[j], s, 0);
-                    f[j][2] |= fifth(ha[j], s, 1);
-                    f[j][3] |= fifth(hb[j], s, 1);
-                }
-            }
+            for (int jp = 0; jp < 2; ++jp) {
+                uint32_t f[2][4];                            // A operands of words 2 jp, 2 jp + 1
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                float acc[4];
-                const uint4 v = frag(nt, s, 0);
-                mma_f16_first(acc, f[0][0], f[0][1], f[0][2], f[0][3], v.x, v.y);
-                mma_f16(acc, f[1][0], f[1][1], f[1][2], f[1][3], v.z, v.w);
-                if (NTERMS == 2) {
-                    const uint4 u = frag(nt, s, 1);
-                    mma_f16(acc, f[0][0], f[0][1], f[0][2], f[0][3], u.x, u.y);
-                    mma_f16(acc, f[1][0], f[1][1], f[1][2], f[1][3], u.z, u.w);
+                for (int jj = 0; jj < 2; ++jj) {
+                    const int j = 2 * jp + jj;
+                    const uint32_t wa = X ? qb_a[j] : qa_a[j], wb = X ? qb_b[j] : qa_b[j];
+                    uint32_t va = nib ? (wa >> 4) & 0x0f0f0f0fu : wa & 0x0f0f0f0fu;
+                    uint32_t vb = nib ? (wb >> 4) & 0x0f0f0f0fu : wb & 0x0f0f0f0fu;
+                    if (Q5) {
+                        va |= ((qh_a[j] >> sub) << 4) & 0x10101010u;
+                        vb |= ((qh_b[j] >> sub) << 4) & 0x10101010u;
+                    }
+                    f[jj][0] = hfma2_u32(__byte_perm(va, 0x64646464u, 0x4240), sa.sc[si], sa.nsc[si]);
+                    f[jj][1] = hfma2_u32(__byte_perm(vb, 0x64646464u, 0x4240), sbk.sc[si], sbk.nsc[si]);
+                    f[jj][2] = hfma2_u32(__byte_perm(va, 0x64646464u, 0x4341), sa.sc[si], sa.nsc[si]);
+                    f[jj][3] = hfma2_u32(__byte_perm(vb, 0x64646464u, 0x4341), sbk.sc[si], sbk.nsc[si]);
                 }
-                float (&dst)[4] = nib ? odd[nt] : even[nt];
-                dst[0] = fmaf(sa.sc[s], acc[0], dst[0]);
-                dst[1] = fmaf(sa.sc[s], acc[1], dst[1]);
-                dst[2] = fmaf(sbk.sc[s], acc[2], dst[2]);
-                dst[3] = fmaf(sbk.sc[s], acc[3], dst[3]);
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    float (&c)[4] = X ? acc2[nt] : acc[nt];
+                    const uint4 h = frag(nt, si * 2 + jp, 0);
+                    uint4 l = make_uint4(0u, 0u, 0u, 0u);
+                    if (NTERMS == 2) l = frag(nt, si * 2 + jp, 1);
+                    mma_f16(c, f[0][0], f[0][1], f[0][2], f[0][3], h.x, h.y);
+                    if (NTERMS == 2) mma_f16(c, f[0][0], f[0][1], f[0][2], f[0][3], l.x, l.y);
+                    mma_f16(c, f[1][0], f[1][1], f[1][2], f[1][3], h.z, h.w);
+                    if (NTERMS == 2) mma_f16(c, f[1][0], f[1][1], f[1][2], f[1][3], l.z, l.w);
+                }
             }
         }
     }
+    const float ma = sa.dmin * 64.0f, mb = sbk.dmin * 64.0f;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        float accm[4];
-        mma_f16_first(accm, sa.mins, sbk.mins, 0u, 0u, sums(nt, 0), 0u);
-        mma_f16(accm, sa.mins, sbk.mins, 0u, 0u, sums(nt, 1), 0u);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float sum = fmaf(0.0625f, odd[nt][i], even[nt][i]);
-            tot[nt][i] = fmaf(i < 2 ? sa.d : sbk.d, sum, fmaf(i < 2 ? -sa.dmin : -sbk.dmin, accm[i], tot[nt][i]));
-        }
+        for (int i = 0; i < 4; ++i) acc[nt][i] += acc2[nt][i];
+        float accm[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_f16(accm, sa.mins, sbk.mins, 0u, 0u, sums(nt, 0), 0u);
+        mma_f16(accm, sa.mins, sbk.mins, 0u, 0u, sums(nt, 1), 0u);
+        tot[nt][0] = fmaf(sa.d, acc[nt][0], fmaf(-ma, accm[0], tot[nt][0]));
+        tot[nt][1] = fmaf(sa.d, acc[nt][1], fmaf(-ma, accm[1], tot[nt][1]));
+        tot[nt][2] = fmaf(sbk.d, acc[nt][2], fmaf(-mb, accm[2], tot[nt][2]));
+        tot[nt][3] = fmaf(sbk.d, acc[nt][3], fmaf(-mb, accm[3], tot[nt][3]));
     }
 }
 
@@ -784,22 +777,23 @@ __device__ __forceinline__ void mma_direct_body(const DirectArgs &a, const Stage
     };
     // item -> byte offset from the block pointers, and stream
     const int sb_step_bytes = a.kp * (a.tiled ? direct_tile_bytes<Q5>() : QB);
-    auto issue_item = [&](const BlockPtrs &p, int item, SuperBlockRegs<Q5> &r) {
+    auto issue_item = [&](const BlockPtrs &p, int item, SuperBlockRegs<Q5> &ra, SuperBlockRegs<Q5> &rb) {
         const int stream = DUAL ? (item & 1) : 0;
         const size_t off = static_cast<size_t>(DUAL ? (item >> 1) : item) * sb_step_bytes;
         if (a.tiled) {
-            load_superblock_tiled<Q5>(r, (stream ? p.b_lo : p.a_lo) + off, lane);
+            load_superblock_tiled<Q5>(ra, rb, (stream ? p.b_lo : p.a_lo) + off, lane);
             return;
         }
-        load_superblock<Q5>(r, (stream ? p.b_lo : p.a_lo) + off, (stream ? p.b_hi : p.a_hi) + off, tig);
+        load_superblock<Q5>(ra, (stream ? p.b_lo : p.a_lo) + off, tig);
+        load_superblock<Q5>(rb, (stream ? p.b_hi : p.a_hi) + off, tig);
     };
 
     int unit_i = static_cast<int>(blk_begin / blocks_per_unit);
     int bi = static_cast<int>(blk_begin - static_cast<long long>(unit_i) * blocks_per_unit);
     BlockPtrs cur_p = block_ptrs(unit_i, bi * rows_per_block), nxt_p = cur_p;
 
-    SuperBlockRegs<Q5> cur, nxt;
-    if (items_per_block > 0) issue_item(cur_p, 0, nxt);
+    SuperBlockRegs<Q5> cur_a, cur_b, nxt_a, nxt_b;
+    if (items_per_block > 0) issue_item(cur_p, 0, nxt_a, nxt_b);
 
     int m_tokens = a.m;
     int seg_begin = 0, cur_unit = -1, last_single = (MODE == 2) ? gp.prepared_row : -1;
@@ -861,19 +855,19 @@ __device__ __forceinline__ void mma_direct_body(const DirectArgs &a, const Stage
             for (int i = 0; i < 4; ++i) tot_a[nt][i] = tot_b[nt][i] = 0.f;
         for (int item = 0; item < items_per_block; ++item) {
             // (copying the prefetched registers measured faster than alternating two register sets)
-            cur = nxt;
+            cur_a = nxt_a;
+            cur_b = nxt_b;
             // request the next item (same block, or the first item of the next block)
-            if (item + 1 < items_per_block) issue_item(cur_p, item + 1, nxt);
-            else if (has_next) issue_item(nxt_p, 0, nxt);
-            if (!a.tiled) transpose_native<Q5>(cur, tig);
+            if (item + 1 < items_per_block) issue_item(cur_p, item + 1, nxt_a, nxt_b);
+            else if (has_next) issue_item(nxt_p, 0, nxt_a, nxt_b);
             const int stream = DUAL ? (item & 1) : 0;
             const int sb = kpi + (DUAL ? (item >> 1) : item) * a.kp;
             const uint4 *bf = reinterpret_cast<const uint4 *>(bfrag) + sb * 256 + lane;
             const uint32_t *xf = xsfrag + sb * 64 + lane;
-            auto frag = [&](int nt, int s, int plane) { return bf[nt * (btile >> 1) + plane * nfrag * 16 + s * 32]; };
+            auto frag = [&](int nt, int p, int plane) { return bf[nt * (btile >> 1) + plane * nfrag * 16 + p * 32]; };
             auto sums = [&](int nt, int term) { return xf[nt * xtile + term * 32]; };
-            if (stream == 0) superblock_mma<Q5, NTERMS, NT>(cur, frag, sums, tig, tot_a);
-            else superblock_mma<Q5, NTERMS, NT>(cur, frag, sums, tig, tot_b);
+            if (stream == 0) superblock_mma<Q5, NTERMS, NT>(cur_a, cur_b, frag, sums, tig, tot_a);
+            else superblock_mma<Q5, NTERMS, NT>(cur_a, cur_b, frag, sums, tig, tot_b);
         }
 
         // combine the kp partial sums of each row group in fixed order:

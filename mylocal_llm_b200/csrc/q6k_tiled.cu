@@ -71,37 +71,55 @@ __global__ void __launch_bounds__(256) q6k_untile_kernel(const uint8_t *src, uin
     blk[209] = in[Q6T_D_OFF + 2 * row + 1];
 }
 
-// Q4_K / Q5_K <-> tile layout: one thread per (tile, lane). A lane moves four 16-byte pieces of its two rows' codes; in
-// between the quad exchanges words (its own inverse), so both sides are read and written in whole pieces. Q5_K adds the
-// fifth-bit words; lanes 0-15 also move one row's first 16 bytes. FORWARD: native -> tiled.
-template <bool Q5, bool FORWARD>
-__global__ void __launch_bounds__(256) q45k_retile_kernel(const uint8_t *src, uint8_t *dst, long long tiles, int nsb) {
-    constexpr int QB = Q5 ? 176 : 144, CODES = Q5 ? 768 : 256, NATIVE_CODES = Q5 ? 48 : 16;
+// Q4_K <-> tile layout: a permutation of 16-byte pieces. One thread per (tile, lane): four pieces of
+// its two rows; lanes 0-15 also move one row's first 16 bytes. FORWARD: native -> tiled.
+template <bool FORWARD>
+__global__ void __launch_bounds__(256) q4k_retile_kernel(const uint8_t *src, uint8_t *dst, long long tiles, int nsb) {
     const long long idx = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
     const long long tile = idx >> 5;
-    if (tile >= tiles) return;                                   // whole warps
+    if (tile >= tiles) return;
     const int lane = static_cast<int>(idx & 31), g = lane >> 2, tig = lane & 3;
     const long long group = tile / nsb;
     const int sb = static_cast<int>(tile - group * nsb);
-    const size_t row_bytes = static_cast<size_t>(nsb) * QB;
-    const size_t tile_off = static_cast<size_t>(tile) * direct_tile_bytes<Q5>();
-    auto native_at = [&](int row, int byte) { return (static_cast<size_t>(group) * 16 + row) * row_bytes + static_cast<size_t>(sb) * QB + byte; };
-    auto move = [&](size_t native_off, size_t tiled_off, bool exchange) {
-        uint4 v = *reinterpret_cast<const uint4 *>(src + (FORWARD ? native_off : tiled_off));
-        if (exchange) v = quad_transpose(v, tig);
-        *reinterpret_cast<uint4 *>(dst + (FORWARD ? tiled_off : native_off)) = v;
+    const size_t row_bytes = static_cast<size_t>(nsb) * 144;
+    const size_t tile_off = static_cast<size_t>(tile) * Q4T_TILE_BYTES;
+    auto native_at = [&](int row, int byte) { return (static_cast<size_t>(group) * 16 + row) * row_bytes + static_cast<size_t>(sb) * 144 + byte; };
+    auto move = [&](size_t native_off, size_t tiled_off) {
+        if (FORWARD) *reinterpret_cast<uint4 *>(dst + tiled_off) = *reinterpret_cast<const uint4 *>(src + native_off);
+        else *reinterpret_cast<uint4 *>(dst + native_off) = *reinterpret_cast<const uint4 *>(src + tiled_off);
     };
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-        move(native_at(g + 8 * (p >> 1), NATIVE_CODES + 64 * (p & 1) + 16 * tig), tile_off + CODES + 512 * p + lane * 16, true);
-    if (Q5) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const size_t n = native_at(g + 8 * (i >> 1), 16 + 16 * (i & 1) + 4 * tig), t = tile_off + 256 + 256 * (i >> 1) + lane * 8 + 4 * (i & 1);
-            *reinterpret_cast<uint32_t *>(dst + (FORWARD ? t : n)) = *reinterpret_cast<const uint32_t *>(src + (FORWARD ? n : t));
-        }
+    move(native_at(g, 16 + 16 * tig), tile_off + 256 + lane * 16);
+    move(native_at(g, 80 + 16 * tig), tile_off + 768 + lane * 16);
+    move(native_at(g + 8, 16 + 16 * tig), tile_off + 1280 + lane * 16);
+    move(native_at(g + 8, 80 + 16 * tig), tile_off + 1792 + lane * 16);
+    if (lane < 16) move(native_at(lane, 0), tile_off + 16 * lane);
+}
+
+// Q5_K <-> tile layout: as Q4_K, plus the rows' 32 bytes of fifth bits (lanes 0-15 move a row's two halves).
+template <bool FORWARD>
+__global__ void __launch_bounds__(256) q5k_retile_kernel(const uint8_t *src, uint8_t *dst, long long tiles, int nsb) {
+    const long long idx = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+    const long long tile = idx >> 5;
+    if (tile >= tiles) return;
+    const int lane = static_cast<int>(idx & 31), g = lane >> 2, tig = lane & 3;
+    const long long group = tile / nsb;
+    const int sb = static_cast<int>(tile - group * nsb);
+    const size_t row_bytes = static_cast<size_t>(nsb) * 176;
+    const size_t tile_off = static_cast<size_t>(tile) * Q5T_TILE_BYTES;
+    auto native_at = [&](int row, int byte) { return (static_cast<size_t>(group) * 16 + row) * row_bytes + static_cast<size_t>(sb) * 176 + byte; };
+    auto move = [&](size_t native_off, size_t tiled_off) {
+        if (FORWARD) *reinterpret_cast<uint4 *>(dst + tiled_off) = *reinterpret_cast<const uint4 *>(src + native_off);
+        else *reinterpret_cast<uint4 *>(dst + native_off) = *reinterpret_cast<const uint4 *>(src + tiled_off);
+    };
+    move(native_at(g, 48 + 16 * tig), tile_off + 768 + lane * 16);
+    move(native_at(g, 112 + 16 * tig), tile_off + 1280 + lane * 16);
+    move(native_at(g + 8, 48 + 16 * tig), tile_off + 1792 + lane * 16);
+    move(native_at(g + 8, 112 + 16 * tig), tile_off + 2304 + lane * 16);
+    if (lane < 16) {
+        move(native_at(lane, 0), tile_off + 16 * lane);
+        move(native_at(lane, 16), tile_off + 256 + 32 * lane);
+        move(native_at(lane, 32), tile_off + 256 + 32 * lane + 16);
     }
-    if (lane < 16) move(native_at(lane, 0), tile_off + 16 * lane, false);
 }
 
 using Q6Fn = void (*)(const Q6TiledArgs);
@@ -368,10 +386,10 @@ static int q4k_retile_common(const void *src, void *dst, long long rows, int k, 
     const long long tiles = rows / 16 * nsb;
     const unsigned blocks = static_cast<unsigned>((tiles * 32 + 255) / 256);
     if (forward)
-        q45k_retile_kernel<false, true><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        q4k_retile_kernel<true><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const uint8_t *>(src), static_cast<uint8_t *>(dst), tiles, nsb);
     else
-        q45k_retile_kernel<false, false><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        q4k_retile_kernel<false><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const uint8_t *>(src), static_cast<uint8_t *>(dst), tiles, nsb);
     return check_launch("q4k_retile");
 }
@@ -387,10 +405,10 @@ static int q5k_retile_common(const void *src, void *dst, long long rows, int k, 
     const long long tiles = rows / 16 * nsb;
     const unsigned blocks = static_cast<unsigned>((tiles * 32 + 255) / 256);
     if (forward)
-        q45k_retile_kernel<true, true><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        q5k_retile_kernel<true><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const uint8_t *>(src), static_cast<uint8_t *>(dst), tiles, nsb);
     else
-        q45k_retile_kernel<true, false><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        q5k_retile_kernel<false><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const uint8_t *>(src), static_cast<uint8_t *>(dst), tiles, nsb);
     return check_launch("q5k_retile");
 }

@@ -18,15 +18,16 @@
 // Layout of the work: as the direct-load kernel (mma_direct.cuh). A CTA of 16 warps = rg row groups
 // of 16 rows x kp parts of K; a warp streams the packed bytes of its rows' super-blocks with 128-bit
 // loads (GGUF layout or the Q4_K tile layout), one item ahead in registers; lane (g, tig) handles
-// rows g and g+8 and, of every sub-block, the values 4 tig.. and 16 + 4 tig.. (the words of SuperBlockRegs). The int8
-// activations of the whole K range sit in shared memory, the sixteen words of a lane in a super-block side by side, with
-// dx and dx * (sum of a block's codes) beside them.
-#include "mma_direct.cuh"
+// rows g and g+8 and, of every super-block, the 16-value halves tig&1 of sub-blocks 2*(tig>>1),
+// +1, +4, +5. The int8 activations of the whole K range sit in shared memory (32-byte blocks, so a
+// half block is one aligned 16-byte load), with dx and dx * (sum of a half block's codes) beside them.
+#include "common.cuh"
 
 namespace b200q {
 
 constexpr int Q8G_WARPS = 16;
 constexpr int Q8G_THREADS = Q8G_WARPS * 32;
+constexpr int Q8G_TILE_BYTES = 2304;      // Q4_K tile: 16 rows x one super-block (b200q_q4k_retile)
 
 struct Q8GemvArgs {
     const uint8_t *w;
@@ -37,6 +38,20 @@ struct Q8GemvArgs {
     void *y;
     int y_dtype;
     int kp, rg;               // K parts and row groups per CTA (kp * rg == 16)
+};
+
+__device__ __forceinline__ uint4 q8g_ldg128(const uint8_t *p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+
+struct Q4Item {
+    uint4 hd_a, hd_b;         // d, dmin, 12 scale bytes of rows g and g+8
+    uint4 qa_a, qb_a, qa_b, qb_b;
+    uint4 qh_a, qh_b;         // Q5_K: the fifth bits of the lane's 16 elements (all eight sub-blocks), rows g and g+8
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -76,15 +91,15 @@ __global__ void q8_1_quantize_kernel(const void *x, int x_dtype, long long total
 template <int MT, bool Q5>
 __global__ void __launch_bounds__(Q8G_THREADS, 1) q4k_q8_gemv_kernel(const Q8GemvArgs a) {
     constexpr int QB = Q5 ? 176 : 144;                        // bytes of a native super-block
-    constexpr int TILE = direct_tile_bytes<Q5>();              // bytes of a 16-row tile (b200q_q4k_retile / b200q_q5k_retile)
+    constexpr int TILE = Q5 ? 2816 : Q8G_TILE_BYTES;           // bytes of a 16-row tile (b200q_q4k_retile / b200q_q5k_retile)
     chain_trigger();
     extern __shared__ __align__(16) uint8_t smem[];
     const int nblk = a.k >> 5, nsb = a.k >> 8;
-    // shared memory: codes [MT][k] | dx [MT][nblk] | dxs [MT][nblk] | partial [2][16 warps][16 rows][MT]
+    // shared memory: codes [MT][k] | dx [MT][nblk] | dxs [MT][nblk][2] | partial [2][16 warps][16 rows][MT]
     int8_t *qs_s = reinterpret_cast<int8_t *>(smem);
     float *dx_s = reinterpret_cast<float *>(smem + static_cast<size_t>(MT) * a.k);
     float *dxs_s = dx_s + MT * nblk;
-    float *partial = dxs_s + MT * nblk;
+    float *partial = dxs_s + 2 * MT * nblk;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tig = lane & 3;
@@ -94,17 +109,39 @@ __global__ void __launch_bounds__(Q8G_THREADS, 1) q4k_q8_gemv_kernel(const Q8Gem
     const int blk_begin = static_cast<int>(static_cast<long long>(total_blocks) * blockIdx.x / gridDim.x);
     const int blk_end = static_cast<int>(static_cast<long long>(total_blocks) * (blockIdx.x + 1) / gridDim.x);
 
-    auto issue = [&](int row0, int sb, SuperBlockRegs<Q5> &it) {
+    auto issue = [&](int row0, int sb, Q4Item &it) {
         if (a.tiled) {
             const int group = min((row0 >> 4) + rgi, (a.n >> 4) - 1);
-            load_superblock_tiled<Q5>(it, a.w + (static_cast<size_t>(group) * nsb + sb) * TILE, lane);
+            const uint8_t *tile = a.w + (static_cast<size_t>(group) * nsb + sb) * TILE;
+            constexpr int P = Q5 ? 768 : 256;                  // first quant plane (Q5_K: behind the fifth bits)
+            it.hd_a = q8g_ldg128(tile + 16 * g);
+            it.hd_b = q8g_ldg128(tile + 16 * (g + 8));
+            if (Q5) {
+                it.qh_a = q8g_ldg128(tile + 256 + 32 * g + 16 * (tig & 1));
+                it.qh_b = q8g_ldg128(tile + 256 + 32 * (g + 8) + 16 * (tig & 1));
+            }
+            it.qa_a = q8g_ldg128(tile + P + lane * 16);
+            it.qb_a = q8g_ldg128(tile + P + 512 + lane * 16);
+            it.qa_b = q8g_ldg128(tile + P + 1024 + lane * 16);
+            it.qb_b = q8g_ldg128(tile + P + 1536 + lane * 16);
         } else {
-            load_superblock<Q5>(it, a.w + static_cast<size_t>(min(row0 + 16 * rgi + g, a.n - 1)) * a.row_bytes + sb * QB,
-                                a.w + static_cast<size_t>(min(row0 + 16 * rgi + g + 8, a.n - 1)) * a.row_bytes + sb * QB, tig);
+            const uint8_t *ra = a.w + static_cast<size_t>(min(row0 + 16 * rgi + g, a.n - 1)) * a.row_bytes + sb * QB;
+            const uint8_t *rb = a.w + static_cast<size_t>(min(row0 + 16 * rgi + g + 8, a.n - 1)) * a.row_bytes + sb * QB;
+            constexpr int Q = Q5 ? 48 : 16;                    // first quant byte of a native block
+            it.hd_a = q8g_ldg128(ra);
+            it.hd_b = q8g_ldg128(rb);
+            if (Q5) {
+                it.qh_a = q8g_ldg128(ra + 16 + 16 * (tig & 1));
+                it.qh_b = q8g_ldg128(rb + 16 + 16 * (tig & 1));
+            }
+            it.qa_a = q8g_ldg128(ra + Q + 16 * tig);
+            it.qb_a = q8g_ldg128(ra + Q + 64 + 16 * tig);
+            it.qa_b = q8g_ldg128(rb + Q + 16 * tig);
+            it.qb_b = q8g_ldg128(rb + Q + 64 + 16 * tig);
         }
     };
     const int sb_count = kpi < nsb ? (nsb - kpi + a.kp - 1) / a.kp : 0;     // this warp's super-blocks: kpi, kpi+kp, ..
-    SuperBlockRegs<Q5> cur, nxt;
+    Q4Item cur, nxt;
     if (blk_begin < blk_end && sb_count > 0) issue(blk_begin * rows_per_block, kpi, nxt);   // weights: before the wait
 
     chain_wait();                 // the activation blocks come from the preceding kernel (the quantiser)
@@ -114,23 +151,25 @@ __global__ void __launch_bounds__(Q8G_THREADS, 1) q4k_q8_gemv_kernel(const Q8Gem
         const bool live = t < a.m;
         const uint8_t *src = a.xq + (static_cast<size_t>(t) * nblk + b) * 36;
         uint32_t wds[8];
-        int sum = 0;
+        int s0 = 0, s1 = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             wds[j] = live ? *reinterpret_cast<const uint32_t *>(src + 4 + 4 * j) : 0u;
-            sum = __dp4a(0x01010101, static_cast<int>(wds[j]), sum);
+            if (j < 4) s0 = __dp4a(0x01010101, static_cast<int>(wds[j]), s0);
+            else s1 = __dp4a(0x01010101, static_cast<int>(wds[j]), s1);
         }
-        // block b & 7 of its super-block: words q and q + 4 belong to lane q of a quad
-        uint8_t *dst = reinterpret_cast<uint8_t *>(qs_s) + static_cast<size_t>(t) * a.k + 256 * (b >> 3) + 8 * (b & 7);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) *reinterpret_cast<uint2 *>(dst + 64 * q) = make_uint2(wds[q], wds[q + 4]);
+        uint4 *dst = reinterpret_cast<uint4 *>(qs_s + static_cast<size_t>(t) * a.k + 32 * b);
+        dst[0] = make_uint4(wds[0], wds[1], wds[2], wds[3]);
+        dst[1] = make_uint4(wds[4], wds[5], wds[6], wds[7]);
         const float dx = live ? __half2float(*reinterpret_cast<const __half *>(src)) : 0.f;
         dx_s[i] = dx;
-        dxs_s[i] = dx * static_cast<float>(sum);
+        dxs_s[2 * i] = dx * static_cast<float>(s0);
+        dxs_s[2 * i + 1] = dx * static_cast<float>(s1);
     }
     __syncthreads();
     if (blk_begin >= blk_end) return;
 
+    const int pair = tig >> 1, half = tig & 1;
     int pbuf = 0;
     for (int blk = blk_begin; blk < blk_end; ++blk) {
         const int row0 = blk * rows_per_block;
@@ -142,60 +181,60 @@ __global__ void __launch_bounds__(Q8G_THREADS, 1) q4k_q8_gemv_kernel(const Q8Gem
             if (it + 1 < sb_count) issue(row0, kpi + (it + 1) * a.kp, nxt);
             else if (blk + 1 < blk_end) issue(row0 + rows_per_block, kpi, nxt);
             const int sb = kpi + it * a.kp;
-            if (!a.tiled) transpose_native<Q5>(cur, tig);
-            // the eight scales of a row, and the minima of the two sub-blocks whose sums this lane adds (2 tig, 2 tig + 1)
-            auto scales = [&](const uint4 &hd, uint32_t (&sc)[2], float (&mn)[2], float &d, float &dmin) {
+            // scales and minima of the lane's four sub-blocks 2*pair, +1, +4, +5 for both rows
+            auto scales = [&](const uint4 &hd, int (&sc)[4], float (&mn)[4], float &d, float &dmin) {
                 d = half_bits_to_float(hd.x & 0xffffu);
                 dmin = half_bits_to_float(hd.x >> 16);
-                sc[0] = hd.y & 0x3f3f3f3fu;
-                sc[1] = (hd.w & 0x0f0f0f0fu) | ((hd.y >> 2) & 0x30303030u);
-                const uint32_t m = ((tig & 2) ? ((hd.w >> 4) & 0x0f0f0f0fu) | ((hd.z >> 2) & 0x30303030u) : hd.z & 0x3f3f3f3fu) >> (16 * (tig & 1));
-                mn[0] = static_cast<float>(m & 0xffu);
-                mn[1] = static_cast<float>((m >> 8) & 0xffu);
+                const uint32_t lo = hd.y >> (16 * pair), lm = hd.z >> (16 * pair), hi = hd.w >> (16 * pair);
+                sc[0] = lo & 63;
+                sc[1] = (lo >> 8) & 63;
+                sc[2] = (hi & 15) | ((lo >> 2) & 48);
+                sc[3] = ((hi >> 8) & 15) | ((lo >> 10) & 48);
+                mn[0] = static_cast<float>(lm & 63);
+                mn[1] = static_cast<float>((lm >> 8) & 63);
+                mn[2] = static_cast<float>(((hi >> 4) & 15) | ((lm >> 2) & 48));
+                mn[3] = static_cast<float>(((hi >> 12) & 15) | ((lm >> 10) & 48));
             };
-            uint32_t sc_a[2], sc_b[2];
-            float mn_a[2], mn_b[2], d_a, dm_a, d_b, dm_b;
-            scales(cur.hd[0], sc_a, mn_a, d_a, dm_a);
-            scales(cur.hd[1], sc_b, mn_b, d_b, dm_b);
-            const uint32_t wa[8] = {cur.q[0].x, cur.q[0].y, cur.q[0].z, cur.q[0].w, cur.q[1].x, cur.q[1].y, cur.q[1].z, cur.q[1].w};
-            const uint32_t wb[8] = {cur.q[2].x, cur.q[2].y, cur.q[2].z, cur.q[2].w, cur.q[3].x, cur.q[3].y, cur.q[3].z, cur.q[3].w};
-            const uint32_t ha[2] = {cur.h[0].x, cur.h[0].y}, hb[2] = {cur.h[1].x, cur.h[1].y};
+            int sc_a[4], sc_b[4];
+            float mn_a[4], mn_b[4], d_a, dm_a, d_b, dm_b;
+            scales(cur.hd_a, sc_a, mn_a, d_a, dm_a);
+            scales(cur.hd_b, sc_b, mn_b, d_b, dm_b);
+            const uint32_t wa[2][4] = {{cur.qa_a.x, cur.qa_a.y, cur.qa_a.z, cur.qa_a.w}, {cur.qb_a.x, cur.qb_a.y, cur.qb_a.z, cur.qb_a.w}};
+            const uint32_t wb[2][4] = {{cur.qa_b.x, cur.qa_b.y, cur.qa_b.z, cur.qa_b.w}, {cur.qb_b.x, cur.qb_b.y, cur.qb_b.z, cur.qb_b.w}};
+            const uint32_t ha[4] = {cur.qh_a.x, cur.qh_a.y, cur.qh_a.z, cur.qh_a.w}, hb[4] = {cur.qh_b.x, cur.qh_b.y, cur.qh_b.z, cur.qh_b.w};
 #pragma unroll
             for (int t = 0; t < MT; ++t) {
-                float sd_a = 0.f, sd_b = 0.f;
-                const uint4 *up = reinterpret_cast<const uint4 *>(qs_s + static_cast<size_t>(t) * a.k + 256 * sb + 64 * tig);
-                const float4 *dp = reinterpret_cast<const float4 *>(dx_s + t * nblk + sb * 8);
+                float sd_a = 0.f, sm_a = 0.f, sd_b = 0.f, sm_b = 0.f;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint4 u = up[c];                                    // sub-block 2c: words j = 0, 1; then 2c + 1
-                    const float4 dx4 = dp[c >> 1];
+                for (int X = 0; X < 2; ++X) {
 #pragma unroll
                     for (int nib = 0; nib < 2; ++nib) {
-                        const int s = 2 * c + nib;
-                        const int uw[2] = {static_cast<int>(nib ? u.z : u.x), static_cast<int>(nib ? u.w : u.y)};
+                        const int si = 2 * X + nib;                       // index into sc / mn
+                        const int ablk = sb * 8 + 4 * X + 2 * pair + nib;  // activation block = sub-block
+                        const uint4 u = *reinterpret_cast<const uint4 *>(qs_s + static_cast<size_t>(t) * a.k + 32 * ablk + 16 * half);
+                        const int uw[4] = {static_cast<int>(u.x), static_cast<int>(u.y), static_cast<int>(u.z), static_cast<int>(u.w)};
                         int dot_a = 0, dot_b = 0;
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            uint32_t ua = (wa[2 * c + j] >> (4 * nib)) & 0x0f0f0f0fu, ub = (wb[2 * c + j] >> (4 * nib)) & 0x0f0f0f0fu;
-                            if (Q5) {                          // bit s of the fifth-bit byte -> bit 4 of the code
-                                ua |= ((ha[j] >> s) << 4) & 0x10101010u;
-                                ub |= ((hb[j] >> s) << 4) & 0x10101010u;
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t ua = (wa[X][j] >> (4 * nib)) & 0x0f0f0f0fu, ub = (wb[X][j] >> (4 * nib)) & 0x0f0f0f0fu;
+                            if (Q5) {                          // bit (sub-block) of the fifth-bit byte -> bit 4 of the code
+                                const int sub = 4 * X + 2 * pair + nib;
+                                ua |= ((ha[j] >> sub) << 4) & 0x10101010u;
+                                ub |= ((hb[j] >> sub) << 4) & 0x10101010u;
                             }
-                            dot_a = __dp4a(static_cast<int>(ua), uw[j], dot_a);
-                            dot_b = __dp4a(static_cast<int>(ub), uw[j], dot_b);
+                            const int ca = static_cast<int>(ua), cb = static_cast<int>(ub);
+                            dot_a = __dp4a(ca, uw[j], dot_a);
+                            dot_b = __dp4a(cb, uw[j], dot_b);
                         }
-                        const int sh = 8 * (s & 3);
-                        const float dx = (s & 3) == 0 ? dx4.x : (s & 3) == 1 ? dx4.y : (s & 3) == 2 ? dx4.z : dx4.w;
-                        // |dot * sc| <= 8 * 31 * 127 * 63 < 2^22: integer -> float by adding it to the bits of 1.5 * 2^23
-                        const int va = dot_a * static_cast<int>((sc_a[s >> 2] >> sh) & 0xffu) + 0x4b400000;
-                        const int vb = dot_b * static_cast<int>((sc_b[s >> 2] >> sh) & 0xffu) + 0x4b400000;
-                        sd_a = fmaf(dx, __int_as_float(va) - 12582912.0f, sd_a);
-                        sd_b = fmaf(dx, __int_as_float(vb) - 12582912.0f, sd_b);
+                        const float dx = dx_s[t * nblk + ablk], dxs = dxs_s[2 * (t * nblk + ablk) + half];
+                        sd_a = fmaf(dx, static_cast<float>(dot_a * sc_a[si]), sd_a);
+                        sd_b = fmaf(dx, static_cast<float>(dot_b * sc_b[si]), sd_b);
+                        sm_a = fmaf(dxs, mn_a[si], sm_a);
+                        sm_b = fmaf(dxs, mn_b[si], sm_b);
                     }
                 }
-                const float2 dxs = *reinterpret_cast<const float2 *>(dxs_s + t * nblk + sb * 8 + 2 * tig);
-                tot_a[t] += d_a * sd_a - dm_a * fmaf(dxs.x, mn_a[0], dxs.y * mn_a[1]);
-                tot_b[t] += d_b * sd_b - dm_b * fmaf(dxs.x, mn_b[0], dxs.y * mn_b[1]);
+                tot_a[t] += d_a * sd_a - dm_a * sm_a;
+                tot_b[t] += d_b * sd_b - dm_b * sm_b;
             }
         }
         // the four lanes of a quad hold the four quarters of each sub-block pair: add them, then the K parts
@@ -272,7 +311,7 @@ extern "C" int b200q_gemv_q8_1(const void *w, int fmt, int n, int k, const void 
         auto blocks_for = [&](int parts) { return (static_cast<long long>(n) + 16 * (Q8G_WARPS / parts) - 1) / (16 * (Q8G_WARPS / parts)); };
         while (kp * 2 <= Q8G_WARPS && kp * 2 <= nsb && blocks_for(kp) < 6LL * sm_count()) kp *= 2;
         a.kp = kp; a.rg = Q8G_WARPS / kp;
-        const size_t smem = static_cast<size_t>(mt) * k + static_cast<size_t>(mt) * (k / 32) * 8 + 2 * Q8G_WARPS * 16 * mt * 4;
+        const size_t smem = static_cast<size_t>(mt) * k + static_cast<size_t>(mt) * (k / 32) * 12 + 2 * Q8G_WARPS * 16 * mt * 4;
         if (smem > 200 * 1024) return fail(B200Q_EUNSUPPORTED, "gemv_q8_1: K=%d too large for the activation tile", k);
         auto fn = q5 ? (mt == 4 ? q4k_q8_gemv_kernel<4, true> : mt == 2 ? q4k_q8_gemv_kernel<2, true> : q4k_q8_gemv_kernel<1, true>)
                      : (mt == 4 ? q4k_q8_gemv_kernel<4, false> : mt == 2 ? q4k_q8_gemv_kernel<2, false> : q4k_q8_gemv_kernel<1, false>);

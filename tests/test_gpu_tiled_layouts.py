@@ -9,6 +9,7 @@ from mylocal_llm_b200 import PackedExpertBank, packed_to_device, quantized_linea
 from mylocal_llm_b200 import moe_ops
 from mylocal_llm_b200.experts_inference import routed_experts_forward, synthetic_bank
 from mylocal_llm_b200.quantize import quantize, random_packed
+from mylocal_llm_b200.quantized_weight import PackedGGUFWeight
 from mylocal_llm_b200 import quantized_swiglu
 from mylocal_llm_b200.quantized_linear import (DevicePackedGGUFWeight, dequantize_device, retile_bytes, retile_q6k,
                                                retile_weight, untile_bytes, untile_q6k)
@@ -249,3 +250,24 @@ def test_q8_0_tiled_identity_columns_are_exact(cuda):
             x[t, start + t] = 1.0
         got = quantized_linear(cuda.from_numpy(x).cuda(), tiled).cpu().numpy()
         np.testing.assert_array_equal(got, deq[:, start:start + 8].T)
+
+
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16"])
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q5_K"])
+def test_small_activations_beside_a_large_one_are_summed_exactly(cuda, fmt, dtype, tiled):
+    """Codes, scales and d of one, one activation of 1 and the others 2^-16: the sum has 17 significant bits, so FP32 sums
+    in any order are exact. (Codes as FP16 subnormals are not: the tensor cores align products by the operands' exponents,
+    and the leading zeros of a subnormal push the small products out of the window.)"""
+    torch = cuda
+    block = np.zeros({"Q4_K": 144, "Q5_K": 176}[fmt], np.uint8)
+    block[0:2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+    block[4:8] = block[12:16] = 1                    # the eight 6-bit scales; minima and dmin are zero
+    block[-128:] = 0x11                              # every code one (no fifth bits)
+    w = packed_to_device(PackedGGUFWeight(np.tile(block, 32), (16, 512), fmt))
+    w = retile_weight(w) if tiled else w
+    for m in (1, 8, 16):
+        x = torch.full((m, 512), 2.0 ** -16, device="cuda")
+        x[torch.arange(m), 31 * torch.arange(m)] = 1.0
+        y = quantized_linear(x.to(getattr(torch, dtype)), w, out_dtype=torch.float32, allow_gemm=False)
+        assert (y == 1.0 + 511 * 2.0 ** -16).all(), (m, y.min().item(), y.max().item())
