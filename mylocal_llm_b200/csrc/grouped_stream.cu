@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) grouped_gate_up_kernel(const Gr
         const uint8_t *image = buf + g * a.smem_stride;
         const uint8_t *fp = image + tig * 16 + kpi * 512, *xp = image + sums_off + tig * 4 + kpi * 32;
         float tg[1][4] = {{0.f, 0.f, 0.f, 0.f}}, tu[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-        auto frag = [&](int, int s, int p) { return *reinterpret_cast<const uint4 *>(fp + s * 64 + p * plane); };
+        auto frag = [&](int, int fi, int p) { return *reinterpret_cast<const uint2 *>(fp + (fi >> 1) * 64 + (fi & 1) * 8 + p * plane); };
         auto sums = [&](int, int term) { return *reinterpret_cast<const uint32_t *>(xp + term * 16); };
         for (int sb = kpi; sb < a.nsb; sb += a.kp) {
             SuperBlockRegs<Q5> ra, rb;

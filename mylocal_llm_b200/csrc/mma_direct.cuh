@@ -215,15 +215,14 @@ __device__ __forceinline__ RowScales decode_scales(const uint4 &hd, int tig) {
 // Activation fragments for the direct kernel. Fragment (sb, fi) with fi = (X*2 + nib)*4 + j holds,
 // for lane (g = lane>>2, tig = lane&3), token g at positions
 //   256*sb + 32*(4*X + 2*(tig>>1) + nib) + 16*(tig&1) + 4*j + {0,2 -> b0 ; 1,3 -> b1}
-// which are exactly the positions of the codes that lane extracts from word j of its quant bytes. Fragments f = sb*16 + fi
-// lie in pairs (one 16-byte load): uint2 entry ((f >> 1) * 32 + lane) * 2 + (f & 1), direct_entry().
+// which are exactly the positions of the codes that lane extracts from word j of its quant bytes.
 // xsfrag (sb, term) holds (sum_x[sub 2*tig], sum_x[sub 2*tig+1]) / 64 for token g.
 // ---------------------------------------------------------------------------------------------
 // Entry of the chunk of four positions that starts at p, token slot t.
 __device__ __forceinline__ int direct_entry(int p, int t) {
     const int sub = (p >> 5) & 7, tig = 2 * ((sub >> 1) & 1) + ((p >> 4) & 1);
     const int f = (p >> 8) * 16 + ((sub >> 2) * 2 + (sub & 1)) * 4 + ((p >> 2) & 3);
-    return ((f >> 1) * 32 + 4 * t + tig) * 2 + (f & 1);
+    return f * 32 + 4 * t + tig;
 }
 // Four consecutive activations starting at element index e (a multiple of 4) as floats.
 // `vec_ok` tells whether the tensor allows aligned vector loads.
@@ -576,8 +575,10 @@ __global__ void __launch_bounds__(MD_THREADS, 1) token_image_kernel(const void *
     uint4 *dst = reinterpret_cast<uint4 *>(images + static_cast<size_t>(row) * units * 16);
     for (int u = tid; u < units; u += MD_THREADS) {
         uint4 v;
-        if (u < nb) v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(bfrag) + (u >> 2) * 512 + (u & 3) * 16);
-        else if (u < units - 1) v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(xsfrag) + (u - nb) * 128);
+        if (u < nb) {
+            const uint2 a = bfrag[(u >> 2) * 64 + (u & 3)], b = bfrag[(u >> 2) * 64 + 32 + (u & 3)];
+            v = make_uint4(a.x, a.y, b.x, b.y);
+        } else if (u < units - 1) v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(xsfrag) + (u - nb) * 128);
         else v = make_uint4(__float_as_uint(tok_scale[0]), __float_as_uint(tok_scale[8]), 0u, 0u);
         dst[u] = v;
     }
@@ -596,8 +597,10 @@ __device__ __forceinline__ void gather_token_images(const uint8_t *images, int i
 #pragma unroll 5
         for (int u = (tid >> 8) * 32 + (tid & 31); u < units; u += 64) {
             const uint4 v = src[u];
-            if (u < nb) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(bfrag) + (u >> 2) * 512 + t * 64 + (u & 3) * 16) = v;
-            else if (u < units - 1) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(xsfrag) + (u - nb) * 128 + t * 16) = v;
+            if (u < nb) {
+                bfrag[(u >> 2) * 64 + 4 * t + (u & 3)] = make_uint2(v.x, v.y);
+                bfrag[(u >> 2) * 64 + 32 + 4 * t + (u & 3)] = make_uint2(v.z, v.w);
+            } else if (u < units - 1) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(xsfrag) + (u - nb) * 128 + t * 16) = v;
             else {
                 tok_scale[t] = __uint_as_float(v.x);
                 tok_scale[8 + t] = __uint_as_float(v.y);
@@ -610,8 +613,8 @@ __device__ __forceinline__ void gather_token_images(const uint8_t *images, int i
 // With NT token tiles (8 tokens each; their fragments `btile` / `xtile` entries apart) every decoded
 // A operand is multiplied into each tile, so the decode cost is paid once per 8*NT tokens; the
 // arithmetic of one token does not depend on NT.
-// frag(nt, pair, plane): the lane's 16 bytes of fragments 2 pair, 2 pair + 1 of the super-block in plane 0 (FP16 high
-// parts) or 1 (remainders) of token tile nt; sums(nt, term): the lane's word of the activation sums.
+// frag(nt, fi, plane): the lane's entry of the super-block's fragment fi in plane 0 (FP16 high parts) or 1 (remainders) of
+// token tile nt; sums(nt, term): the lane's word of the activation sums.
 template <bool Q5, int NTERMS, int NT, typename FragFn, typename SumFn>
 __device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &ra, const SuperBlockRegs<Q5> &rb, const FragFn frag,
                                                const SumFn sums, int tig, float (&tot)[NT][4]) {
@@ -633,33 +636,27 @@ __device__ __forceinline__ void superblock_mma(const SuperBlockRegs<Q5> &ra, con
             // Q5_K: bit (sub-block index) of the high-bit byte, moved to bit 4 of the code
             const int sub = 4 * X + 2 * pair + nib;
 #pragma unroll
-            for (int jp = 0; jp < 2; ++jp) {
-                uint32_t f[2][4];                            // A operands of words 2 jp, 2 jp + 1
-#pragma unroll
-                for (int jj = 0; jj < 2; ++jj) {
-                    const int j = 2 * jp + jj;
-                    const uint32_t wa = X ? qb_a[j] : qa_a[j], wb = X ? qb_b[j] : qa_b[j];
-                    uint32_t va = nib ? (wa >> 4) & 0x0f0f0f0fu : wa & 0x0f0f0f0fu;
-                    uint32_t vb = nib ? (wb >> 4) & 0x0f0f0f0fu : wb & 0x0f0f0f0fu;
-                    if (Q5) {
-                        va |= ((qh_a[j] >> sub) << 4) & 0x10101010u;
-                        vb |= ((qh_b[j] >> sub) << 4) & 0x10101010u;
-                    }
-                    f[jj][0] = hfma2_u32(__byte_perm(va, 0x64646464u, 0x4240), sa.sc[si], sa.nsc[si]);
-                    f[jj][1] = hfma2_u32(__byte_perm(vb, 0x64646464u, 0x4240), sbk.sc[si], sbk.nsc[si]);
-                    f[jj][2] = hfma2_u32(__byte_perm(va, 0x64646464u, 0x4341), sa.sc[si], sa.nsc[si]);
-                    f[jj][3] = hfma2_u32(__byte_perm(vb, 0x64646464u, 0x4341), sbk.sc[si], sbk.nsc[si]);
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t wa = X ? qb_a[j] : qa_a[j], wb = X ? qb_b[j] : qa_b[j];
+                uint32_t va = nib ? (wa >> 4) & 0x0f0f0f0fu : wa & 0x0f0f0f0fu;
+                uint32_t vb = nib ? (wb >> 4) & 0x0f0f0f0fu : wb & 0x0f0f0f0fu;
+                if (Q5) {
+                    va |= ((qh_a[j] >> sub) << 4) & 0x10101010u;
+                    vb |= ((qh_b[j] >> sub) << 4) & 0x10101010u;
                 }
+                const uint32_t a0 = hfma2_u32(__byte_perm(va, 0x64646464u, 0x4240), sa.sc[si], sa.nsc[si]);
+                const uint32_t a2 = hfma2_u32(__byte_perm(va, 0x64646464u, 0x4341), sa.sc[si], sa.nsc[si]);
+                const uint32_t a1 = hfma2_u32(__byte_perm(vb, 0x64646464u, 0x4240), sbk.sc[si], sbk.nsc[si]);
+                const uint32_t a3 = hfma2_u32(__byte_perm(vb, 0x64646464u, 0x4341), sbk.sc[si], sbk.nsc[si]);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
                     float (&c)[4] = X ? acc2[nt] : acc[nt];
-                    const uint4 h = frag(nt, si * 2 + jp, 0);
-                    uint4 l = make_uint4(0u, 0u, 0u, 0u);
-                    if (NTERMS == 2) l = frag(nt, si * 2 + jp, 1);
-                    mma_f16(c, f[0][0], f[0][1], f[0][2], f[0][3], h.x, h.y);
-                    if (NTERMS == 2) mma_f16(c, f[0][0], f[0][1], f[0][2], f[0][3], l.x, l.y);
-                    mma_f16(c, f[1][0], f[1][1], f[1][2], f[1][3], h.z, h.w);
-                    if (NTERMS == 2) mma_f16(c, f[1][0], f[1][1], f[1][2], f[1][3], l.z, l.w);
+                    const uint2 h = frag(nt, si * 4 + j, 0);
+                    mma_f16(c, a0, a1, a2, a3, h.x, h.y);
+                    if (NTERMS == 2) {
+                        const uint2 l = frag(nt, si * 4 + j, 1);
+                        mma_f16(c, a0, a1, a2, a3, l.x, l.y);
+                    }
                 }
             }
         }
@@ -862,9 +859,9 @@ __device__ __forceinline__ void mma_direct_body(const DirectArgs &a, const Stage
             else if (has_next) issue_item(nxt_p, 0, nxt_a, nxt_b);
             const int stream = DUAL ? (item & 1) : 0;
             const int sb = kpi + (DUAL ? (item >> 1) : item) * a.kp;
-            const uint4 *bf = reinterpret_cast<const uint4 *>(bfrag) + sb * 256 + lane;
+            const uint2 *bf = bfrag + sb * 512 + lane;
             const uint32_t *xf = xsfrag + sb * 64 + lane;
-            auto frag = [&](int nt, int p, int plane) { return bf[nt * (btile >> 1) + plane * nfrag * 16 + p * 32]; };
+            auto frag = [&](int nt, int fi, int plane) { return bf[nt * btile + (plane * nfrag + fi) * 32]; };
             auto sums = [&](int nt, int term) { return xf[nt * xtile + term * 32]; };
             if (stream == 0) superblock_mma<Q5, NTERMS, NT>(cur_a, cur_b, frag, sums, tig, tot_a);
             else superblock_mma<Q5, NTERMS, NT>(cur_a, cur_b, frag, sums, tig, tot_b);
