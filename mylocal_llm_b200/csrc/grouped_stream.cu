@@ -43,9 +43,9 @@ __global__ void __launch_bounds__(GS_THREADS, 1) grouped_gate_up_kernel(const Gr
     auto work = [&](int seg, int group, const uint8_t *buf, TileStream<TILE, true> &stream) -> bool {
         const int begin = a.seg_begin[seg], count = min(a.seg_count[seg], 8);
         const uint8_t *image = buf + g * a.smem_stride;
-        const uint8_t *fp = image + tig * 16 + kpi * 512, *xp = image + sums_off + tig * 4 + kpi * 32;
+        const uint8_t *fp = image + tig * 8 + kpi * 512, *xp = image + sums_off + tig * 4 + kpi * 32;
         float tg[1][4] = {{0.f, 0.f, 0.f, 0.f}}, tu[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-        auto frag = [&](int, int fi, int p) { return *reinterpret_cast<const uint2 *>(fp + (fi >> 1) * 64 + (fi & 1) * 8 + p * plane); };
+        auto frag = [&](int, int fi, int p) { return *reinterpret_cast<const uint2 *>(fp + fi * 32 + p * plane); };
         auto sums = [&](int, int term) { return *reinterpret_cast<const uint32_t *>(xp + term * 16); };
         for (int sb = kpi; sb < a.nsb; sb += a.kp) {
             SuperBlockRegs<Q5> ra, rb;
@@ -219,14 +219,14 @@ int hidden_images(const float *h, int rows, int k, void *images, cudaStream_t st
     return check_launch("hidden images");
 }
 
-// Fills the shared part of the arguments; false when two segment buffers do not fit in shared memory.
-static bool grouped_args(const MmaRequest &q, int image_bytes, int tile_bytes, GroupedArgs &a, size_t &smem) {
+// Fills the shared part of the arguments (row_bytes: what the four lanes of a token read side by side); false when two segment buffers do not fit in shared memory.
+static bool grouped_args(const MmaRequest &q, int image_bytes, int row_bytes, int tile_bytes, GroupedArgs &a, size_t &smem) {
     a.wa = q.wa; a.wb = q.wb; a.stride_a = q.stride_a; a.stride_b = q.stride_b;
     a.table_a = q.table_a; a.table_b = q.table_b;
     a.n = q.n; a.nsb = q.k / 256; a.kp = grouped_kp(q.n, a.nsb, q.max_segments);
     a.images = static_cast<const uint8_t *>(q.images);
     a.image_bytes = image_bytes;
-    a.smem_stride = (image_bytes + 63) / 128 * 128 + 64;
+    a.smem_stride = (image_bytes + 127 - row_bytes) / 128 * 128 + row_bytes;
     // two segment buffers and two tiles per warp at least; what is left goes to the tile rings first
     a.off_ring = GS_CTRL_BYTES + (a.kp > 1 ? GS_PART_BYTES : 0);
     const int room = MM_SMEM_LIMIT - a.off_ring, buf_bytes = 8 * a.smem_stride, ring_bytes = GS_WARPS * tile_bytes;
@@ -261,7 +261,7 @@ int grouped_gate_up_launch(const MmaRequest &q, cudaStream_t stream, bool *launc
     const int image_bytes = direct_token_image_bytes(q.k, q.x_dtype);
     if (!q.images || !q.tiled || image_bytes == 0 || (reinterpret_cast<uintptr_t>(q.images) & 15) || q.max_segments <= GROUPED_FEW_SEGMENTS)
         return B200Q_OK;
-    if (!grouped_args(q, image_bytes, q.fmt_a == B200Q_Q5_K ? Q5T_TILE_BYTES : Q4T_TILE_BYTES, a, smem)) return B200Q_OK;
+    if (!grouped_args(q, image_bytes, 32, q.fmt_a == B200Q_Q5_K ? Q5T_TILE_BYTES : Q4T_TILE_BYTES, a, smem)) return B200Q_OK;
     const bool two = q.x_dtype == B200Q_F32, q5 = q.fmt_a == B200Q_Q5_K;
     auto fn = q5 ? (two ? grouped_gate_up_kernel<true, 2> : grouped_gate_up_kernel<true, 1>)
                  : (two ? grouped_gate_up_kernel<false, 2> : grouped_gate_up_kernel<false, 1>);
@@ -275,7 +275,7 @@ int grouped_down_launch(const MmaRequest &q, cudaStream_t stream, bool *launched
     size_t smem = 0;
     if (!q.images || hidden_image_bytes(q.k) == 0 || (reinterpret_cast<uintptr_t>(q.images) & 15) || q.max_segments <= GROUPED_FEW_SEGMENTS)
         return B200Q_OK;
-    if (!grouped_args(q, hidden_image_bytes(q.k), q.fmt_a == B200Q_Q8_0_TILED ? Q8T_TILE_BYTES : Q6T_TILE_BYTES, a, smem)) return B200Q_OK;
+    if (!grouped_args(q, hidden_image_bytes(q.k), 64, q.fmt_a == B200Q_Q8_0_TILED ? Q8T_TILE_BYTES : Q6T_TILE_BYTES, a, smem)) return B200Q_OK;
     *launched = true;
     return launch_grouped(q.fmt_a == B200Q_Q8_0_TILED ? grouped_down_kernel<Q8Tile> : grouped_down_kernel<Q6Tile>, a, smem, stream,
                           "grouped down");

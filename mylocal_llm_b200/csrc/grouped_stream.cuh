@@ -12,8 +12,9 @@
 //   * weights come by one bulk copy per tile into a ring of the warp's own (two to four tiles of 2.3-4.4 KB), refilled as
 //     soon as a tile is in registers: 100-200 KB per SM are on their way at any time (two register sets in turn kept 37 KB
 //     in flight and the warps waited for memory: 3.3 stalled per issue).
-// Image rows lie behind one another in shared memory, 64 bytes more than a multiple of 128 apart, so the eight lanes of a
-// quarter warp (two tokens x 64 bytes) read eight different 16-byte banks groups.
+// Image rows lie behind one another in shared memory, 32 (token images, 8 bytes per lane and fragment) or 64 bytes (hidden
+// images, pairs of fragments, 16 bytes per lane) more than a multiple of 128 apart, so the tokens of one wavefront read
+// different banks.
 // The sums are those of the block-structured kernels with the same kp, bit for bit.
 // Bound by instruction issue (256 tokens, 512 experts: 0.63-0.68 of the slots, ALU pipe 0.54, DRAM 0.53 / 0.40): positions
 // in the run of row groups are kept by steps instead of divisions, and the copies are predicated, not branched around

@@ -550,7 +550,7 @@ __device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k
 // a token routed to k experts would be converted k times (at 64 tokens: 704 conversions of 64 distinct
 // rows, each a chain of dependent loads, a reduction and three barriers). token_image_kernel runs
 // prepare_direct once per token - same code, so the same bits - and stores what it wrote for token slot 0:
-//   [NTERMS * nfrag * 32 bytes]  the slot's four lanes (tig 0..3, 16 bytes each) of every pair of fragments
+//   [NTERMS * nfrag * 32 bytes]  the slot's four fragment lanes (tig 0..3, 8 bytes each) of every fragment
 //   [nsb * 2 * 16 bytes]         the slot's four words of every activation-sum row
 //   [16 bytes]                   scale, inverse scale
 // gather_token_images copies the images of a segment's tokens into the slots of the CTA's buffers with
@@ -575,10 +575,8 @@ __global__ void __launch_bounds__(MD_THREADS, 1) token_image_kernel(const void *
     uint4 *dst = reinterpret_cast<uint4 *>(images + static_cast<size_t>(row) * units * 16);
     for (int u = tid; u < units; u += MD_THREADS) {
         uint4 v;
-        if (u < nb) {
-            const uint2 a = bfrag[(u >> 2) * 64 + (u & 3)], b = bfrag[(u >> 2) * 64 + 32 + (u & 3)];
-            v = make_uint4(a.x, a.y, b.x, b.y);
-        } else if (u < units - 1) v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(xsfrag) + (u - nb) * 128);
+        if (u < nb) v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(bfrag) + (u >> 1) * 256 + (u & 1) * 16);
+        else if (u < units - 1) v = *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(xsfrag) + (u - nb) * 128);
         else v = make_uint4(__float_as_uint(tok_scale[0]), __float_as_uint(tok_scale[8]), 0u, 0u);
         dst[u] = v;
     }
@@ -597,10 +595,8 @@ __device__ __forceinline__ void gather_token_images(const uint8_t *images, int i
 #pragma unroll 5
         for (int u = (tid >> 8) * 32 + (tid & 31); u < units; u += 64) {
             const uint4 v = src[u];
-            if (u < nb) {
-                bfrag[(u >> 2) * 64 + 4 * t + (u & 3)] = make_uint2(v.x, v.y);
-                bfrag[(u >> 2) * 64 + 32 + 4 * t + (u & 3)] = make_uint2(v.z, v.w);
-            } else if (u < units - 1) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(xsfrag) + (u - nb) * 128 + t * 16) = v;
+            if (u < nb) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(bfrag) + (u >> 1) * 256 + t * 32 + (u & 1) * 16) = v;
+            else if (u < units - 1) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(xsfrag) + (u - nb) * 128 + t * 16) = v;
             else {
                 tok_scale[t] = __uint_as_float(v.x);
                 tok_scale[8 + t] = __uint_as_float(v.y);
