@@ -263,6 +263,11 @@ int b200q_moe_down(const void *down_base, int64_t down_stride, int down_fmt, con
  * rows * b200q_moe_hidden_image_bytes(f) bytes, 16-byte aligned (0: this f has no images); kernels that do not use images
  * ignore the buffer. */
 int b200q_moe_hidden_image_bytes(int f);
+/* 1 where the grouped launch of these types and sizes reads the images as its segments' operands and is the faster one
+ * with them, their conversion included (tile layouts, plans of many segments); 0: b200q_moe_down without images, and
+ * b200q_moe_gate_up with token images from 32 rows on. A function of its arguments alone. */
+int b200q_moe_gate_up_streams(int fmt, int f, int d, int x_dtype, int max_segments);
+int b200q_moe_down_streams(int fmt, int d, int f, int max_segments);
 int b200q_moe_hidden_images(const float *hbuf, int rows, int f, void *images, void *stream);
 int b200q_moe_down_images(const void *down_base, int64_t down_stride, int down_fmt, const uint64_t *down_table,
                           int tables_aligned16, int flat_rows, int d, int f, const float *hbuf, const void *images,

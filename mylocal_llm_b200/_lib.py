@@ -98,6 +98,8 @@ SIGNATURES = {
     "b200q_moe_down": [_ptr, _c_i64, _c_int, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr,
                        _c_int, _ptr, _ptr],
     "b200q_moe_hidden_image_bytes": [_c_int],
+    "b200q_moe_gate_up_streams": [_c_int] * 5,
+    "b200q_moe_down_streams": [_c_int] * 4,
     "b200q_moe_hidden_images": [_ptr, _c_int, _c_int, _ptr, _ptr],
     "b200q_moe_down_images": [_ptr, _c_i64, _c_int, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr,
                               _ptr, _ptr, _c_int, _ptr, _ptr],

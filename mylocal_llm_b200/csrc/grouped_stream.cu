@@ -190,12 +190,11 @@ __global__ void __launch_bounds__(256) hidden_image_kernel(const float *h, int r
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
-// Warps per 16-row group (parts of K) for a grouped launch over tile-layout weights with more than a few segments; a
-// function of the plan's bound only, so that every caller with that bound adds in the same order. A CTA deals its row
-// groups to 16 / kp teams: the last round is on average half empty, which costs 1 / (2 kp) of a round, while every
-// doubling of kp adds a meeting of the team per group (about 2 % of a group of eight super-blocks). About 65 % of the
-// bound are segments that exist (measured 62-73 % for 16 to 256 tokens over 512 experts).
-int grouped_kp(int n, int nsb, int max_segments) {
+// Warps per 16-row group (parts of K). A CTA deals its row groups to 16 / kp teams: the last round is on average half
+// empty, which costs 1 / (2 kp) of a round, while every doubling of kp adds a meeting of the team per group (about 2 % of a
+// group of eight super-blocks). About 65 % of the bound are segments that exist (measured 62-73 % for 16 to 256 tokens over
+// 512 experts).
+static int grouped_kp(int n, int nsb, int max_segments) {
     const double groups = 0.65 * max_segments * (n / 16) / sm_count();
     int best = 1;
     double cost = 1e30;
@@ -209,6 +208,56 @@ int grouped_kp(int n, int nsb, int max_segments) {
     return best;
 }
 
+// Shared memory of a launch: false when two segment buffers and two tiles per warp do not fit; what is left goes to the
+// tile rings first. row_bytes: what the four lanes of a token read side by side.
+static bool grouped_plan(int kp, int image_bytes, int row_bytes, int tile_bytes, GroupedArgs &a, size_t &smem) {
+    a.kp = kp;
+    a.image_bytes = image_bytes;
+    a.smem_stride = (image_bytes + 127 - row_bytes) / 128 * 128 + row_bytes;
+    a.off_ring = GS_CTRL_BYTES + (kp > 1 ? GS_PART_BYTES : 0);
+    const int room = MM_SMEM_LIMIT - a.off_ring, buf_bytes = 8 * a.smem_stride, ring_bytes = GS_WARPS * tile_bytes;
+    a.ring = (room - 2 * buf_bytes) / ring_bytes;
+    if (a.ring > GS_MAX_RING) a.ring = GS_MAX_RING;
+    if (room < 2 * buf_bytes || a.ring < 2) return false;
+    a.bufs = (room - a.ring * ring_bytes) / buf_bytes;
+    if (a.bufs > GS_MAX_BUFS) a.bufs = GS_MAX_BUFS;
+    a.off_bufs = a.off_ring + a.ring * ring_bytes;
+    smem = a.off_bufs + static_cast<size_t>(a.bufs) * 8 * a.smem_stride;
+    return true;
+}
+
+static bool plan_gate_up(int fmt, int n, int k, int x_dtype, int max_segments, GroupedArgs &a, size_t &smem) {
+    const int image_bytes = direct_token_image_bytes(k, x_dtype);
+    return image_bytes && n % 16 == 0 &&
+           grouped_plan(grouped_kp(n, k / 256, max_segments), image_bytes, 32, fmt == B200Q_Q5_K ? Q5T_TILE_BYTES : Q4T_TILE_BYTES, a, smem);
+}
+static bool plan_down(int fmt, int n, int k, int max_segments, GroupedArgs &a, size_t &smem) {
+    const int image_bytes = hidden_image_bytes(k);
+    return image_bytes && n % 16 == 0 &&
+           grouped_plan(grouped_kp(n, k / 256, max_segments), image_bytes, 64, fmt == B200Q_Q8_0_TILED ? Q8T_TILE_BYTES : Q6T_TILE_BYTES, a, smem);
+}
+
+// Where streaming, the images' conversion included, is the faster one (device time of the two launches against the
+// block-structured kernel's, 148 SMs; nine shapes of 64-512 experts, 2-512 tokens):
+//   gate/up from 113 segments on: 512 experts of 512 x 2048, top 11, BF16: 8 tokens (99 segments) 1.02, 16 (198) 0.98,
+//     64 0.92, 256 0.92; 128 of 256 x 2048: 72 segments 1.02, 144 0.89; 64 of 2048 x 2048: 84 segments 1.06, 144 0.98.
+//   down from 41 segments on, up to 1024 columns: 512 of 1024 x 512 (Q6_K): 37 segments 1.21, 49 0.86, 688 0.88; 64 of
+//     2048 x 1024: 45 segments 0.85; wider rows leave two tiles per warp and lose (64 of 1024 x 1536: 1.07-1.15).
+//   Q8_0 (tiles a third larger, less to decode) with one super-block per row 0.92-1.06, with two above 256 segments
+//     0.96-1.04: left to the block-structured kernel; 512 of 2048 x 512: 198 segments 0.83, 128 of 2048 x 768: 0.70-0.99.
+int grouped_gate_up_kp(int fmt, int n, int k, int x_dtype, int max_segments) {
+    GroupedArgs a{};
+    size_t smem = 0;
+    return max_segments > 112 && plan_gate_up(fmt, n, k, x_dtype, max_segments, a, smem) ? a.kp : 0;
+}
+int grouped_down_kp(int fmt, int n, int k, int max_segments) {
+    GroupedArgs a{};
+    size_t smem = 0;
+    if (max_segments <= 40 || k > 1024) return 0;
+    if (fmt == B200Q_Q8_0_TILED && (k < 512 || (k == 512 && max_segments > 256))) return 0;
+    return plan_down(fmt, n, k, max_segments, a, smem) ? a.kp : 0;
+}
+
 int hidden_image_bytes(int k) { return k > 0 && k % 256 == 0 && k <= 8192 ? k * 4 + 16 : 0; }
 
 int hidden_images(const float *h, int rows, int k, void *images, cudaStream_t stream) {
@@ -219,29 +268,15 @@ int hidden_images(const float *h, int rows, int k, void *images, cudaStream_t st
     return check_launch("hidden images");
 }
 
-// Fills the shared part of the arguments (row_bytes: what the four lanes of a token read side by side); false when two segment buffers do not fit in shared memory.
-static bool grouped_args(const MmaRequest &q, int image_bytes, int row_bytes, int tile_bytes, GroupedArgs &a, size_t &smem) {
+static bool grouped_args(const MmaRequest &q, GroupedArgs &a) {
     a.wa = q.wa; a.wb = q.wb; a.stride_a = q.stride_a; a.stride_b = q.stride_b;
     a.table_a = q.table_a; a.table_b = q.table_b;
-    a.n = q.n; a.nsb = q.k / 256; a.kp = grouped_kp(q.n, a.nsb, q.max_segments);
+    a.n = q.n; a.nsb = q.k / 256;
     a.images = static_cast<const uint8_t *>(q.images);
-    a.image_bytes = image_bytes;
-    a.smem_stride = (image_bytes + 127 - row_bytes) / 128 * 128 + row_bytes;
-    // two segment buffers and two tiles per warp at least; what is left goes to the tile rings first
-    a.off_ring = GS_CTRL_BYTES + (a.kp > 1 ? GS_PART_BYTES : 0);
-    const int room = MM_SMEM_LIMIT - a.off_ring, buf_bytes = 8 * a.smem_stride, ring_bytes = GS_WARPS * tile_bytes;
-    a.bufs = 2;
-    a.ring = (room - 2 * buf_bytes) / ring_bytes;
-    if (a.ring > GS_MAX_RING) a.ring = GS_MAX_RING;
-    if (room < 2 * buf_bytes || a.ring < 2) return false;
-    a.bufs = (room - a.ring * ring_bytes) / buf_bytes;
-    if (a.bufs > GS_MAX_BUFS) a.bufs = GS_MAX_BUFS;
-    a.off_bufs = a.off_ring + a.ring * ring_bytes;
     a.topk = q.topk; a.order = q.order; a.seg_expert = q.seg_expert; a.seg_begin = q.seg_begin; a.seg_count = q.seg_count;
     a.num_segments = q.num_segments; a.max_segments = q.max_segments; a.y = static_cast<float *>(q.y); a.route = q.route;
     a.flat_rows = q.flat_rows; a.y_table = q.y_table; a.rows_per_rank = q.rows_per_rank;
     a.status = device_status_word();
-    smem = a.off_bufs + static_cast<size_t>(a.bufs) * 8 * a.smem_stride;
     return a.status != nullptr;
 }
 
@@ -256,12 +291,12 @@ static int launch_grouped(void (*fn)(const GroupedArgs), const GroupedArgs &a, s
 
 int grouped_gate_up_launch(const MmaRequest &q, cudaStream_t stream, bool *launched) {
     *launched = false;
+    if (!q.images || !q.tiled || (reinterpret_cast<uintptr_t>(q.images) & 15) ||
+        !grouped_gate_up_kp(q.fmt_a, q.n, q.k, q.x_dtype, q.max_segments))
+        return B200Q_OK;
     GroupedArgs a{};
     size_t smem = 0;
-    const int image_bytes = direct_token_image_bytes(q.k, q.x_dtype);
-    if (!q.images || !q.tiled || image_bytes == 0 || (reinterpret_cast<uintptr_t>(q.images) & 15) || q.max_segments <= GROUPED_FEW_SEGMENTS)
-        return B200Q_OK;
-    if (!grouped_args(q, image_bytes, 32, q.fmt_a == B200Q_Q5_K ? Q5T_TILE_BYTES : Q4T_TILE_BYTES, a, smem)) return B200Q_OK;
+    if (!plan_gate_up(q.fmt_a, q.n, q.k, q.x_dtype, q.max_segments, a, smem) || !grouped_args(q, a)) return B200Q_OK;
     const bool two = q.x_dtype == B200Q_F32, q5 = q.fmt_a == B200Q_Q5_K;
     auto fn = q5 ? (two ? grouped_gate_up_kernel<true, 2> : grouped_gate_up_kernel<true, 1>)
                  : (two ? grouped_gate_up_kernel<false, 2> : grouped_gate_up_kernel<false, 1>);
@@ -271,11 +306,10 @@ int grouped_gate_up_launch(const MmaRequest &q, cudaStream_t stream, bool *launc
 
 int grouped_down_launch(const MmaRequest &q, cudaStream_t stream, bool *launched) {
     *launched = false;
+    if (!q.images || (reinterpret_cast<uintptr_t>(q.images) & 15) || !grouped_down_kp(q.fmt_a, q.n, q.k, q.max_segments)) return B200Q_OK;
     GroupedArgs a{};
     size_t smem = 0;
-    if (!q.images || hidden_image_bytes(q.k) == 0 || (reinterpret_cast<uintptr_t>(q.images) & 15) || q.max_segments <= GROUPED_FEW_SEGMENTS)
-        return B200Q_OK;
-    if (!grouped_args(q, hidden_image_bytes(q.k), 64, q.fmt_a == B200Q_Q8_0_TILED ? Q8T_TILE_BYTES : Q6T_TILE_BYTES, a, smem)) return B200Q_OK;
+    if (!plan_down(q.fmt_a, q.n, q.k, q.max_segments, a, smem) || !grouped_args(q, a)) return B200Q_OK;
     *launched = true;
     return launch_grouped(q.fmt_a == B200Q_Q8_0_TILED ? grouped_down_kernel<Q8Tile> : grouped_down_kernel<Q6Tile>, a, smem, stream,
                           "grouped down");

@@ -32,7 +32,7 @@ struct Api {
     FN(last_error); FN(gemv); FN(gemm); FN(gemm_ws); FN(gemm_workspace_bytes); FN(gemm_supported); FN(rmsnorm);
     FN(residual_rmsnorm); FN(gemv_norm); FN(gemv_norm_supported); FN(router_logits_t); FN(router_topk_ex);
     FN(router_topk_plan_row); FN(shared_gate); FN(moe_plan_ex); FN(moe_token_image_bytes); FN(moe_token_images);
-    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
+    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_gate_up_streams); FN(moe_down_streams); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
     FN(prefill_attention); FN(embed_rows);
 #undef FN
 } api;
@@ -43,7 +43,7 @@ void bind(const py::dict &addresses, py::object error_type) {
     FN(last_error); FN(gemv); FN(gemm); FN(gemm_ws); FN(gemm_workspace_bytes); FN(gemm_supported); FN(rmsnorm);
     FN(residual_rmsnorm); FN(gemv_norm); FN(gemv_norm_supported); FN(router_logits_t); FN(router_topk_ex);
     FN(router_topk_plan_row); FN(shared_gate); FN(moe_plan_ex); FN(moe_token_image_bytes); FN(moe_token_images);
-    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
+    FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_gate_up_streams); FN(moe_down_streams); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
     FN(prefill_attention); FN(embed_rows);
 #undef FN
     b200q_error = error_type.release().ptr();
@@ -137,7 +137,7 @@ struct Carver {
 };
 
 constexpr int SEGMENT_CAP = 8;          // tokens of one expert per pass of the grouped kernels
-constexpr int TOKEN_IMAGE_MIN_ROWS = 2;
+constexpr int TOKEN_IMAGE_MIN_ROWS = 32;  // of moe_ops: images for the block-structured gate/up kernels
 
 struct MoeLayer {
     at::Tensor router, bias, gate_vector;               // [E, D] FP32; bias / shared-expert gate may be undefined
@@ -155,9 +155,10 @@ struct MoeLayer {
         const int max_segments = std::min(plan_experts, total) + total / SEGMENT_CAP;
         const bool q45 = gate_fmt == up_fmt && (gate_fmt == B200Q_Q4_K || gate_fmt == B200Q_Q5_K ||
                                                 gate_fmt == B200Q_Q4_K_TILED || gate_fmt == B200Q_Q5_K_TILED);
-        const bool images = t >= TOKEN_IMAGE_MIN_ROWS && !env_is("B200Q_TOKEN_IMAGES", "0");
-        const int image_bytes = q45 && images ? std::max(0, api.moe_token_image_bytes(d, xdt)) : 0;
-        const int hidden_bytes = images && (down_fmt == B200Q_Q6_K_TILED || down_fmt == B200Q_Q8_0_TILED) ? api.moe_hidden_image_bytes(f) : 0;
+        const bool images = !env_is("B200Q_TOKEN_IMAGES", "0");
+        const int image_bytes = images && q45 && (t >= TOKEN_IMAGE_MIN_ROWS || api.moe_gate_up_streams(gate_fmt, f, d, xdt, max_segments))
+                                    ? std::max(0, api.moe_token_image_bytes(d, xdt)) : 0;
+        const int hidden_bytes = images && api.moe_down_streams(down_fmt, d, f, max_segments) ? api.moe_hidden_image_bytes(f) : 0;
         Carver c;
         const size_t o_logits = c.take(sizeof(float) * t * experts), o_weights = c.take(sizeof(float) * total),
                      o_ids = c.take(sizeof(int64_t) * total), o_scale = c.take(sizeof(float) * t),

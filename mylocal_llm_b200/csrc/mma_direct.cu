@@ -76,7 +76,8 @@ bool direct_plan_args(const MmaRequest &q, DirectArgs *out, long long *smem_out)
         if (most(kp) > sm_count() && most(kp) <= 2LL * sm_count())
             while (kp > 1 && most(kp) > sm_count()) kp /= 2;
     }
-    if (grouped && q.max_segments > GROUPED_FEW_SEGMENTS) kp = grouped_kp(q.n, nsb, q.max_segments);
+    if (q.mode == 2 && q.tiled)
+        if (const int parts = grouped_gate_up_kp(q.fmt_a, q.n, q.k, q.x_dtype, q.max_segments)) kp = parts;
     a.kp = kp;
     a.rg = MD_WARPS / kp;
     a.off_bfrag = MD_CTRL_BYTES + token_tiles * MD_PART_BYTES;

@@ -56,10 +56,13 @@ int direct_tokens_per_pass(int fmt, int mode, int k, int x_dtype);
 int direct_token_image_bytes(int k, int x_dtype);
 int direct_token_images(const void *x, int x_dtype, int rows, int k, void *images, cudaStream_t stream);
 
-// Grouped launches over images (grouped_stream.cu): plans of more segments than a single decoded row's; *launched stays
-// false where they do not apply and the block-structured kernels take the request.
-constexpr int GROUPED_FEW_SEGMENTS = 16;
-int grouped_kp(int n, int nsb, int max_segments);
+// Grouped launches over images (grouped_stream.cu). grouped_*_kp: the warps per row group with which a plan of that bound
+// streams (fmt: B200Q_Q4_K / Q5_K tiles for gate/up, B200Q_Q6_K_TILED / Q8_0_TILED for down), 0 where the block-structured
+// kernels are the better ones or two segment buffers do not fit; a function of types, sizes and the bound alone, so that
+// the block-structured kernels take the same kp when such a plan comes without images (or with peers' rows) and add in the
+// same order. *launched stays false where the request does not stream.
+int grouped_gate_up_kp(int fmt, int n, int k, int x_dtype, int max_segments);
+int grouped_down_kp(int fmt, int n, int k, int max_segments);
 int grouped_gate_up_launch(const MmaRequest &q, cudaStream_t stream, bool *launched);
 int grouped_down_launch(const MmaRequest &q, cudaStream_t stream, bool *launched);
 int hidden_image_bytes(int k);

@@ -207,7 +207,7 @@ int tiled_plan_args(const MmaRequest &q, Q6TiledArgs *out, long long *smem_out) 
         };
         if (most(kp) > sm_count() && most(kp) <= 2LL * sm_count())
             while (kp > 1 && most(kp) > sm_count()) kp /= 2;
-        if (q.max_segments > GROUPED_FEW_SEGMENTS) kp = grouped_kp(q.n, nsb, q.max_segments);
+        if (const int parts = grouped_down_kp(q.fmt_a, q.n, q.k, q.max_segments)) kp = parts;
     }
     a.kp = kp;
     a.rg = Q6T_WARPS / kp;

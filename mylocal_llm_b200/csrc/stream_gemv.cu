@@ -437,6 +437,15 @@ int b200q_moe_down(const void *down_base, int64_t down_stride, int down_fmt, con
 
 int b200q_moe_hidden_image_bytes(int f) { return hidden_image_bytes(f); }
 
+int b200q_moe_gate_up_streams(int fmt, int f, int d, int x_dtype, int max_segments) {
+    return direct_tiled_base(fmt) >= 0 && f > 0 && d > 0 &&
+           grouped_gate_up_kp(direct_tiled_base(fmt), f, d, x_dtype, max_segments) > 0;
+}
+
+int b200q_moe_down_streams(int fmt, int d, int f, int max_segments) {
+    return (fmt == B200Q_Q6_K_TILED || fmt == B200Q_Q8_0_TILED) && f > 0 && d > 0 && grouped_down_kp(fmt, d, f, max_segments) > 0;
+}
+
 int b200q_moe_hidden_images(const float *hbuf, int rows, int f, void *images, void *stream) {
     if (!hbuf || !images) return fail(B200Q_EINVAL, "moe_hidden_images: NULL pointer");
     if (rows <= 0 || f <= 0) return fail(B200Q_EINVAL, "moe_hidden_images: bad shape rows=%d f=%d", rows, f);

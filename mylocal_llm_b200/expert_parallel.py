@@ -320,7 +320,7 @@ class DeviceExpertEngine:
             return None
         terms = torch.zeros((ids.shape[0] * ids.shape[1], bank.d_model), dtype=torch.float32, device=x_all.device)
         moe_ops.moe_down(hbuf, route, plan, None, bank.down_type, bank.d_model, bank.d_ff, 0,
-                         down_table=self.tables[2], tables_aligned16=self.aligned, flat_rows=True, out=terms)
+                         down_table=self.tables[2], tables_aligned16=self.aligned, flat_rows=True, out=terms, images=False)
         _phase("down")
         return terms
 

@@ -155,9 +155,10 @@ def router_topk_plan_row(logits2d, k, n_experts, *, renormalize=True, floor=2.0 
     return weights, ids, plan
 
 
-# Rows of activations from which the grouped launches are fed with images (one small launch before each that converts
-# every row once; a single row's plan of a few one-token segments converts its row itself).
-TOKEN_IMAGE_MIN_ROWS = 2
+# Rows of activations from which the block-structured grouped gate/up launch is fed with per-token images (one extra small
+# launch that converts every row once; below this the segments convert their few tokens themselves). The streaming
+# launches read nothing else and take images whatever the rows (``b200q_moe_gate_up_streams`` / ``_down_streams``).
+TOKEN_IMAGE_MIN_ROWS = 32
 
 
 def token_images(x2d):
@@ -181,14 +182,16 @@ def moe_gate_up(x2d, plan, gate_bank, up_bank, gate_fmt, up_fmt, f, d, gate_stri
 
     Experts live either in contiguous banks (``*_bank`` + byte stride) or behind device pointer
     tables (int64 tensors with one address per expert). ``images`` = ``token_images(x2d)``; by default they
-    are made here when ``x2d`` has at least ``TOKEN_IMAGE_MIN_ROWS`` rows (``B200Q_TOKEN_IMAGES=0`` or
-    ``images=False`` turns that off). The results are the same bits either way."""
+    are made here when ``x2d`` has at least ``TOKEN_IMAGE_MIN_ROWS`` rows or the launch streams
+    (``B200Q_TOKEN_IMAGES=0`` or ``images=False`` turns that off). The results are the same bits either way."""
     torch = _torch()
     hbuf = torch.empty((plan.rows * plan.k, f), dtype=torch.float32, device=x2d.device)
     if images is False:          # the caller knows its plan executes too few of the rows for images to pay
         images = None
-    elif images is None and x2d.shape[0] >= TOKEN_IMAGE_MIN_ROWS and os.environ.get("B200Q_TOKEN_IMAGES", "1") != "0" \
-            and gate_fmt in ("Q4_K", "Q5_K", "Q4_K_TILED", "Q5_K_TILED") and gate_fmt == up_fmt:
+    elif images is None and os.environ.get("B200Q_TOKEN_IMAGES", "1") != "0" \
+            and gate_fmt in ("Q4_K", "Q5_K", "Q4_K_TILED", "Q5_K_TILED") and gate_fmt == up_fmt \
+            and (x2d.shape[0] >= TOKEN_IMAGE_MIN_ROWS or _lib.load().b200q_moe_gate_up_streams(
+                _lib.FORMAT_ID[gate_fmt], int(f), int(d), _dtype_id(x2d), plan.max_segments)):
         images = token_images(x2d)
     if images is not None:
         _lib.call("b200q_moe_gate_up_images", _ptr(gate_bank), int(gate_stride), _lib.FORMAT_ID[gate_fmt],
@@ -206,25 +209,27 @@ def moe_gate_up(x2d, plan, gate_bank, up_bank, gate_fmt, up_fmt, f, d, gate_stri
 
 
 def moe_down(hbuf, route_weights, plan, down_bank, down_fmt, d, f, down_stride, *, down_table=None,
-             tables_aligned16=False, flat_rows=False, out=None):
+             tables_aligned16=False, flat_rows=False, out=None, images=None):
     """Route-weighted FP32 terms ``[T*k, D]`` in sorted-assignment order, or (``flat_rows``) at the
-    flat assignment index ``row*k+slot``; ``out`` lets the caller supply (and pre-zero) the buffer."""
+    flat assignment index ``row*k+slot``; ``out`` lets the caller supply (and pre-zero) the buffer. ``images=False``: do not
+    convert the rows of ``hbuf`` ahead of the launch (the plan executes few of them)."""
     torch = _torch()
     if route_weights.dtype != torch.float32 or not route_weights.is_contiguous():
         raise ValueError("routing weights must be a contiguous FP32 tensor")
     terms = out if out is not None else torch.empty((plan.rows * plan.k, d), dtype=torch.float32,
                                                      device=hbuf.device)
-    # the tile-layout kernels of larger plans read images of the hidden rows (made here; the same bits either way)
-    if plan.rows >= TOKEN_IMAGE_MIN_ROWS and down_fmt in ("Q6_K_TILED", "Q8_0_TILED") and os.environ.get("B200Q_TOKEN_IMAGES", "1") != "0":
+    # a launch that streams reads images of the hidden rows (made here; the same bits either way)
+    if (images is not False and os.environ.get("B200Q_TOKEN_IMAGES", "1") != "0" and hbuf.data_ptr() % 16 == 0
+            and _lib.load().b200q_moe_down_streams(_lib.FORMAT_ID[down_fmt], int(d), int(f), plan.max_segments)):
         per_row = _lib.load().b200q_moe_hidden_image_bytes(int(f))
-        if per_row:
-            images = torch.empty((plan.rows * plan.k, per_row), dtype=torch.uint8, device=hbuf.device)
-            _lib.call("b200q_moe_hidden_images", _ptr(hbuf), plan.rows * plan.k, f, _ptr(images), _lib.current_stream())
-            _lib.call("b200q_moe_down_images", _ptr(down_bank), int(down_stride), _lib.FORMAT_ID[down_fmt], _ptr(down_table),
-                      1 if tables_aligned16 else 0, 1 if flat_rows else 0, d, f, _ptr(hbuf), _ptr(images), _ptr(route_weights),
-                      _ptr(plan.order), _ptr(plan.seg_expert), _ptr(plan.seg_begin), _ptr(plan.seg_count),
-                      _ptr(plan.num_segments), plan.max_segments, _ptr(terms), _lib.current_stream())
-            return terms
+        rows = hbuf.numel() // f
+        images = torch.empty((rows, per_row), dtype=torch.uint8, device=hbuf.device)
+        _lib.call("b200q_moe_hidden_images", _ptr(hbuf), rows, f, _ptr(images), _lib.current_stream())
+        _lib.call("b200q_moe_down_images", _ptr(down_bank), int(down_stride), _lib.FORMAT_ID[down_fmt], _ptr(down_table),
+                  1 if tables_aligned16 else 0, 1 if flat_rows else 0, d, f, _ptr(hbuf), _ptr(images), _ptr(route_weights),
+                  _ptr(plan.order), _ptr(plan.seg_expert), _ptr(plan.seg_begin), _ptr(plan.seg_count),
+                  _ptr(plan.num_segments), plan.max_segments, _ptr(terms), _lib.current_stream())
+        return terms
     _lib.call("b200q_moe_down", _ptr(down_bank), int(down_stride), _lib.FORMAT_ID[down_fmt], _ptr(down_table),
               1 if tables_aligned16 else 0, 1 if flat_rows else 0, d, f, _ptr(hbuf),
               _ptr(route_weights), _ptr(plan.order), _ptr(plan.seg_expert), _ptr(plan.seg_begin),

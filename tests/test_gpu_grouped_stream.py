@@ -4,7 +4,7 @@ many row groups per segment (fewer than a CTA has teams included), one to nine s
 
 import pytest
 
-from mylocal_llm_b200 import moe_ops
+from mylocal_llm_b200 import _lib, moe_ops
 from mylocal_llm_b200.quantize import random_packed
 from mylocal_llm_b200.quantized_linear import retile_bytes
 
@@ -25,7 +25,7 @@ def both(monkeypatch, run):
     return images, plain
 
 
-@pytest.mark.parametrize("tokens,e,k", [(17, 7, 2), (40, 24, 4), (33, 120, 3), (64, 96, 6), (256, 40, 8)])
+@pytest.mark.parametrize("tokens,e,k", [(17, 7, 2), (40, 24, 4), (33, 120, 3), (64, 96, 6), (256, 40, 8), (45, 120, 3), (70, 300, 3)])
 @pytest.mark.parametrize("d,f", [(256, 16), (2048, 48), (768, 512), (2304, 256)])
 def test_same_bits_as_the_block_kernels(cuda, monkeypatch, tokens, e, k, d, f):
     torch = cuda
@@ -48,3 +48,28 @@ def test_same_bits_as_the_block_kernels(cuda, monkeypatch, tokens, e, k, d, f):
         for flat in (False, True):
             a, b = both(monkeypatch, lambda: moe_ops.moe_down(hidden, route, plan, down, fmt + "_TILED", d, wide, stride, flat_rows=flat))
             assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("tokens,e,k,d,f,fmts,gate_up,down", [
+    (2, 64, 5, 1024, 512, ("Q4_K", "Q6_K"), 0, 0),             # 11 segments at most: the block-structured kernels
+    (8, 64, 5, 1024, 512, ("Q4_K", "Q6_K"), 0, 1),             # 45
+    (8, 64, 5, 1024, 512, ("Q4_K", "Q8_0"), 0, 1),
+    (24, 64, 5, 1024, 2048, ("Q5_K", "Q6_K"), 0, 0),           # rows of 2048 hidden values: no room for the tile rings
+    (32, 64, 5, 1024, 512, ("Q4_K", "Q6_K"), 1, 1),            # 84: token images for the block-structured gate/up
+    (16, 512, 11, 1024, 512, ("Q4_K", "Q6_K"), 1, 1),          # 198: both stream
+])
+def test_images_are_made_for_the_launches_that_read_them(cuda, tokens, e, k, d, f, fmts, gate_up, down):
+    torch = cuda
+    ids = torch.rand((tokens, e), device="cuda").topk(k, dim=1).indices.contiguous()
+    plan = moe_ops.moe_plan(ids, e)
+    x = torch.randn((tokens, d), device="cuda").bfloat16()
+    (gate, stride), (up, _), (down_bank, down_stride) = (bank(torch, fmt, e, n, w, s) for fmt, n, w, s in (
+        (fmts[0], f, d, 1), (fmts[0], f, d, 2), (fmts[1], d, f, 3)))
+    real, calls = _lib.call, []
+    _lib.call = lambda name, *a: (calls.append(name), real(name, *a))[1]
+    try:
+        hidden = moe_ops.moe_gate_up(x, plan, gate, up, fmts[0] + "_TILED", fmts[0] + "_TILED", f, d, stride, stride)
+        moe_ops.moe_down(hidden, torch.rand((tokens, k), device="cuda"), plan, down_bank, fmts[1] + "_TILED", d, f, down_stride)
+    finally:
+        _lib.call = real
+    assert (calls.count("b200q_moe_token_images"), calls.count("b200q_moe_hidden_images")) == (gate_up, down)
