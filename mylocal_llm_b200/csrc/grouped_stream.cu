@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) grouped_down_kernel(const Group
             if (!stream.next(tile)) return false;
             T::read(r, tile, lane);
             stream.refill(lane);
-            T::template mma<2, 1>(r, frag, tot);
+            T::template mma<2, 1, 8>(r, frag, tot);
             fp += a.kp * 512;
         }
         if (!add_parts(tot[0], partial, pbuf, a.kp, team, kpi, warp, lane)) return true;
@@ -239,8 +239,9 @@ static bool plan_down(int fmt, int n, int k, int max_segments, GroupedArgs &a, s
 
 // Where streaming, the images' conversion included, is the faster one (device time of the two launches against the
 // block-structured kernel's, 148 SMs; nine shapes of 64-512 experts, 2-512 tokens):
-//   gate/up from 113 segments on: 512 experts of 512 x 2048, top 11, BF16: 8 tokens (99 segments) 1.02, 16 (198) 0.98,
-//     64 0.92, 256 0.92; 128 of 256 x 2048: 72 segments 1.02, 144 0.89; 64 of 2048 x 2048: 84 segments 1.06, 144 0.98.
+//   gate/up from 113 segments and 162 tiles of each matrix per SM on: 512 experts of 512 x 2048, top 11, BF16: 8 tokens
+//     (99 segments) 1.02, 16 (198) 0.90, 64 0.91, 256 0.93; 64 of 2048 x 2048: 84 segments 1.06, 125 0.93; 128 of
+//     512 x 1024: 169 segments (146 tiles) 1.06, 189 (163) 0.91.
 //   down from 41 segments on, up to 1024 columns: 512 of 1024 x 512 (Q6_K): 37 segments 1.21, 49 0.86, 688 0.88; 64 of
 //     2048 x 1024: 45 segments 0.85; wider rows leave two tiles per warp and lose (64 of 1024 x 1536: 1.07-1.15).
 //   Q8_0 (tiles a third larger, less to decode) with one super-block per row 0.92-1.06, with two above 256 segments
@@ -248,7 +249,8 @@ static bool plan_down(int fmt, int n, int k, int max_segments, GroupedArgs &a, s
 int grouped_gate_up_kp(int fmt, int n, int k, int x_dtype, int max_segments) {
     GroupedArgs a{};
     size_t smem = 0;
-    return max_segments > 112 && plan_gate_up(fmt, n, k, x_dtype, max_segments, a, smem) ? a.kp : 0;
+    if (max_segments <= 112 || static_cast<long long>(max_segments) * (n / 16) * (k / 256) < 162LL * sm_count()) return 0;
+    return plan_gate_up(fmt, n, k, x_dtype, max_segments, a, smem) ? a.kp : 0;
 }
 int grouped_down_kp(int fmt, int n, int k, int max_segments) {
     GroupedArgs a{};

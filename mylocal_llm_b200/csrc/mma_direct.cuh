@@ -224,6 +224,13 @@ __device__ __forceinline__ int direct_entry(int p, int t) {
     const int f = (p >> 8) * 16 + ((sub >> 2) * 2 + (sub & 1)) * 4 + ((p >> 2) & 3);
     return f * 32 + 4 * t + tig;
 }
+// The same in the natural order of the Q6_K / Q8_0 tiles: fragment f = p >> 4, lane 4t + ((p >> 2) & 3); the fragments
+// behind one another, or PAIRED: two of them side by side.
+template <bool PAIRED>
+__device__ __forceinline__ int natural_entry(int p, int t) {
+    const int lane = 4 * t + ((p >> 2) & 3);
+    return PAIRED ? ((p >> 5) * 32 + lane) * 2 + ((p >> 4) & 1) : (p >> 4) * 32 + lane;
+}
 // Four consecutive activations starting at element index e (a multiple of 4) as floats.
 // `vec_ok` tells whether the tensor allows aligned vector loads.
 __device__ __forceinline__ void load4(const void *x, int x_dtype, size_t e, bool vec_ok, float (&v)[4]) {
@@ -431,9 +438,10 @@ __device__ __forceinline__ void chunk_values(const RawChunk<NTERMS> &r, bool f16
 // waits for it. Launches of 8 tokens: Q4_K [8192 x 2048] 11.7 -> 8.7 us, Q8_0 [2048 x 8192] 27.7 -> 14.6 us; 16 tokens,
 // Q8_0 [2048 x 2048] 14.6 -> 8.8 us. Up to MD_FEW_CHUNKS chunks per thread the short code above is the faster one: these copies of a chunk's
 // code cost about 1 us of instruction fetch in a launch that uses one or two of them.
-// SUMS: also the activation sums of the sub-blocks.
+// SUMS: this kernel's order, and the activation sums of the sub-blocks; else the natural order of q6k_tiled.cuh, PAIRED or
+// not.
 constexpr int MD_FEW_CHUNKS = 4;
-template <int NTERMS, int BATCH, bool SUMS, int THREADS, int BARRIER, typename RowFn>
+template <int NTERMS, int BATCH, bool SUMS, bool PAIRED, int THREADS, int BARRIER, typename RowFn>
 __device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k, const void *x, int x_dtype,
                                                uint2 *bfrag, uint32_t *xsfrag, float *tok_scale, int tid) {
     const int lane = tid & 31;
@@ -489,8 +497,7 @@ __device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k
         tok_scale[8 + tid] = 1.0f / s;
     }
     named_barrier_sync(BARRIER, THREADS);
-    // 2. scale, split, store: with the sums in this kernel's order, else in the natural one of q6k_tiled.cuh (fragment
-    //    f = p>>4, lane 4t + ((p>>2)&3))
+    // 2. scale, split, store
     auto store_chunk = [&](int c0, const RawChunk<NTERMS> &r) {
         const int t = token_of(c0);
         const int p = (c0 + lane - t * chunks_per_token) * 4;
@@ -511,7 +518,7 @@ __device__ __forceinline__ void prepare_tokens(RowFn row_of, int m_tokens, int k
                 if (SUMS) sum += __half2float(l);
             }
         }
-        const int entry = SUMS ? direct_entry(p, t) : ((p >> 5) * 32 + 4 * t + ((p >> 2) & 3)) * 2 + ((p >> 4) & 1);
+        const int entry = SUMS ? direct_entry(p, t) : natural_entry<PAIRED>(p, t);
         bfrag[entry] = make_uint2(hi[0] | (static_cast<uint32_t>(hi[2]) << 16), hi[1] | (static_cast<uint32_t>(hi[3]) << 16));
         if (NTERMS == 2)
             bfrag[nfrag * 32 + entry] = make_uint2(lo[0] | (static_cast<uint32_t>(lo[2]) << 16), lo[1] | (static_cast<uint32_t>(lo[3]) << 16));
@@ -796,7 +803,7 @@ __device__ __forceinline__ void mma_direct_body(const DirectArgs &a, const Stage
             const auto row_of = [nt](int t) { return 8 * nt + t; };
             const int tokens = max(min(a.m - 8 * nt, 8), 0);
             if (NT == 2 || tokens * (a.k >> 2) > MD_FEW_CHUNKS * MD_THREADS)
-                prepare_tokens<NTERMS, 8, true, MD_THREADS, 1>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * btile,
+                prepare_tokens<NTERMS, 8, true, false, MD_THREADS, 1>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * btile,
                                                                xsfrag + nt * xtile, tok_scale + nt * MD_TOK_STRIDE, tid);
             else
                 prepare_direct<NTERMS, MD_FEW_CHUNKS>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * btile,

@@ -136,9 +136,11 @@ __device__ __forceinline__ void biased_bytes_to_float2(uint32_t wa, uint32_t wb,
 }
 
 // One tile: 16 scale groups = 16 mma steps; tot += d * sum_s scale_s * (codes_s . x_s). frag(nt, pair, plane) points to the
-// lane's 16 bytes of fragments 2 pair, 2 pair + 1 of the tile (plane 0: FP16 high parts, 1: remainders) of token tile nt:
-// every decoded A operand is multiplied into each token tile, so the decode cost is paid once per 8*NT tokens.
-template <int NTERMS, int NT, typename FragFn>
+// lane's entry of fragment 2 pair of the tile (plane 0: FP16 high parts, 1: remainders) of token tile nt, that of 2 pair + 1
+// lies STEP bytes on (8: paired, 256: behind one another; eight-byte reads of pairs are two-way bank conflicts, 2-5 % of a
+// grouped launch): every decoded A operand is multiplied into each token tile, so the decode cost is paid once per 8*NT
+// tokens.
+template <int NTERMS, int NT, int STEP, typename FragFn>
 __device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const FragFn frag, float (&tot)[NT][4]) {
     const uint32_t magic = 0x64006400u, neg = 0xe420e420u;       // 1024 | code ; -(1024 + 32)
     const uint32_t wa[12] = {r.c[0].x, r.c[0].y, r.c[0].z, r.c[0].w, r.c[1].x, r.c[1].y,
@@ -179,10 +181,10 @@ __device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const FragFn fr
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 float acc[4];
-                const uint2 bh = *reinterpret_cast<const uint2 *>(frag(nt, s >> 1, 0) + 8 * (s & 1));
+                const uint2 bh = *reinterpret_cast<const uint2 *>(frag(nt, s >> 1, 0) + STEP * (s & 1));
                 mma_f16_first(acc, a0, a1, a2, a3, bh.x, bh.y);
                 if (NTERMS == 2) {
-                    const uint2 bl = *reinterpret_cast<const uint2 *>(frag(nt, s >> 1, 1) + 8 * (s & 1));
+                    const uint2 bl = *reinterpret_cast<const uint2 *>(frag(nt, s >> 1, 1) + STEP * (s & 1));
                     mma_f16(acc, a0, a1, a2, a3, bl.x, bl.y);
                 }
                 blk[nt][0] = fmaf(fa, acc[0], blk[nt][0]);
@@ -205,6 +207,7 @@ __device__ __forceinline__ void q6_tile_mma(const Q6TileRegs &r, const FragFn fr
 // Tile policies of the kernel below: bytes per 16-row x 256-value tile, the registers of one tile,
 // how a lane loads them and how it multiplies them into its four accumulators.
 struct Q6Tile {
+    static constexpr bool PAIRED = false;         // fragments in shared memory, see natural_entry
     static constexpr int BYTES = Q6T_TILE_BYTES;
     using Regs = Q6TileRegs;
     static __device__ __forceinline__ void load(Regs &r, const uint8_t *tile, int lane) { load_q6_tile(r, tile, lane); }
@@ -217,9 +220,9 @@ struct Q6Tile {
         const uint16_t *d = reinterpret_cast<const uint16_t *>(tile + Q6T_D_OFF);
         r.dd = d[g] | (static_cast<uint32_t>(d[g + 8]) << 16);
     }
-    template <int NTERMS, int NT, typename FragFn>
+    template <int NTERMS, int NT, int STEP, typename FragFn>
     static __device__ __forceinline__ void mma(const Regs &r, const FragFn frag, float (&tot)[NT][4]) {
-        q6_tile_mma<NTERMS, NT>(r, frag, tot);
+        q6_tile_mma<NTERMS, NT, STEP>(r, frag, tot);
     }
 };
 
@@ -235,6 +238,7 @@ struct Q8TileRegs {
     uint4 da, db;      // eight fp16 scales of row g / row g+8
 };
 struct Q8Tile {
+    static constexpr bool PAIRED = true;
     static constexpr int BYTES = Q8T_TILE_BYTES;
     using Regs = Q8TileRegs;
     static __device__ __forceinline__ void load(Regs &r, const uint8_t *tile, int lane) {
@@ -251,7 +255,7 @@ struct Q8Tile {
         r.da = *reinterpret_cast<const uint4 *>(tile + Q8T_SCALES_OFF + 16 * g);
         r.db = *reinterpret_cast<const uint4 *>(tile + Q8T_SCALES_OFF + 16 * (g + 8));
     }
-    template <int NTERMS, int NT, typename FragFn>
+    template <int NTERMS, int NT, int STEP, typename FragFn>       // (STEP: paired fragments only)
     static __device__ __forceinline__ void mma(const Regs &r, const FragFn frag, float (&tot)[NT][4]) {
         const uint32_t neg = 0xe480e480u;                       // -(1024 + 128)
         const uint32_t wa[16] = {r.c[0].x, r.c[0].y, r.c[0].z, r.c[0].w, r.c[1].x, r.c[1].y, r.c[1].z, r.c[1].w,
@@ -297,10 +301,9 @@ struct Q8Tile {
 };
 
 // Activation fragments in natural order: fragment f (16 positions 16f..16f+15), lane (g, tig):
-// token g, positions 16f + 4tig + {0,2} -> b0, {1,3} -> b1, the two fragments of a pair side by side as in
-// prepare_direct (uint2 entry ((f >> 1) * 32 + lane) * 2 + (f & 1)); FP16 high part (+ remainder plane for
+// token g, positions 16f + 4tig + {0,2} -> b0, {1,3} -> b1 (natural_entry); FP16 high part (+ remainder plane for
 // FP32 inputs) after a per-token power-of-two scaling. All Q6T_THREADS threads take part.
-template <int NTERMS, int KEEP, typename RowFn>
+template <int NTERMS, int KEEP, bool PAIRED, typename RowFn>
 __device__ __forceinline__ void prepare_fragments(RowFn row_of, int m_tokens, int k, const void *x, int x_dtype,
                                                   uint2 *bfrag, float *tok_scale, int tid) {
     const int lane = tid & 31;
@@ -359,7 +362,7 @@ __device__ __forceinline__ void prepare_fragments(RowFn row_of, int m_tokens, in
             hi[i] = __half_as_ushort(h);
             lo[i] = __half_as_ushort(__float2half_rn(sv - __half2float(h)));
         }
-        const int entry = ((p >> 5) * 32 + 4 * t + ((p >> 2) & 3)) * 2 + ((p >> 4) & 1);
+        const int entry = natural_entry<PAIRED>(p, t);
         bfrag[entry] = make_uint2(hi[0] | (static_cast<uint32_t>(hi[2]) << 16),
                                          hi[1] | (static_cast<uint32_t>(hi[3]) << 16));
         if (NTERMS == 2)
@@ -451,10 +454,10 @@ __device__ __forceinline__ void tiled_body(const Q6TiledArgs &a, const StagePoin
             const auto row_of = [nt](int t) { return 8 * nt + t; };
             const int tokens = max(min(a.m - 8 * nt, 8), 0);
             if (NT == 2 || tokens * (a.k >> 2) > MD_FEW_CHUNKS * Q6T_THREADS)
-                prepare_tokens<NTERMS, 8, false, Q6T_THREADS, 1>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * tile_stride,
+                prepare_tokens<NTERMS, 8, false, TILE::PAIRED, Q6T_THREADS, 1>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * tile_stride,
                                                                  nullptr, tok_scale + nt * Q6T_TOK_STRIDE, tid);
             else
-                prepare_fragments<NTERMS, MD_FEW_CHUNKS>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * tile_stride,
+                prepare_fragments<NTERMS, MD_FEW_CHUNKS, TILE::PAIRED>(row_of, tokens, a.k, gp.x, a.x_dtype, bfrag + nt * tile_stride,
                                                          tok_scale + nt * Q6T_TOK_STRIDE, tid);
         }
     }
@@ -479,7 +482,7 @@ __device__ __forceinline__ void tiled_body(const Q6TiledArgs &a, const StagePoin
                                                 a.flat_rows ? flat : seg_begin + tid);
             }
             named_barrier_sync(1, Q6T_THREADS);
-            prepare_fragments<NTERMS, 2>([&](int t) { return seg_tokens[t]; }, m_tokens, a.k, gp.x, a.x_dtype, bfrag,
+            prepare_fragments<NTERMS, 2, TILE::PAIRED>([&](int t) { return seg_tokens[t]; }, m_tokens, a.k, gp.x, a.x_dtype, bfrag,
                                       tok_scale, tid);
         }
 
@@ -492,9 +495,9 @@ __device__ __forceinline__ void tiled_body(const Q6TiledArgs &a, const StagePoin
             cur = nxt;
             if (item + 1 < items_per_block) TILE::load(nxt, cur_p + (item + 1) * item_step, lane);
             else if (has_next) TILE::load(nxt, nxt_p, lane);
-            const uint4 *bf = reinterpret_cast<const uint4 *>(bfrag) + (kpi + item * a.kp) * 256 + lane;
-            TILE::template mma<NTERMS, NT>(cur, [&](int nt, int pair, int plane) {
-                return reinterpret_cast<const uint8_t *>(bf + nt * (tile_stride >> 1) + plane * nfrag * 16 + pair * 32);
+            const uint2 *bf = bfrag + (kpi + item * a.kp) * 512 + lane * (TILE::PAIRED ? 2 : 1);
+            TILE::template mma<NTERMS, NT, TILE::PAIRED ? 8 : 256>(cur, [&](int nt, int pair, int plane) {
+                return reinterpret_cast<const uint8_t *>(bf + nt * tile_stride + plane * nfrag * 32 + pair * 64);
             }, tot);
         }
 
