@@ -119,6 +119,7 @@ int direct_try_launch(const MmaRequest &q, cudaStream_t stream, bool *launched) 
         cudaGetLastError();
         return fail(B200Q_ECUDA, "direct gemv: shared memory opt-in failed: %s", cudaGetErrorString(err));
     }
+    if (grouped) roomy_l1(reinterpret_cast<const void *>(fn));
     int grid = sm_count();
     if (!grouped) {
         const int blocks = (q.n + 16 * a.rg - 1) / (16 * a.rg);

@@ -251,6 +251,7 @@ int q6k_tiled_launch(const MmaRequest &q, cudaStream_t stream) {
         cudaGetLastError();
         return fail(B200Q_ECUDA, "tiled Q6_K: shared memory opt-in failed: %s", cudaGetErrorString(err));
     }
+    if (grouped) roomy_l1(reinterpret_cast<const void *>(fn));
     int grid = sm_count();
     if (!grouped) {
         const int blocks = (q.n / 16 + a.rg - 1) / a.rg;
