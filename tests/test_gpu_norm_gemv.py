@@ -191,3 +191,21 @@ def test_llama_one_token_step_fusions_change_no_bit(cuda, monkeypatch):
     for a, b in zip(k_got + v_got, k_want + v_want):
         assert torch.equal(a, b)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("act", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("rows,f", [(1, 4), (3, 252), (3, 256), (2, 260), (5, 1026), (70000, 64)])
+def test_silu_product_is_the_same_from_quads_and_single_elements(cuda, rows, f, act):
+    """Aligned rows of 256 columns and more go in quads; the same rows four bytes further on do not."""
+    torch = cuda
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    base = torch.randn(rows * 2 * f + 1, device="cuda")
+    out, ref = (torch.empty((rows, f), dtype=getattr(torch, act), device="cuda") for _ in range(2))
+    dt = _lib.DTYPE_ID[act]
+    _lib.call("b200q_silu_mul", ptr(base[1:]), rows, f, ptr(ref), dt, _lib.current_stream())
+    aligned = base[1:].clone()
+    _lib.call("b200q_silu_mul", ptr(aligned), rows, f, ptr(out), dt, _lib.current_stream())
+    assert torch.equal(out, ref)
+    gate, up = aligned.view(rows, 2 * f).double().split(f, dim=1)
+    want = gate / (1 + torch.exp(-gate)) * up      # FP32 exponential, quotient, products: some units in the last place
+    torch.testing.assert_close(out.double(), want, rtol={"float32": 8 * 2 ** -24, "float16": 2 ** -10, "bfloat16": 2 ** -7}[act], atol=1e-7)
