@@ -309,9 +309,10 @@ extern "C" int b200q_router_logits_t(const void *x, int x_dtype, int t, int d, c
     if (reinterpret_cast<uintptr_t>(wt) & 15) return fail(B200Q_EINVAL, "router_logits_t: weight must be 16-byte aligned");
     // Register tiles from 40960 logits on (d = 2048: 96 tokens x 512 experts 26.0 -> 12.8 us, 256 66.6 -> 24.3, 512 124 ->
     // 43; 256 tokens x 128 experts, below the line, 19.0 against 12.3). 64 x 512 is 15.3 against 12.4 alone, but an 8-layer
-    // step of that size took 1962 us with the kernel above and 1980 with the tiles; 32 x 512 8.4 against 10.6.
-    if (static_cast<long long>(t) * e >= 40960 && d <= RT_CHUNK) {
-        constexpr int R = 4, TOK = 8;
+    // step of that size took 1962 us with the kernel above and 1980 with the tiles; 32 x 512 8.4 against 10.6. Token tiles
+    // lie along grid.y: the kernel above has twice as many tokens per CTA, so the largest batches stay with it.
+    constexpr int R = 4, TOK = 8;
+    if (static_cast<long long>(t) * e >= 40960 && d <= RT_CHUNK && t <= 65535 * TOK) {
         auto fn = router_logits_tile_kernel<R, TOK>;
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, TOK * RT_CHUNK * 4) != cudaSuccess) {
             cudaGetLastError();

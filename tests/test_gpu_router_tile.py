@@ -30,3 +30,12 @@ def test_many_tokens_equal_few(cuda, t, d, e, dtype):
     odd = torch.empty(t * d + 1, dtype=x.dtype, device="cuda")[1:].view(t, d)
     odd.copy_(x)
     assert torch.equal(moe_ops.router_logits_t(odd, w, bias), many)
+
+
+@pytest.mark.parametrize("t", [65535 * 8, 65535 * 8 + 1])
+def test_the_largest_batches(cuda, t):
+    torch = cuda
+    x, w = torch.randn((t, 4), device="cuda"), torch.randn((1, 4), device="cuda")
+    got = moe_ops.router_logits_t(x, w).double()
+    ref, scale = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert ((got - ref).abs() <= scale * 7 * 2.0 ** -24).all()
