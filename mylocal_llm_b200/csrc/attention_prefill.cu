@@ -22,6 +22,7 @@ namespace b200q {
 
 constexpr int PA_KEYS = 256;         // key positions per tile of the score product
 constexpr int PA_VALUES = 64;        // positions per tile of the value product
+constexpr int PA_SMEM_LIMIT = 232448;     // of every launch: one thread's prompt must not lower another's limit
 
 __device__ __forceinline__ uint64_t pa_pack2(float lo, float hi) {
     uint64_t r;
@@ -382,7 +383,7 @@ int b200q_prefill_attention(const float *q, const float *k, const float *v, int6
     const size_t smem = prefill_smem(t);
     auto kernel = rows == 64 ? prefill_attention_kernel<64> : prefill_attention_kernel<32>;
     if (cudaFuncSetAttribute(reinterpret_cast<const void *>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess) {
+                             PA_SMEM_LIMIT) != cudaSuccess) {
         cudaGetLastError();
         return fail(B200Q_ECUDA, "prefill_attention: shared memory opt-in failed");
     }

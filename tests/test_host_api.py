@@ -112,3 +112,19 @@ def test_quantisers_emit_valid_blocks_close_to_the_source(fmt):
     assert np.abs(dense - w).max() <= bound * np.abs(w).max()
     zeros = quantize(np.zeros((1, 256), np.float32), fmt)
     np.testing.assert_array_equal(po.dequantize(zeros.data, zeros.shape, fmt), np.zeros((1, 256), np.float32))
+
+
+def test_launchers_raise_the_shared_memory_limit_to_a_constant():
+    """The limit belongs to the kernel, not to the launch: a size that depends on the call lets one thread lower it between
+    another thread's setting and its launch. (The persistent step raises its own under a lock and never lowers it.)"""
+    import re
+    from pathlib import Path
+    import mylocal_llm_b200
+    calls = []
+    for path in sorted((Path(mylocal_llm_b200.__file__).parent / "csrc").glob("*.cu")):
+        if path.stem == "moe_decode_stack":
+            continue
+        calls += re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*?)\)\s*(?:!=|;)", path.read_text())
+    assert len(calls) >= 10
+    for value in calls:
+        assert re.fullmatch(r"[A-Z0-9_ *]+|static_cast<int>\([A-Z0-9_ *]+\)", value.strip()), value
