@@ -127,4 +127,4 @@ def test_launchers_raise_the_shared_memory_limit_to_a_constant():
         calls += re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*?)\)\s*(?:!=|;)", path.read_text())
     assert len(calls) >= 10
     for value in calls:
-        assert re.fullmatch(r"[A-Z0-9_ *]+|static_cast<int>\([A-Z0-9_ *]+\)", value.strip()), value
+        assert re.fullmatch(r"[A-Z0-9_ *-]+|static_cast<int>\([A-Z0-9_ *-]+\)", value.strip()), value
