@@ -8,26 +8,6 @@
 
 namespace b200q {
 
-// Sums the K parts of a team's row group in ascending order: every warp but the first stores its eight sums, the team
-// meets, the first warp adds. Two buffers in turn: a warp stores into a buffer again only after the team's next meeting,
-// which the first warp reaches with its reads of that buffer done. Returns true in the warp that holds the total.
-template <int COUNT>
-__device__ __forceinline__ bool add_parts(float (&v)[COUNT], float *partial, int &pbuf, int kp, int team, int kpi, int warp, int lane) {
-    if (kp == 1) return true;
-    float *buf = partial + pbuf * (GS_WARPS * 32 * 8);
-    pbuf ^= 1;
-    if (kpi) {
-#pragma unroll
-        for (int i = 0; i < COUNT; ++i) buf[(warp * 8 + i) * 32 + lane] = v[i];
-    }
-    named_barrier_sync(1 + team, kp * 32);
-    if (kpi) return false;
-    for (int q = 1; q < kp; ++q)
-#pragma unroll
-        for (int i = 0; i < COUNT; ++i) v[i] += buf[((warp + q) * 8 + i) * 32 + lane];
-    return true;
-}
-
 // Gate/up + SwiGLU over Q4_K / Q5_K tiles: hbuf[sorted assignment, row].
 template <bool Q5, int NTERMS>
 __global__ void __launch_bounds__(GS_THREADS, 1) grouped_gate_up_kernel(const GroupedArgs a) {
@@ -47,14 +27,15 @@ __global__ void __launch_bounds__(GS_THREADS, 1) grouped_gate_up_kernel(const Gr
         float tg[1][4] = {{0.f, 0.f, 0.f, 0.f}}, tu[1][4] = {{0.f, 0.f, 0.f, 0.f}};
         auto frag = [&](int, int fi, int p) { return *reinterpret_cast<const uint2 *>(fp + fi * 32 + p * plane); };
         auto sums = [&](int, int term) { return *reinterpret_cast<const uint32_t *>(xp + term * 16); };
+        bool ok = true;
         for (int sb = kpi; sb < a.nsb; sb += a.kp) {
             SuperBlockRegs<Q5> ra, rb;
             const uint8_t *tile;
-            if (!stream.next(tile)) return false;
+            if (!(ok = stream.next(tile))) break;
             read_superblock_tile<Q5>(ra, rb, tile, lane);
             stream.refill(lane);
             superblock_mma<Q5, NTERMS, 1>(ra, rb, frag, sums, tig, tg);
-            if (!stream.next(tile)) return false;
+            if (!(ok = stream.next(tile))) break;
             read_superblock_tile<Q5>(ra, rb, tile, lane);
             stream.refill(lane);
             superblock_mma<Q5, NTERMS, 1>(ra, rb, frag, sums, tig, tu);
@@ -62,7 +43,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) grouped_gate_up_kernel(const Gr
             xp += a.kp * 32;
         }
         float v[8] = {tg[0][0], tg[0][1], tg[0][2], tg[0][3], tu[0][0], tu[0][1], tu[0][2], tu[0][3]};
-        if (!add_parts(v, partial, pbuf, a.kp, team, kpi, warp, lane)) return true;
+        if (!add_parts(v, partial, pbuf, a.kp, team, kpi, warp, lane) || !ok) return ok;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int t = 2 * tig + e;
@@ -106,16 +87,17 @@ __global__ void __launch_bounds__(GS_THREADS, 1) grouped_down_kernel(const Group
         const uint8_t *fp = buf + g * a.smem_stride + tig * 16 + kpi * 512;
         float tot[1][4] = {{0.f, 0.f, 0.f, 0.f}};
         auto frag = [&](int, int pair, int p) { return fp + pair * 64 + p * plane; };
+        bool ok = true;
         for (int sb = kpi; sb < a.nsb; sb += a.kp) {
             typename T::Regs r;
             const uint8_t *tile;
-            if (!stream.next(tile)) return false;
+            if (!(ok = stream.next(tile))) break;
             T::read(r, tile, lane);
             stream.refill(lane);
             T::template mma<2, 1, 8>(r, frag, tot);
             fp += a.kp * 512;
         }
-        if (!add_parts(tot[0], partial, pbuf, a.kp, team, kpi, warp, lane)) return true;
+        if (!add_parts(tot[0], partial, pbuf, a.kp, team, kpi, warp, lane) || !ok) return ok;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int t = 2 * tig + e;

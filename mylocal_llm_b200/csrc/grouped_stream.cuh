@@ -174,9 +174,31 @@ struct TileStream {
     }
 };
 
+// Sums the K parts of a team's row group in ascending order: every warp but the first stores its eight sums, the team
+// meets, the first warp adds. Two buffers in turn: a warp stores into a buffer again only after the team's next meeting,
+// which the first warp reaches with its reads of that buffer done. Returns true in the warp that holds the total. A warp whose
+// wait gave up comes here too: the meeting has no limit of its own.
+template <int COUNT>
+__device__ __forceinline__ bool add_parts(float (&v)[COUNT], float *partial, int &pbuf, int kp, int team, int kpi, int warp, int lane) {
+    if (kp == 1) return true;
+    float *buf = partial + pbuf * (GS_WARPS * 32 * 8);
+    pbuf ^= 1;
+    if (kpi) {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) buf[(warp * 8 + i) * 32 + lane] = v[i];
+    }
+    named_barrier_sync(1 + team, kp * 32);
+    if (kpi) return false;
+    for (int q = 1; q < kp; ++q)
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) v[i] += buf[((warp + q) * 8 + i) * 32 + lane];
+    return true;
+}
+
 // Warp-level walk over the CTA's work. SORTED: image rows are sorted assignments. The functor
 // `work(seg, group, images, stream)` computes one row group from the images of its segment and the stream's next tiles;
-// it returns false when a wait gave up.
+// it returns false when a wait gave up, after it has met its team. A warp that gave up meets its team once for each of its
+// remaining groups as well, so that the others get past it to their own limits.
 template <bool SORTED, int TILE, bool DUAL, typename WorkFn>
 __device__ __forceinline__ void grouped_walk(const GroupedArgs &a, uint8_t *smem, const WorkFn work) {
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + 4;
@@ -248,6 +270,8 @@ __device__ __forceinline__ void grouped_walk(const GroupedArgs &a, uint8_t *smem
         // after its first group of a segment the producer asks for the one whose buffer the others have left by now
         if (warp == 0 && ok && ring.issued <= min(seg + ahead, ring.last)) ok = request_segment<SORTED>(a, ring, ring.issued++, bufs, lane);
     }
+    if (!ok && a.kp > 1)
+        for (; at.item < end; at.step(teams, groups_per_seg)) named_barrier_sync(1 + team, a.kp * 32);
     advance(ring.last + 1);
     if (!ok) {
         // gave up: copies may still be on their way into this CTA's shared memory - let each of them land (bounded)
