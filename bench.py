@@ -522,8 +522,8 @@ def exit_watchdog(seconds=90):
 MOE_SHAPE = dict(d_model=2048, d_ff=512, n_experts=512, top_k=10, shared_d_ff=512)
 EXPERT_BYTES = 2 * packed_bytes("Q4_K", 512, 2048) + packed_bytes("Q6_K", 2048, 512)
 # DRAM traffic of the grouped gate/up kernel over its algorithmic bytes in one ncu capture of the 64-token
-# single-GPU layer (448.3 MB moved for 430.2 MB); other token counts and rank counts were not captured.
-GATE_UP_TRAFFIC_RATIO = 1.04
+# single-GPU layer (434.7 MB moved for 428.7 MB); other token counts and rank counts were not captured.
+GATE_UP_TRAFFIC_RATIO = 1.01
 
 
 def split_rows(tokens, world, rank):
@@ -760,6 +760,42 @@ def ep_breakdown(torch, stream, step_fn, layers):
     return {k: round(v / (2 * layers), 2) for k, v in totals.items()}
 
 
+def gate_up_records(torch, stream, stack, step_fn):
+    """``(start event, end event, tokens per expert)`` of every grouped gate/up launch of one eager step. The native host
+    path launches without passing through ``moe_ops``, so the step runs on the Python layers; a one-token step runs as one
+    persistent kernel otherwise, whose gate/up stage is the same device function as the separate launch timed here."""
+    from mylocal_llm_b200 import moe_ops
+    records = []
+    real_gate_up = moe_ops.moe_gate_up
+
+    def timed_gate_up(x2d, plan, *a, **kw):
+        a0, a1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a0.record(stream)
+        res = real_gate_up(x2d, plan, *a, **kw)
+        a1.record(stream)
+        records.append((a0, a1, plan.counts))
+        return res
+
+    persistent, host = getattr(stack, "persistent_step", False), os.environ.get("B200Q_HOST")
+    moe_ops.moe_gate_up, os.environ["B200Q_HOST"] = timed_gate_up, "0"
+    if persistent:
+        stack.persistent_step = False
+    try:
+        for _ in range(2):
+            records.clear()
+            step_fn()
+            stream.synchronize()
+    finally:
+        moe_ops.moe_gate_up = real_gate_up
+        if host is None:
+            del os.environ["B200Q_HOST"]
+        else:
+            os.environ["B200Q_HOST"] = host
+        if persistent:
+            stack.persistent_step = True
+    return records
+
+
 def run_moe_gpu_arm(args, name):
     import torch
     import torch.distributed as dist
@@ -860,30 +896,7 @@ def run_moe_gpu_arm(args, name):
         clocks = sampler.stop() if rank == 0 else None
 
         # dominant kernel (grouped gate/up): its own duration and bytes, eager launches with events
-        records = []
-        real_gate_up = moe_ops.moe_gate_up
-
-        def timed_gate_up(x2d, plan, *a, **kw):
-            a0, a1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a0.record(stream)
-            res = real_gate_up(x2d, plan, *a, **kw)
-            a1.record(stream)
-            records.append((a0, a1, plan.counts))
-            return res
-
-        moe_ops.moe_gate_up = timed_gate_up
-        # (a one-token step runs as one persistent kernel; its gate/up stage is the same device function as the
-        # separate launch timed here)
-        persistent = getattr(stack, "persistent_step", False)
-        if persistent:
-            stack.persistent_step = False
-        for _ in range(2):
-            records.clear()
-            step_fn()
-            stream.synchronize()
-        moe_ops.moe_gate_up = real_gate_up
-        if persistent:
-            stack.persistent_step = True
+        records = gate_up_records(torch, stream, stack, step_fn)
         gate_up_ms = [a0.elapsed_time(a1) for a0, a1, _ in records]
         # expert-parallel plans end with one entry counting the assignments other ranks execute
         executed = [c[:-1] if world > 1 else c for _, _, c in records]
@@ -914,6 +927,9 @@ def run_moe_gpu_arm(args, name):
         layer_bytes = statistics.mean(distinct) * EXPERT_BYTES + (EXPERT_BYTES if world > 1 else 0) \
             + 4 * 2048 * 512 + 2 * tokens * d * 2
         single = world == 1 and tokens == 64
+        streams = _lib.load().b200q_moe_gate_up_streams(
+            _lib.FORMAT_ID["Q4_K_TILED"], MOE_SHAPE["d_ff"], d, _lib.DTYPE_ID["bfloat16"],
+            moe_ops.max_segments_for(tokens, MOE_SHAPE["top_k"] + 1, MOE_SHAPE["n_experts"] + 1))
         line = {
             "metric": "MoE decode tokens/s", "value": round(value, 2), "unit": "tokens/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(dev_ms / args.steps, 5),
@@ -930,10 +946,11 @@ def run_moe_gpu_arm(args, name):
                          "frac": round(achieved / peak, 4), "peak_source": f"of {peak_kind}",
                          "frac_of_nominal_8TBs": round(achieved / 8000.0, 4),
                          "traffic": int(gu_bytes * GATE_UP_TRAFFIC_RATIO) if single else None,
-                         "traffic_source": ("dram bytes read+write / algorithmic bytes = 1.04 in an ncu capture of this "
-                                            "kernel on the 64-token single-GPU layer, scaled to this launch") if single
+                         "traffic_source": ("dram bytes read+write / algorithmic bytes = %.2f in an ncu capture of this "
+                                            "kernel on the 64-token single-GPU layer, scaled to this launch"
+                                            % GATE_UP_TRAFFIC_RATIO) if single
                          else "not captured for this token / rank count",
-                         "kernel": "grouped gate/up + SwiGLU (mma_direct_kernel, mode 2)",
+                         "kernel": "grouped gate/up + SwiGLU (" + ("grouped_gate_up_kernel)" if streams else "mma_direct_kernel, mode 2)"),
                          "us_per_launch": round(gu_us, 3), "algorithmic_bytes_per_launch": int(gu_bytes)},
             "e2e": {"value": round(e2e_value, 2), "unit": "tokens/s",
                     "h2d_bytes_per_step": int(host_x.numel() * 4), "d2h_bytes_per_step": int(host_y.numel() * 4)},
