@@ -73,6 +73,9 @@ int b200q_dequantize(const void *w, int fmt, int64_t n, int k, float *out, void 
  * as one launch (the token embedding of a packed model). An id outside [0, n) gives zeros and stores 302 in the device
  * status word. */
 int b200q_embed_rows(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, void *stream);
+/* The same for the first step of a model: the row of an id outside the vocabulary is NaN, so that it shows in everything
+ * computed from it (the logits of its sequence), without a wait for the status word. */
+int b200q_embed_tokens(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, void *stream);
 
 /* y[m,n] = x[m,k] @ W[n,k]^T, FP32 accumulation; W is read once for up to 8 tokens.
  * Replaces quantized_linear's device branch and its Triton kernel

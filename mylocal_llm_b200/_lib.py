@@ -80,6 +80,7 @@ SIGNATURES = {
     "b200q_rope_attention": [_ptr, _ptr, _ptr, _c_i64, _c_i64, _c_i64, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int,
                              _c_int, _c_int, _ptr, _ptr, _c_int, _c_f32, _ptr, _c_int, _ptr],
     "b200q_embed_rows": [_ptr, _c_int, _c_i64, _c_int, _ptr, _c_int, _ptr, _ptr],
+    "b200q_embed_tokens": [_ptr, _c_int, _c_i64, _c_int, _ptr, _c_int, _ptr, _ptr],
     "b200q_prefill_attention_supported": [_c_int] * 7,
     "b200q_prefill_attention": [_ptr, _ptr, _ptr, _c_i64, _c_i64, _c_i64, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
                                 _c_int, _c_int, _ptr, _ptr, _c_int, _c_f32, _ptr, _c_int, _ptr],

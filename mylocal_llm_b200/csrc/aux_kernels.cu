@@ -70,10 +70,11 @@ __global__ void dequantize_kernel(const uint8_t *w, int fmt, long long total, fl
     }
 }
 
-// Selected rows (token embedding): grid.y = output row, a thread per weight of the row.
+// Selected rows (token embedding): grid.y = output row, a thread per weight of the row. `absent` fills the rows of indices
+// outside the matrix.
 constexpr int STATUS_ROW_RANGE = 302;      // a row index lay outside the matrix
 __global__ void __launch_bounds__(256) embed_rows_kernel(const uint8_t *w, int fmt, long long n, int k, const long long *ids,
-                                                         int count, float *out, int *status) {
+                                                         int count, float *out, int *status, float absent) {
     chain_trigger();
     chain_wait();         // the ids come from the preceding kernel
     const int qk = fmt_elems(fmt), qb = fmt_bytes(fmt);
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const uint8_t *w, int f
         const bool ok = row >= 0 && row < n;
         if (!ok && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(status, STATUS_ROW_RANGE);
         for (int e = blockIdx.x * 256 + threadIdx.x; e < k; e += gridDim.x * 256)
-            out[static_cast<size_t>(i) * k + e] = ok ? decode_one(w + row * row_bytes + static_cast<long long>(e / qk) * qb, fmt, e % qk) : 0.f;
+            out[static_cast<size_t>(i) * k + e] = ok ? decode_one(w + row * row_bytes + static_cast<long long>(e / qk) * qb, fmt, e % qk) : absent;
     }
 }
 
@@ -521,7 +522,7 @@ int b200q_dequantize(const void *w, int fmt, int64_t n, int k, float *out, void 
     return check_launch("dequantize");
 }
 
-int b200q_embed_rows(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, void *stream) {
+static int embed(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, float absent, void *stream) {
     if (!w || !ids || !out) return fail(B200Q_EINVAL, "embed_rows: NULL pointer");
     if (!fmt_valid(fmt)) return fail(B200Q_EINVAL, "embed_rows: unknown format %d", fmt);
     if (n <= 0 || k <= 0 || k % fmt_elems(fmt) || count <= 0) return fail(B200Q_EINVAL, "embed_rows: bad shape");
@@ -529,8 +530,16 @@ int b200q_embed_rows(const void *w, int fmt, int64_t n, int k, const int64_t *id
     if (!status) return fail(B200Q_ECUDA, "embed_rows: no CUDA device");
     launch_chained(embed_rows_kernel, dim3((k + 255) / 256, std::min(count, 65535)), dim3(256), 0,
                    static_cast<cudaStream_t>(stream), static_cast<const uint8_t *>(w), fmt, static_cast<long long>(n), k,
-                   reinterpret_cast<const long long *>(ids), count, out, status);
+                   reinterpret_cast<const long long *>(ids), count, out, status, absent);
     return check_launch("embed_rows");
+}
+
+int b200q_embed_rows(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, void *stream) {
+    return embed(w, fmt, n, k, ids, count, out, 0.f, stream);
+}
+
+int b200q_embed_tokens(const void *w, int fmt, int64_t n, int k, const int64_t *ids, int count, float *out, void *stream) {
+    return embed(w, fmt, n, k, ids, count, out, __builtin_nanf(""), stream);
 }
 
 int b200q_rmsnorm(const void *x, int x_dtype, const void *gamma, int gamma_dtype, int rows, int d, float eps,

@@ -6,7 +6,8 @@
 // (torch's caching allocator, so streams and CUDA-graph pools behave as before) and C ABI calls in C++. It contains no
 // computation and no kernels of its own: every launch goes through the entry points of libb200q.so, whose addresses
 // Python hands over once (bind). A call outside what it covers returns None and the Python layer, which raises the
-// documented exceptions, takes over; the results are the same bits either way.
+// documented exceptions, takes over; the results are the same bits either way. (Token ids outside the vocabulary: NaN for
+// their sequence here, a device-side assertion of the gather there.)
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -33,7 +34,7 @@ struct Api {
     FN(residual_rmsnorm); FN(gemv_norm); FN(gemv_norm_supported); FN(router_logits_t); FN(router_topk_ex);
     FN(router_topk_plan_row); FN(shared_gate); FN(moe_plan_ex); FN(moe_token_image_bytes); FN(moe_token_images);
     FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_gate_up_streams); FN(moe_down_streams); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
-    FN(prefill_attention); FN(embed_rows);
+    FN(prefill_attention); FN(embed_tokens);
 #undef FN
 } api;
 PyObject *b200q_error = nullptr;        // the package's exception for CUDA errors
@@ -44,7 +45,7 @@ void bind(const py::dict &addresses, py::object error_type) {
     FN(residual_rmsnorm); FN(gemv_norm); FN(gemv_norm_supported); FN(router_logits_t); FN(router_topk_ex);
     FN(router_topk_plan_row); FN(shared_gate); FN(moe_plan_ex); FN(moe_token_image_bytes); FN(moe_token_images);
     FN(moe_gate_up); FN(moe_gate_up_images); FN(moe_down); FN(moe_hidden_image_bytes); FN(moe_gate_up_streams); FN(moe_down_streams); FN(moe_hidden_images); FN(moe_down_images); FN(moe_combine); FN(silu_mul); FN(rope_attention);
-    FN(prefill_attention); FN(embed_rows);
+    FN(prefill_attention); FN(embed_tokens);
 #undef FN
     b200q_error = error_type.release().ptr();
 }
@@ -275,7 +276,7 @@ struct Llama {
     }
     at::Tensor embed_tokens(const at::Tensor &ids) const {
         at::Tensor r = empty({ids.numel(), d}, at::kFloat, ids.device());
-        CALL(embed_rows, embed.data_ptr(), embed_fmt, vocab, d, ids.data_ptr<int64_t>(), static_cast<int>(ids.numel()),
+        CALL(embed_tokens, embed.data_ptr(), embed_fmt, vocab, d, ids.data_ptr<int64_t>(), static_cast<int>(ids.numel()),
              r.data_ptr<float>(), stream());
         return r;
     }

@@ -477,7 +477,8 @@ class ExternalLlamaModel:
 
     def prefill(self, token_ids, state):
         """token_ids [B, T] int64 CUDA tensor; fills the cache from position 0; returns the logits of
-        the last position, FP32 [B, vocab]."""
+        the last position, FP32 [B, vocab]. An id outside the vocabulary makes the logits of its sequence NaN and
+        sets device status 302 (without the native host path: a device-side assertion)."""
         self._require_weights()
         torch = _torch()
         b, t = token_ids.shape
@@ -501,7 +502,8 @@ class ExternalLlamaModel:
         return quantized_linear(hidden[:, -1].contiguous(), self.lm_head, out_dtype=torch.float32)
 
     def decode_one(self, token_ids, state):
-        """token_ids [B] int64 CUDA tensor: appends one position; returns FP32 logits [B, vocab].
+        """token_ids [B] int64 CUDA tensor: appends one position; returns FP32 logits [B, vocab] (NaN for an id outside
+        the vocabulary, as in ``prefill``).
         All shapes are static and the position lives on the device (CUDA-graph capturable; the host
         counter ``state.length`` is advisory and is not advanced inside a captured graph)."""
         self._require_weights()

@@ -114,6 +114,24 @@ def test_caches_of_another_model_are_refused(cuda, monkeypatch, host):
     assert torch.equal(strided.v[0], plain.v[0]) and torch.equal(strided.k[0], plain.k[0])
 
 
+@pytest.mark.parametrize("bad", [512, -1, 2 ** 40])
+def test_a_token_outside_the_vocabulary_shows_in_its_sequence(cuda, bad):
+    """(By the kernel's own bounds check; the native path only.)"""
+    torch = cuda
+    model, ids = small_llama(), torch.randint(0, 512, (3, 6), device="cuda")
+    assert model._native(ids, model.create_generation_state(3, 32)) is not None
+    good, state = model.create_generation_state(3, 32), model.create_generation_state(3, 32)
+    want = model.prefill(ids, good)
+    ids[1, 2] = bad
+    logits = model.prefill(ids, state)
+    assert torch.isnan(logits[1]).all() and torch.equal(logits[0], want[0]) and torch.equal(logits[2], want[2])
+    step = torch.tensor([5, 6, bad], device="cuda")
+    logits = model.decode_one(step, good)
+    assert torch.isnan(logits[2]).all() and torch.isfinite(logits[:2]).all()
+    assert _lib.device_status() == 302
+    _lib.clear_device_status()
+
+
 @pytest.mark.parametrize("fmt", ["Q8_0", "Q4_K", "Q6_K"])
 def test_embed_rows_is_the_gather_of_dequantised_rows(cuda, fmt):
     torch = cuda
