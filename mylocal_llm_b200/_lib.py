@@ -155,15 +155,16 @@ def call(name, *args):
 
 
 _CALL = call
-_HOST = None
+_HOST = None            # the module once loaded; False: not available
 
 
 def host():
-    """The native host path (``_b200q_host.so``: launch sequences of the operators in C++), or ``None`` while every
-    entry point has to pass through ``call`` - somebody has replaced it to see the calls - or with ``B200Q_HOST=0``."""
+    """The native host path (an extension module: launch sequences of the operators in C++), or ``None`` while every
+    entry point has to pass through ``call`` - somebody has replaced it to see the calls -, with ``B200Q_HOST=0``, or where
+    the module can be neither loaded nor built for the installed torch: the Python layers make the same calls."""
     if call is not _CALL or os.environ.get("B200Q_HOST", "1") == "0":
         return None
-    return _HOST or _load_host()
+    return (_HOST if _HOST is not None else _load_host()) or None
 
 
 def _load_host():
@@ -173,16 +174,21 @@ def _load_host():
     with _LOCK:
         if _HOST is None:
             from . import build as _build
-            path = _build.HOST_LIB
-            if not path.exists():
-                _build.build_host()
-            import torch  # noqa: F401  (the extension links against its libraries)
-            spec = importlib.util.spec_from_file_location("_b200q_host", path)
-            module = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(module)
-            address = lambda fn: ctypes.cast(fn, _ptr).value
-            module.bind({name: address(getattr(lib, name)) for name in [*SIGNATURES, "b200q_last_error"]}, B200QError)
-            _HOST = module
+            try:
+                path = _build.HOST_LIB
+                if not path.exists():
+                    _build.build_host()
+                import torch  # noqa: F401  (the extension links against its libraries)
+                spec = importlib.util.spec_from_file_location("_b200q_host", path)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                address = lambda fn: ctypes.cast(fn, _ptr).value
+                module.bind({name: address(getattr(lib, name)) for name in [*SIGNATURES, "b200q_last_error"]}, B200QError)
+                _HOST = module
+            except Exception as error:
+                import warnings
+                warnings.warn(f"native host path not available, the Python layers run instead: {error}", RuntimeWarning)
+                _HOST = False
     return _HOST
 
 

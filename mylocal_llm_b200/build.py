@@ -7,6 +7,7 @@ it is rebuilt only when a source or header is newer.
 """
 
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -19,7 +20,20 @@ INCLUDE = PKG.parent / "include"
 LIB = PKG / "libb200q.so"
 OBJ_DIR = CSRC / "build"
 HOST_SRC = CSRC / "host" / "host_ops.cpp"
-HOST_LIB = PKG / "_b200q_host.so"
+
+
+def _host_lib():
+    """The host extension is compiled against one torch: its version is part of the name, so that another torch finds none
+    and does not load what it cannot bind."""
+    from importlib import metadata
+    try:
+        tag = re.sub(r"[^0-9A-Za-z.]", "_", metadata.version("torch"))
+    except metadata.PackageNotFoundError:
+        tag = "none"
+    return PKG / f"_b200q_host.{tag}.so"
+
+
+HOST_LIB = _host_lib()
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -58,7 +72,7 @@ def needs_host_build():
 
 
 def build_host(force=False):
-    """Compile ``_b200q_host.so`` (C++ only, against the installed torch); returns its path."""
+    """Compile the host extension (C++ only, against the installed torch); returns its path."""
     if not force and not needs_host_build():
         return HOST_LIB
     import sysconfig

@@ -1,4 +1,4 @@
-"""The native host path (``_b200q_host.so``) against the Python layers (``B200Q_HOST=0``): the same entry points in the
+"""The native host path (the host extension) against the Python layers (``B200Q_HOST=0``): the same entry points in the
 same order, so every result has to be the same bits - linears on both sides of the GEMM rule, MoE layers with and
 without pointer tables and token images, a stack, a Llama prompt and its decode steps."""
 

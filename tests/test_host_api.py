@@ -128,3 +128,23 @@ def test_launchers_raise_the_shared_memory_limit_to_a_constant():
     assert len(calls) >= 10
     for value in calls:
         assert re.fullmatch(r"[A-Z0-9_ *-]+|static_cast<int>\([A-Z0-9_ *-]+\)", value.strip()), value
+
+
+@pytest.mark.parametrize("content", [None, b"not an object file"])
+def test_without_the_host_extension_the_python_layers_run(monkeypatch, tmp_path, content):
+    from mylocal_llm_b200 import _lib, build
+    path = tmp_path / "host.so"
+    if content is not None:
+        path.write_bytes(content)
+    monkeypatch.setattr(build, "HOST_LIB", path)
+    monkeypatch.setenv("CXX", str(tmp_path / "no-compiler"))
+    monkeypatch.setattr(_lib, "_HOST", None)
+    with pytest.warns(RuntimeWarning, match="Python layers"):
+        assert _lib.host() is None
+    assert _lib.host() is None          # (and says so once)
+
+
+def test_the_host_extension_belongs_to_the_installed_torch():
+    import torch
+    from mylocal_llm_b200 import build
+    assert torch.__version__.split("+")[0] in build.HOST_LIB.name
