@@ -192,6 +192,12 @@ def _load_host():
     return _HOST
 
 
+def as_defined(obj, cls):
+    """Whether ``obj`` is a plain ``cls``: no subclass, no method replaced on the instance (a wrapped ``forward``, a hook).
+    The native host path makes the calls that the class's own methods would make."""
+    return type(obj) is cls and not any(callable(getattr(cls, name, None)) for name in vars(obj))
+
+
 def current_stream():
     """Raw handle of the framework's current CUDA stream (the launch stream of every call)."""
     import torch

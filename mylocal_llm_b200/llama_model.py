@@ -19,6 +19,7 @@ adapter; here they stay packed and resident in HBM, which is the point of the ex
 """
 
 import ctypes
+import operator
 import os
 from dataclasses import dataclass
 
@@ -87,7 +88,7 @@ class ExternalLlamaModel:
         # launch of its own; the results are the same bits)
         self.fused_norm_linear = os.environ.get("B200Q_NORM_GEMV", "1") != "0"
         self._loaded = False
-        self._host = None              # native host path of the loaded weights (False: they need the Python layers)
+        self._host = (None, None)      # (what it was built from, native plan or None) - see _native()
 
     def expected_shapes(self):
         cfg = self.config
@@ -198,7 +199,7 @@ class ExternalLlamaModel:
         ang = np.arange(cfg.max_position_embeddings)[:, None] * inv[None, :]
         self._cos = torch.as_tensor(np.cos(ang), dtype=torch.float32).to(self.device)
         self._sin = torch.as_tensor(np.sin(ang), dtype=torch.float32).to(self.device)
-        self._host = None
+        self._host = (None, None)
         self._loaded = True
 
     @property
@@ -453,27 +454,51 @@ class ExternalLlamaModel:
         host = _lib.host()
         device = self.embed.data.device
         fits = lambda cache: self._stacked_cache_fits(cache, state.batch, state.horizon)
-        if (host is None or self._host is False or not self.fused_decode or token_ids.dtype != torch.int64
+        if (host is None or not self.fused_decode or token_ids.dtype != torch.int64
                 or token_ids.device != device or not token_ids.numel() or not fits(state.k) or not fits(state.v)
                 or state.position.dtype != torch.int64 or state.position.device != device):
             return None
-        if self._host is None:
-            cfg = self.config
-            stacked = all(layer["qkv"] is not None and layer["gate_up"] is not None for layer in self.layers)
-            fits = stacked and cfg.head_dim in (64, 128) and self.embed.quant_type in _lib.FORMAT_ID
+        # what the plan holds, compared on every call: a norm weight, a matrix or a layer replaced since shows in it
+        cfg = self.config
+        key = [host, self.embed, self.lm_head, self.final_norm, self.final_norm.gamma, self.final_norm.eps, self._cos, self._sin,
+               self.dtype, cfg.hidden_size, cfg.intermediate_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
+               cfg.vocab_size, len(vars(self))]
+        native_of = self.native_of.get
+        for layer in self.layers:
+            norm1, norm2, matrices = layer["norm1"], layer["norm2"], [layer[n] for n in ("qkv", "o", "gate_up", "down")]
+            key += [norm1, norm1.gamma, norm1.eps, norm2, norm2.gamma, norm2.eps, *matrices, *[native_of(id(w)) for w in matrices]]
+        built, plan = self._host
+        if built is None or len(built) != len(key) or not all(map(operator.is_, built, key)):
+            plan = self._build_native(host)
+            self._host = (key, plan)
+        return plan
 
-            def matrix(w):
-                native = self.native_of.get(id(w))
-                return (w.data, w._format_id, w.shape[0], w.shape[1], None if native is None else native.data,
-                        -1 if native is None else native._format_id)
+    def _build_native(self, host):
+        """The plan of the native host path, or ``None``: a layer is not stacked, a method is replaced or overridden, norms
+        differ in what the path takes as one."""
+        torch = _torch()
+        cfg = self.config
+        norms = [layer[n] for layer in self.layers for n in ("norm1", "norm2")] + [self.final_norm]
+        gammas = [n.gamma for n in norms]
+        if (not _lib.as_defined(self, ExternalLlamaModel) or not all(_lib.as_defined(n, RMSNormInference) for n in norms)
+                or any(layer["qkv"] is None or layer["gate_up"] is None for layer in self.layers)
+                or cfg.head_dim not in (64, 128) or self.embed.quant_type not in _lib.FORMAT_ID
+                or len({n.eps for n in norms}) != 1 or any(n.d_model != cfg.hidden_size for n in norms)
+                or any(not isinstance(g, torch.Tensor) or g.dtype != self.dtype or g.shape != (cfg.hidden_size,) or not g.is_contiguous()
+                       or g.device != self.embed.data.device for g in gammas)):
+            return None
 
-            self._host = False if not fits else host.Llama(dict(
-                embed=self.embed.data, embed_fmt=self.embed._format_id, final_norm=self.final_norm.gamma, lm_head=matrix(self.lm_head),
-                cos=self._cos, sin=self._sin, d=cfg.hidden_size, f=cfg.intermediate_size, heads=cfg.num_attention_heads,
-                kv_heads=cfg.num_key_value_heads, head_dim=cfg.head_dim, vocab=cfg.vocab_size, eps=cfg.rms_norm_eps,
-                layers=[(layer["norm1"].gamma, layer["norm2"].gamma, matrix(layer["qkv"]), matrix(layer["o"]),
-                         matrix(layer["gate_up"]), matrix(layer["down"])) for layer in self.layers]))
-        return self._host or None
+        def matrix(w):
+            native = self.native_of.get(id(w))
+            return (w.data, w._format_id, w.shape[0], w.shape[1], None if native is None else native.data,
+                    -1 if native is None else native._format_id)
+
+        return host.Llama(dict(
+            embed=self.embed.data, embed_fmt=self.embed._format_id, final_norm=self.final_norm.gamma, lm_head=matrix(self.lm_head),
+            cos=self._cos, sin=self._sin, d=cfg.hidden_size, f=cfg.intermediate_size, heads=cfg.num_attention_heads,
+            kv_heads=cfg.num_key_value_heads, head_dim=cfg.head_dim, vocab=cfg.vocab_size, eps=norms[0].eps,
+            layers=[(layer["norm1"].gamma, layer["norm2"].gamma, matrix(layer["qkv"]), matrix(layer["o"]),
+                     matrix(layer["gate_up"]), matrix(layer["down"])) for layer in self.layers]))
 
     def prefill(self, token_ids, state):
         """token_ids [B, T] int64 CUDA tensor; fills the cache from position 0; returns the logits of

@@ -114,6 +114,42 @@ def test_caches_of_another_model_are_refused(cuda, monkeypatch, host):
     assert torch.equal(strided.v[0], plain.v[0]) and torch.equal(strided.k[0], plain.k[0])
 
 
+def test_what_is_replaced_after_the_first_call_counts(cuda, monkeypatch):
+    """A norm weight, an epsilon, a matrix, a wrapped method: the native path gives what the Python layers give."""
+    torch = cuda
+    model, other, ids = small_llama(), small_llama(seed=2), torch.randint(0, 512, (2, 5), device="cuda")
+
+    def step():
+        state = model.create_generation_state(2, 32)
+        return torch.stack([model.prefill(ids, state), model.decode_one(ids[:, 0].contiguous(), state)])
+
+    def check(changed=True):
+        nonlocal before
+        native, python = both(monkeypatch, step)
+        assert torch.equal(native, python) and torch.equal(native, before) != changed
+        before = native
+
+    before = step()
+    check(changed=False)
+    gamma = torch.linspace(0.5, 1.5, 256, device="cuda").bfloat16()
+    model.layers[1]["norm2"].set_weights(gamma)
+    check()
+    model.final_norm.eps = 0.1
+    check()
+    model.layers[0]["down"] = other.layers[0]["down"]
+    check()
+    model.lm_head = other.lm_head
+    check()
+    model.layers[0]["norm1"].set_weights(gamma.float())          # another type: the Python layers take it
+    check()
+    model.layers[0]["norm1"].set_weights(gamma)
+    check()
+    linear, seen = model._linear, []
+    model._linear = lambda *a: (seen.append(1), linear(*a))[1]
+    check(changed=False)
+    assert seen
+
+
 @pytest.mark.parametrize("bad", [512, -1, 2 ** 40])
 def test_a_token_outside_the_vocabulary_shows_in_its_sequence(cuda, bad):
     """(By the kernel's own bounds check; the native path only.)"""
