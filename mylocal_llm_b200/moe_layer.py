@@ -16,6 +16,7 @@ layer also accepts BF16/FP16 (accumulation stays FP32, the output is rounded onc
 """
 
 import ctypes
+import operator
 import os
 
 from . import _lib, moe_ops
@@ -151,16 +152,29 @@ class PackedMoELayer:
     def native(self, host):
         """The layer for the native host path (``_b200q_host.MoeLayer``), or ``None`` when it needs the Python one: another
         executor, a shared expert that does not fit the grouped kernels, a router without an expert-major weight."""
-        router, bank = self.router, self.bank
-        key = (router._w_expert_major, router.b_router, self.shared_gate, self._tables, self.executor, bank, self.fuse_row_plan,
-               router.normalization_floor, router.k)
+        router, bank, executor = self.router, self.bank, self.executor
+        # what the plan holds, compared on every call
+        key = (host, router, router._w_expert_major, router.b_router, self.shared, self.shared_gate, self._tables, executor,
+               executor.banks.get(self.layer_id) if isinstance(executor, ResidentExpertExecutor) else None, bank, bank.gate, bank.up,
+               bank.down, bank.gate_type, bank.up_type, bank.down_type, bank.n_experts, bank.d_model, bank.d_ff, self.fuse_row_plan,
+               router.normalization_floor, router.k, len(vars(router)), len(vars(executor)))
         built, layer = self._host
-        if built is not None and all(a is b for a, b in zip(built, key)):
+        if built is not None and all(map(operator.is_, built, key)):
             return layer
+        torch = _torch()
+        device = bank.gate.device
+
+        def vector(v, n):
+            return v is None or (isinstance(v, torch.Tensor) and v.dtype == torch.float32 and v.is_contiguous() and v.numel() == n
+                                 and v.device == device)
+
         w = router._w_expert_major
         layer = None
-        if (type(self.executor) is ResidentExpertExecutor and self.executor.banks.get(self.layer_id) is bank and w is not None
-                and w.is_cuda and w.dtype == _torch().float32 and w.is_contiguous() and w.shape[1] % 4 == 0 and w.data_ptr() % 16 == 0
+        if (type(executor) is ResidentExpertExecutor and _lib.as_defined(executor, ResidentExpertExecutor)
+                and _lib.as_defined(router, RouterInference) and executor.banks.get(self.layer_id) is bank and w is not None
+                and w.device == device and w.is_cuda and w.dtype == torch.float32 and w.is_contiguous()
+                and tuple(w.shape) == (bank.n_experts, bank.d_model) and w.shape[1] % 4 == 0 and w.data_ptr() % 16 == 0
+                and vector(router.b_router, bank.n_experts) and vector(self.shared_gate, bank.d_model)
                 and (self._tables is not None or (self.shared is None and self.shared_gate is None))):
             tables, aligned = self._tables if self._tables is not None else (None, False)
             layer = host.MoeLayer(w, router.b_router, self.shared_gate, bank.gate, bank.up, bank.down,
@@ -179,7 +193,8 @@ class PackedMoELayer:
         torch = _torch()
         host = _lib.host() if residual_norm is None else None
         if (host is not None and type(hidden) is torch.Tensor and hidden.is_cuda and hidden.ndim == 3 and hidden.is_contiguous()
-                and hidden.numel() and hidden.shape[-1] == self.bank.d_model and str(hidden.dtype)[6:] in _lib.DTYPE_ID):
+                and hidden.numel() and hidden.shape[-1] == self.bank.d_model and str(hidden.dtype)[6:] in _lib.DTYPE_ID
+                and hidden.device == self.bank.gate.device):
             layer = self.native(host)
             if layer is not None:
                 return layer.forward(hidden)

@@ -53,6 +53,33 @@ def test_moe_layer(cuda, monkeypatch, t, shared, dtype):
     assert a.dtype == b.dtype and torch.equal(a, b)
 
 
+def test_a_layer_shows_what_is_replaced_after_its_first_call(cuda, monkeypatch):
+    torch = cuda
+    types, d, f, e = ("Q4_K", "Q4_K", "Q6_K"), 512, 256, 16
+    bank, other = synthetic_bank(e, d, f, types, seed=3), synthetic_bank(e, d, f, types, seed=4)
+    layer = PackedMoELayer(bank, 0.05 * torch.randn((d, e), device="cuda"), 4)
+    x = torch.randn((1, 5, d), device="cuda")
+    before = layer.forward(x)
+
+    def check():
+        nonlocal before
+        a, b = both(monkeypatch, lambda: layer.forward(x))
+        assert torch.equal(a, b) and not torch.equal(a, before)
+        before = a
+
+    layer.bank.down = PackedMoELayer(other, layer.router.W_router, 4).bank.down
+    check()
+    layer.router.b_router = torch.linspace(0, 3, e, device="cuda")
+    check()
+    layer.router.k = 2
+    check()
+    layer.executor.banks[0] = PackedMoELayer(other, layer.router.W_router, 4).bank
+    check()
+    routed, seen = layer.executor.forward_routed, []
+    layer.executor.forward_routed = lambda *a, **kw: (seen.append(1), routed(*a, **kw))[1]
+    assert torch.equal(layer.forward(x), before) and seen
+
+
 @pytest.mark.parametrize("t", [2, 33])
 def test_moe_stack(cuda, monkeypatch, t):
     torch = cuda
