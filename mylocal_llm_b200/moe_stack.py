@@ -111,16 +111,20 @@ class PackedMoEStack:
         torch = _torch()
         host = _lib.host()
         norms = [*self.norms, self.final_norm]
-        gammas = [n.gamma for n in norms]
-        if (host is None or residual.dtype != torch.float32 or not residual.is_cuda or not residual.is_contiguous()
-                or not residual.numel() or residual.shape[-1] != norms[0].d_model):
+        if (host is None or residual.ndim != 3 or residual.dtype != torch.float32 or not residual.is_cuda
+                or not residual.is_contiguous() or not residual.numel() or residual.shape[-1] != norms[0].d_model
+                or not all(_lib.as_defined(layer, PackedMoELayer) for layer in self.layers)
+                or not all(_lib.as_defined(n, RMSNormInference) for n in norms)):
             return None
         layers = [layer.native(host) for layer in self.layers]
+        gammas = [n.gamma for n in norms]
         if (any(layer is None for layer in layers) or len({n.eps for n in norms}) != 1
-                or any(g is None or g.dtype != gammas[0].dtype or g.shape != gammas[0].shape or not g.is_contiguous() for g in gammas)
-                or gammas[0].shape != (residual.shape[-1],)):
+                or any(layer.bank.d_model != residual.shape[-1] or layer.bank.gate.device != residual.device for layer in self.layers)
+                or any(not isinstance(g, torch.Tensor) or g.dtype != gammas[0].dtype or g.shape != (residual.shape[-1],)
+                       or not g.is_contiguous() or g.device != residual.device for g in gammas)
+                or str(gammas[0].dtype)[6:] not in _lib.DTYPE_ID):
             return None
-        key = (*layers, *gammas)
+        key = (*layers, *gammas, norms[0].eps)
         built, stack = self._host
         if built is None or len(built) != len(key) or any(a is not b for a, b in zip(built, key)):
             stack = host.MoeStack(layers, gammas, norms[0].eps)

@@ -90,6 +90,32 @@ def test_moe_stack(cuda, monkeypatch, t):
     assert torch.equal(x, kept) and torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
 
 
+def test_a_stack_runs_its_layers_as_they_are(cuda, monkeypatch):
+    """A subclass, a wrapped method, another epsilon, a residual of two dimensions: as on the Python layers."""
+    torch = cuda
+    stack = PackedMoEStack.synthetic(3, d_model=512, d_ff=256, n_experts=16, top_k=4, shared_d_ff=256, seed=5)
+    x = torch.randn((7, 1, 512), device="cuda")
+    with pytest.raises(ValueError, match="hidden must have shape"):
+        stack.forward(x[:, 0])
+    before = stack.forward(x)
+    for norm in [*stack.norms, stack.final_norm]:
+        norm.eps = 0.5
+    a, b = both(monkeypatch, lambda: stack.forward(x))
+    assert torch.equal(a[1], b[1]) and not torch.equal(a[1], before[1])
+    seen, forward = [], stack.layers[1].forward
+    stack.layers[1].forward = lambda *args: (seen.append("wrapped"), forward(*args))[1]
+    assert torch.equal(stack.forward(x)[1], a[1]) and seen == ["wrapped"]
+
+    class Doubled(PackedMoELayer):
+        def forward(self, hidden, residual_norm=None):
+            seen.append("subclass")
+            return 2 * super().forward(hidden)
+
+    del stack.layers[1].forward
+    stack.layers[1].__class__ = Doubled
+    assert not torch.equal(stack.forward(x)[1], a[1]) and seen[-1] == "subclass"
+
+
 @pytest.mark.parametrize("batch", [1, 3, 17])
 def test_llama_prompt_and_steps(cuda, monkeypatch, batch):
     torch = cuda
