@@ -79,12 +79,19 @@ at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t, const at::Device &devi
 }
 bool gguf_gemm_format(int fmt) { return fmt == B200Q_Q8_0 || fmt == B200Q_Q4_K || fmt == B200Q_Q5_K || fmt == B200Q_Q6_K; }
 
-int gemm_min_tokens = 9;                // tokens from which BF16 calls on GGUF-layout weights take the GEMM
+// Tokens from which BF16 calls on GGUF-layout weights take the GEMM, by format (0: never): quantized_linear.GEMM_MIN_TOKENS
+// as it stands at the call.
+struct GemmRule {
+    int q8_0 = 0, q4_k = 0, q5_k = 0, q6_k = 0;
+    int of(int fmt) const {
+        return fmt == B200Q_Q8_0 ? q8_0 : fmt == B200Q_Q4_K ? q4_k : fmt == B200Q_Q5_K ? q5_k : fmt == B200Q_Q6_K ? q6_k : 0;
+    }
+};
 
 // y[m, n] = x[m, k] W^T by the rule of quantized_linear (GEMM for many BF16 tokens on a GGUF layout, else GEMV).
 void linear_into(const void *x, int x_dtype, int m, const void *w, int fmt, int n, int k, void *y, int y_dtype,
-                 bool allow_gemm, const at::Device &device) {
-    if (allow_gemm && m >= gemm_min_tokens && gguf_gemm_format(fmt) && x_dtype == B200Q_BF16 &&
+                 int gemm_min_tokens, const at::Device &device) {
+    if (gemm_min_tokens > 0 && m >= gemm_min_tokens && gguf_gemm_format(fmt) && x_dtype == B200Q_BF16 &&
         (reinterpret_cast<uintptr_t>(x) & 15) == 0 && reinterpret_cast<uintptr_t>(w) % (fmt == B200Q_Q8_0 ? 4 : 2) == 0 &&
         !env_is("B200Q_GEMM", "0") && !env_set_other_than("B200Q_KERNEL", "auto") && api.gemm_supported(fmt, n, k, x_dtype, m)) {
         const long long bytes = api.gemm_workspace_bytes(fmt, n, k, x_dtype, m);
@@ -100,13 +107,13 @@ void linear_into(const void *x, int x_dtype, int m, const void *w, int fmt, int 
 }
 
 // ------------------------------------------------------------------------------------------------ linear
-// linear(x, data, fmt, n, k, out_dtype | None, allow_gemm): the tensor, or None when the call needs the Python layer.
+// linear(x, data, fmt, n, k, out_dtype | None, GEMM from this many tokens on or 0): the tensor, or None when the call needs the Python layer.
 PyObject *linear_fast(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (nargs != 7 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) Py_RETURN_NONE;
     HANDLE_TH_ERRORS
         const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]);
         const int fmt = static_cast<int>(PyLong_AsLong(args[2])), n = static_cast<int>(PyLong_AsLong(args[3])),
-                  k = static_cast<int>(PyLong_AsLong(args[4]));
+                  k = static_cast<int>(PyLong_AsLong(args[4])), gemm_min = static_cast<int>(PyLong_AsLong(args[6]));
         const int64_t nd = x.dim();
         const int dt = dtype_id(x.scalar_type());
         if (!x.is_cuda() || (nd != 2 && nd != 3) || x.size(nd - 1) != k || dt < 0 || !x.is_contiguous() || x.device() != w.device())
@@ -120,7 +127,7 @@ PyObject *linear_fast(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         const int64_t m = x.numel() / k;
         if (ydt < 0 || m == 0 || m > 0x7fffffff) Py_RETURN_NONE;
         at::Tensor y = nd == 2 ? empty({m, n}, out_type, x.device()) : empty({x.size(0), x.size(1), n}, out_type, x.device());
-        linear_into(x.data_ptr(), dt, static_cast<int>(m), w.data_ptr(), fmt, n, k, y.data_ptr(), ydt, args[6] == Py_True, x.device());
+        linear_into(x.data_ptr(), dt, static_cast<int>(m), w.data_ptr(), fmt, n, k, y.data_ptr(), ydt, gemm_min, x.device());
         return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -269,10 +276,12 @@ struct Llama {
 
     int dt() const { return dtype_id(type); }
     // ExternalLlamaModel._linear: many BF16 rows read the GGUF copy, everything else the decode layout
-    void linear(const at::Tensor &x, int64_t m, const Matrix &w, at::Tensor &y, bool choose = true) const {
-        const bool native = choose && w.native.defined() && type == at::kBFloat16 && m >= gemm_min_tokens;
+    void linear(const at::Tensor &x, int64_t m, const Matrix &w, at::Tensor &y, const GemmRule &rule, bool choose = true) const {
+        const int from = choose && w.native.defined() ? rule.of(w.native_fmt) : 0;
+        const bool native = from > 0 && type == at::kBFloat16 && m >= from;
         linear_into(x.data_ptr(), dtype_id(x.scalar_type()), static_cast<int>(m), native ? w.native.data_ptr() : w.data.data_ptr(),
-                    native ? w.native_fmt : w.fmt, w.n, w.k, y.data_ptr(), dtype_id(y.scalar_type()), true, x.device());
+                    native ? w.native_fmt : w.fmt, w.n, w.k, y.data_ptr(), dtype_id(y.scalar_type()),
+                    rule.of(native ? w.native_fmt : w.fmt), x.device());
     }
     at::Tensor embed_tokens(const at::Tensor &ids) const {
         at::Tensor r = empty({ids.numel(), d}, at::kFloat, ids.device());
@@ -292,7 +301,8 @@ struct Llama {
     }
 
     // One token per sequence: ids [B], caches [layers, B, kv_heads, horizon, head_dim], position [1] int64 (device).
-    at::Tensor decode(const at::Tensor &ids, const at::Tensor &kc, const at::Tensor &vc, const at::Tensor &position) const {
+    at::Tensor decode(const at::Tensor &ids, const at::Tensor &kc, const at::Tensor &vc, const at::Tensor &position,
+                      const GemmRule &rule) const {
         const int64_t b = ids.numel(), qd = static_cast<int64_t>(heads) * head_dim, kd = static_cast<int64_t>(kv_heads) * head_dim;
         const at::Device dev = ids.device();
         at::Tensor residual = embed_tokens(ids), hidden = empty({b, d}, type, dev), qkv = empty({b, qd + 2 * kd}, at::kFloat, dev),
@@ -310,13 +320,13 @@ struct Llama {
                 return;
             }
             add_norm(residual, branch, gamma, b, hidden);
-            linear(hidden, b, w, y);
+            linear(hidden, b, w, y, rule);
         };
         for (size_t i = 0; i < layers.size(); ++i) {
             const LlamaLayer &l = layers[i];
             if (i == 0) {
                 norm(residual, l.norm1, b, hidden);
-                linear(hidden, b, l.qkv, qkv);
+                linear(hidden, b, l.qkv, qkv, rule);
             } else {
                 norm_linear(l.norm1, l.qkv, qkv);
             }
@@ -326,17 +336,17 @@ struct Llama {
                  sin.data_ptr<float>(), static_cast<int>(cos.size(0)), static_cast<int>(b), heads, kv_heads, head_dim,
                  static_cast<int>(kc.size(3)), static_cast<uint8_t *>(kc.data_ptr()) + i * layer_bytes,
                  static_cast<uint8_t *>(vc.data_ptr()) + i * layer_bytes, dt(), scale, ctx.data_ptr(), dt(), stream());
-            linear(ctx, b, l.o, branch, false);
+            linear(ctx, b, l.o, branch, rule, false);
             norm_linear(l.norm2, l.gate_up, gu);
             silu(gu, b, act);
-            linear(act, b, l.down, branch);
+            linear(act, b, l.down, branch, rule);
         }
         norm_linear(final_norm, lm_head, logits);
         return logits;
     }
 
     // The whole prompt from position 0 on: ids [B, T]; logits of the last position.
-    at::Tensor prefill(const at::Tensor &ids, const at::Tensor &kc, const at::Tensor &vc) const {
+    at::Tensor prefill(const at::Tensor &ids, const at::Tensor &kc, const at::Tensor &vc, const GemmRule &rule) const {
         const int64_t b = ids.size(0), t = ids.size(1), rows = b * t, qd = static_cast<int64_t>(heads) * head_dim,
                       kd = static_cast<int64_t>(kv_heads) * head_dim;
         const at::Device dev = ids.device();
@@ -348,26 +358,27 @@ struct Llama {
         norm(residual, layers[0].norm1, rows, hidden);
         for (size_t i = 0; i < layers.size(); ++i) {
             const LlamaLayer &l = layers[i];
-            linear(hidden, rows, l.qkv, qkv);
+            linear(hidden, rows, l.qkv, qkv, rule);
             float *q = qkv.data_ptr<float>();
             CALL(prefill_attention, q, q + qd, q + qd + kd, row, row, row, cos.data_ptr<float>(), sin.data_ptr<float>(),
                  static_cast<int>(cos.size(0)), static_cast<int>(b), static_cast<int>(t), heads, kv_heads, head_dim,
                  static_cast<int>(kc.size(3)), static_cast<uint8_t *>(kc.data_ptr()) + i * layer_bytes,
                  static_cast<uint8_t *>(vc.data_ptr()) + i * layer_bytes, dt(), scale, ctx.data_ptr(), dt(), stream());
-            linear(ctx, rows, l.o, branch);
+            linear(ctx, rows, l.o, branch, rule);
             add_norm(residual, branch, l.norm2, rows, hidden);
-            linear(hidden, rows, l.gate_up, gu);
+            linear(hidden, rows, l.gate_up, gu, rule);
             silu(gu, rows, act);
-            linear(act, rows, l.down, branch);
+            linear(act, rows, l.down, branch, rule);
             add_norm(residual, branch, i + 1 < layers.size() ? layers[i + 1].norm1 : final_norm, rows, hidden);
         }
         const at::Tensor last = hidden.view({b, t, d}).select(1, t - 1).contiguous();
         at::Tensor logits = empty({b, vocab}, at::kFloat, dev);
-        linear(last, b, lm_head, logits, false);
+        linear(last, b, lm_head, logits, rule, false);
         return logits;
     }
 };
 
+GemmRule gemm_rule(const std::vector<int> &v) { return {v.at(0), v.at(1), v.at(2), v.at(3)}; }
 at::Tensor or_undefined(const py::object &o) { return o.is_none() ? at::Tensor() : o.cast<at::Tensor>(); }
 
 }  // namespace
@@ -430,6 +441,10 @@ PYBIND11_MODULE(_b200q_host, m) {
             }
             return l;
         }))
-        .def("decode", &Llama::decode)
-        .def("prefill", &Llama::prefill);
+        .def("decode", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, at::Tensor position, const std::vector<int> &rule) {
+            return m.decode(ids, k, v, position, gemm_rule(rule));
+        })
+        .def("prefill", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, const std::vector<int> &rule) {
+            return m.prefill(ids, k, v, gemm_rule(rule));
+        });
 }

@@ -27,7 +27,7 @@ import numpy as np
 
 from . import _lib
 from .moe_layer import RMSNormInference
-from .quantized_linear import (GEMM_MIN_TOKENS, DevicePackedGGUFWeight, dequantize_device, packed_to_device, quantized_linear,
+from .quantized_linear import (GEMM_MIN_TOKENS, DevicePackedGGUFWeight, dequantize_device, gemm_rule, packed_to_device, quantized_linear,
                                quantized_swiglu, retile_enabled, retile_gate_up, retile_weight)
 from .quantized_weight import PackedGGUFWeight, block_format
 
@@ -513,7 +513,7 @@ class ExternalLlamaModel:
         if self._prefill_kernel_fits(b, t, state):
             native = self._native(token_ids, state)
             if native is not None:
-                logits = native.prefill(token_ids.contiguous(), state.k, state.v)
+                logits = native.prefill(token_ids.contiguous(), state.k, state.v, gemm_rule())
                 state.position.fill_(t)
                 state.length = t
                 return logits
@@ -539,7 +539,7 @@ class ExternalLlamaModel:
                 and os.environ.get("B200Q_ROPE_ATTENTION", "1") != "0" and token_ids.numel() == state.batch):
             native = self._native(token_ids, state)
             if native is not None:
-                logits = native.decode(token_ids.contiguous(), state.k, state.v, state.position)
+                logits = native.decode(token_ids.contiguous(), state.k, state.v, state.position, gemm_rule())
                 state.position.add_(1)
                 state.length += 1
                 return logits

@@ -2,6 +2,8 @@
 same order, so every result has to be the same bits - linears on both sides of the GEMM rule, MoE layers with and
 without pointer tables and token images, a stack, a Llama prompt and its decode steps."""
 
+import sys
+
 import numpy as np
 import pytest
 
@@ -35,6 +37,26 @@ def test_linear(cuda, monkeypatch, fmt, dtype, tiled, m):
     for kwargs in ({}, {"out_dtype": torch.float32}, {"allow_gemm": False}):
         a, b = both(monkeypatch, lambda: quantized_linear(x, w, **kwargs))
         assert a.shape == b.shape == (1, m, 80) and a.dtype == b.dtype and torch.equal(a, b)
+
+
+def test_the_gemm_rule_is_the_one_of_the_python_layers(cuda, monkeypatch):
+    torch = cuda
+    w = packed_to_device(random_packed("Q8_0", (128, 512), seed=1, d=0.01))
+    x = torch.randn((12, 512), device="cuda").bfloat16()
+    gemv, gemm = quantized_linear(x, w, allow_gemm=False), quantized_linear(x, w)
+    assert not torch.equal(gemv, gemm)                          # (BF16 weights on the tensor cores)
+    for yes, no in ((1, 0), (np.True_, np.False_)):
+        assert torch.equal(quantized_linear(x, w, allow_gemm=yes), gemm) and torch.equal(quantized_linear(x, w, allow_gemm=no), gemv)
+    model, ids = small_llama(), torch.randint(0, 512, (12, 4), device="cuda")
+    step = lambda: model.prefill(ids, model.create_generation_state(12, 32))
+    before = step()
+    for table in ({"Q8_0": 13}, {}):
+        for module in ("quantized_linear", "llama_model"):
+            monkeypatch.setattr(sys.modules["mylocal_llm_b200." + module], "GEMM_MIN_TOKENS", table)
+        a, b = both(monkeypatch, lambda: quantized_linear(x, w))
+        assert torch.equal(a, gemv) and torch.equal(b, gemv)
+        a, b = both(monkeypatch, step)
+        assert torch.equal(a, b) and torch.equal(a, before) == bool(table)
 
 
 @pytest.mark.parametrize("t", [1, 5, 40])
