@@ -50,7 +50,9 @@ static void mbar_arrive_expect_tx(uint64_t *b, uint32_t) { mbar_arrive(b); }    
 static bool mbar_wait_bounded(uint64_t *b, uint32_t parity, int *status, int code) {
     std::unique_lock<std::mutex> l(mu);
     const bool refuse = threadIdx.x / 32 == fail_warp && waits++ == fail_at;
-    if (!refuse && cv.wait_for(l, std::chrono::milliseconds(gave_up ? 40 : 5000), [&] { return bar(b).phase != (int)parity; })) return true;
+    // (the first give-up is the planted one; from then on every wait has 40 ms, those that had begun included)
+    for (int slices = 0; !refuse && (!gave_up || slices < 2); slices += gave_up > 0)
+        if (cv.wait_for(l, std::chrono::milliseconds(20), [&] { return bar(b).phase != (int)parity; })) return true;
     ++gave_up;
     *status = code;
     return false;
@@ -62,7 +64,7 @@ static void named_barrier_sync(int id, int threads) {                           
     Meet &m = meets[id];
     const int round = m.round;
     if (++m.arrived == threads / 32) { m.arrived = 0; ++m.round; cv.notify_all(); return; }
-    if (!cv.wait_for(l, std::chrono::milliseconds(3000), [&] { return m.round != round; })) { hung = true; m.arrived = 0; ++m.round; cv.notify_all(); }
+    if (!cv.wait_for(l, std::chrono::seconds(10), [&] { return m.round != round; })) { hung = true; m.arrived = 0; ++m.round; cv.notify_all(); }
 }
 static std::mutex sync_mu;
 static void __syncthreads();
@@ -140,7 +142,7 @@ def walk(tmp_path_factory):
 
 
 def run(walk, kp, warp, at):
-    out = subprocess.run([str(walk), str(kp), str(warp), str(at)], capture_output=True, text=True, timeout=60, check=True).stdout
+    out = subprocess.run([str(walk), str(kp), str(warp), str(at)], capture_output=True, text=True, timeout=100, check=True).stdout
     return [int(v) for v in out.split()]
 
 
