@@ -50,12 +50,15 @@ void bind(const py::dict &addresses, py::object error_type) {
     b200q_error = error_type.release().ptr();
 }
 
-// Non-zero return codes become the exceptions _lib.call raises.
+// Non-zero return codes become the exceptions _lib.call raises. The launches run without the interpreter's lock, as they do
+// through ctypes (a launch into a full queue waits for the GPU): the code travels as a C++ exception.
+struct CallError {
+    int rc;
+    std::string text;
+    void raise() const { PyErr_SetString(rc == 1 ? PyExc_ValueError : rc == 3 ? PyExc_NotImplementedError : b200q_error, text.c_str()); }
+};
 void check(int rc, const char *name) {
-    if (rc == 0) return;
-    const std::string text = std::string(name) + ": " + api.last_error();
-    PyErr_SetString(rc == 1 ? PyExc_ValueError : rc == 3 ? PyExc_NotImplementedError : b200q_error, text.c_str());
-    throw py::error_already_set();
+    if (rc) throw CallError{rc, std::string(name) + ": " + api.last_error()};
 }
 #define CALL(name, ...) check(api.name(__VA_ARGS__), "b200q_" #name)
 
@@ -127,7 +130,13 @@ PyObject *linear_fast(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         const int64_t m = x.numel() / k;
         if (ydt < 0 || m == 0 || m > 0x7fffffff) Py_RETURN_NONE;
         at::Tensor y = nd == 2 ? empty({m, n}, out_type, x.device()) : empty({x.size(0), x.size(1), n}, out_type, x.device());
-        linear_into(x.data_ptr(), dt, static_cast<int>(m), w.data_ptr(), fmt, n, k, y.data_ptr(), ydt, gemm_min, x.device());
+        try {
+            py::gil_scoped_release unlocked;
+            linear_into(x.data_ptr(), dt, static_cast<int>(m), w.data_ptr(), fmt, n, k, y.data_ptr(), ydt, gemm_min, x.device());
+        } catch (const CallError &e) {
+            e.raise();
+            return nullptr;
+        }
         return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
 }
@@ -384,9 +393,12 @@ at::Tensor or_undefined(const py::object &o) { return o.is_none() ? at::Tensor()
 }  // namespace
 
 PYBIND11_MODULE(_b200q_host, m) {
+    using Unlocked = py::call_guard<py::gil_scoped_release>;
     py::register_local_exception_translator([](std::exception_ptr p) {
         try {
             if (p) std::rethrow_exception(p);
+        } catch (const CallError &e) {
+            e.raise();
         } catch (const c10::Error &) {
             torch::translate_exception_to_python(std::current_exception());
         }
@@ -410,14 +422,14 @@ PYBIND11_MODULE(_b200q_host, m) {
             l.floor = static_cast<float>(floor); l.row_plan = row_plan;
             return l;
         }))
-        .def("forward", &MoeLayer::forward);
+        .def("forward", &MoeLayer::forward, Unlocked());
     py::class_<MoeStack>(m, "MoeStack")
         .def(py::init([](std::vector<MoeLayer> layers, std::vector<at::Tensor> gammas, double eps) {
             MoeStack s;
             s.layers = std::move(layers); s.gammas = std::move(gammas); s.eps = static_cast<float>(eps);
             return s;
         }))
-        .def("forward", &MoeStack::forward);
+        .def("forward", &MoeStack::forward, Unlocked());
     py::class_<Llama>(m, "Llama")
         .def(py::init([](const py::dict &c) {
             auto matrix = [](const py::handle &h) {
@@ -443,8 +455,8 @@ PYBIND11_MODULE(_b200q_host, m) {
         }))
         .def("decode", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, at::Tensor position, const std::vector<int> &rule) {
             return m.decode(ids, k, v, position, gemm_rule(rule));
-        })
+        }, Unlocked())
         .def("prefill", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, const std::vector<int> &rule) {
             return m.prefill(ids, k, v, gemm_rule(rule));
-        });
+        }, Unlocked());
 }

@@ -283,3 +283,48 @@ def test_errors_are_those_of_the_python_layer(cuda):
         quantized_linear(np.zeros((1, 32), np.float32), w)
     with pytest.raises(TypeError, match="FP16, BF16, or FP32"):
         quantized_linear(torch.zeros((1, 32), dtype=torch.float64, device="cuda"), w)
+
+
+@pytest.mark.parametrize("what", ["linear", "layer", "stack", "prefill", "decode"])
+def test_other_threads_run_while_a_launch_waits(cuda, what):
+    """A launch into a full queue waits for the GPU; the interpreter's lock is free meanwhile, as it is in a ctypes call."""
+    torch = cuda
+    import threading
+    import time
+    if what == "linear":
+        w = packed_to_device(random_packed("Q8_0", (64, 256), seed=2, d=0.01))
+        x = torch.zeros((1, 256), device="cuda")
+        run, calls = lambda: quantized_linear(x, w), 3000
+    elif what in ("layer", "stack"):
+        stack = PackedMoEStack.synthetic(2, d_model=512, d_ff=256, n_experts=16, top_k=4, shared_d_ff=256, seed=5)
+        x = torch.randn((3, 1, 512), device="cuda")
+        run, calls = (lambda: stack.forward(x)) if what == "stack" else (lambda: stack.layers[0].forward(x)), 400
+    else:
+        model, ids = small_llama(), torch.zeros((2, 4), dtype=torch.int64, device="cuda")
+        state = model.create_generation_state(2, 64)
+        run, calls = (lambda: model.prefill(ids, state)) if what == "prefill" else (
+            lambda: (setattr(state, "length", 0), state.position.zero_(), model.decode_one(ids[:, 0].contiguous(), state))), 150
+    run()
+    torch.cuda.synchronize()
+    gaps, done = [0.0], threading.Event()
+
+    def watch():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=watch)
+    thread.start()
+    torch.cuda._sleep(1_500_000_000)                    # most of a second
+    t0 = time.perf_counter()
+    for _ in range(calls):
+        run()
+    waited = time.perf_counter() - t0
+    done.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert waited > 0.4, "the queue did not fill"
+    assert max(gaps) < 0.2, max(gaps)
