@@ -83,7 +83,13 @@ at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t, const at::Device &devi
 bool gguf_gemm_format(int fmt) { return fmt == B200Q_Q8_0 || fmt == B200Q_Q4_K || fmt == B200Q_Q5_K || fmt == B200Q_Q6_K; }
 
 // Tokens from which BF16 calls on GGUF-layout weights take the GEMM, by format (0: never): quantized_linear.GEMM_MIN_TOKENS
-// as it stands at the call.
+// as it stands at the call (None: no entry).
+int gemm_from(PyObject *tokens) {
+    if (tokens == Py_None) return 0;
+    int overflow = 0;
+    const long v = PyLong_AsLongAndOverflow(tokens, &overflow);
+    return overflow > 0 || v > 0x7fffffff ? 0x7fffffff : v < 1 ? 1 : static_cast<int>(v);
+}
 struct GemmRule {
     int q8_0 = 0, q4_k = 0, q5_k = 0, q6_k = 0;
     int of(int fmt) const {
@@ -110,13 +116,14 @@ void linear_into(const void *x, int x_dtype, int m, const void *w, int fmt, int 
 }
 
 // ------------------------------------------------------------------------------------------------ linear
-// linear(x, data, fmt, n, k, out_dtype | None, GEMM from this many tokens on or 0): the tensor, or None when the call needs the Python layer.
+// linear(x, data, fmt, n, k, out_dtype | None, GEMM from this many tokens on | None): the tensor, or None when the call needs the Python layer.
 PyObject *linear_fast(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (nargs != 7 || !THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) Py_RETURN_NONE;
     HANDLE_TH_ERRORS
         const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]);
         const int fmt = static_cast<int>(PyLong_AsLong(args[2])), n = static_cast<int>(PyLong_AsLong(args[3])),
-                  k = static_cast<int>(PyLong_AsLong(args[4])), gemm_min = static_cast<int>(PyLong_AsLong(args[6]));
+                  k = static_cast<int>(PyLong_AsLong(args[4])), gemm_min = gemm_from(args[6]);
+        if (PyErr_Occurred()) return nullptr;
         const int64_t nd = x.dim();
         const int dt = dtype_id(x.scalar_type());
         if (!x.is_cuda() || (nd != 2 && nd != 3) || x.size(nd - 1) != k || dt < 0 || !x.is_contiguous() || x.device() != w.device())
@@ -387,7 +394,9 @@ struct Llama {
     }
 };
 
-GemmRule gemm_rule(const std::vector<int> &v) { return {v.at(0), v.at(1), v.at(2), v.at(3)}; }
+GemmRule gemm_rule(const py::list &v) {
+    return {gemm_from(py::object(v[0]).ptr()), gemm_from(py::object(v[1]).ptr()), gemm_from(py::object(v[2]).ptr()), gemm_from(py::object(v[3]).ptr())};
+}
 at::Tensor or_undefined(const py::object &o) { return o.is_none() ? at::Tensor() : o.cast<at::Tensor>(); }
 
 }  // namespace
@@ -453,10 +462,14 @@ PYBIND11_MODULE(_b200q_host, m) {
             }
             return l;
         }))
-        .def("decode", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, at::Tensor position, const std::vector<int> &rule) {
-            return m.decode(ids, k, v, position, gemm_rule(rule));
-        }, Unlocked())
-        .def("prefill", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, const std::vector<int> &rule) {
-            return m.prefill(ids, k, v, gemm_rule(rule));
-        }, Unlocked());
+        .def("decode", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, at::Tensor position, const py::list &rule) {
+            const GemmRule from = gemm_rule(rule);
+            py::gil_scoped_release unlocked;
+            return m.decode(ids, k, v, position, from);
+        })
+        .def("prefill", [](const Llama &m, at::Tensor ids, at::Tensor k, at::Tensor v, const py::list &rule) {
+            const GemmRule from = gemm_rule(rule);
+            py::gil_scoped_release unlocked;
+            return m.prefill(ids, k, v, from);
+        });
 }

@@ -212,7 +212,7 @@ def quantized_linear(x, weight, *, block_k=512, cpu_packed_backend="reference", 
         host = _lib.host()
         if host is not None:
             y = host.linear(x, weight.data, weight._format_id, weight.shape[0], weight.shape[1], out_dtype,
-                            _gemm_from(weight.quant_type) if allow_gemm else 0)
+                            GEMM_MIN_TOKENS.get(weight.quant_type) if allow_gemm else None)
             if y is not None:
                 return y
     _check_activation(x)
@@ -268,14 +268,9 @@ GEMM_MIN_TOKENS = {"Q4_K": 9, "Q5_K": 9, "Q6_K": 9, "Q8_0": 9}
 SWIGLU_GEMM_MIN_TOKENS = 17
 
 
-def _gemm_from(fmt):
-    """The entry of ``GEMM_MIN_TOKENS`` as the native host path takes it (0: never)."""
-    tokens = GEMM_MIN_TOKENS.get(fmt)
-    return 0 if tokens is None else min(max(1, tokens), 0x7fffffff)
-
-
 def gemm_rule():
-    return [_gemm_from(fmt) for fmt in ("Q8_0", "Q4_K", "Q5_K", "Q6_K")]
+    """``GEMM_MIN_TOKENS`` as the native Llama path takes it."""
+    return [GEMM_MIN_TOKENS.get(fmt) for fmt in ("Q8_0", "Q4_K", "Q5_K", "Q6_K")]
 
 
 def _use_gemm(weight, x, m, n, k, dt):
