@@ -495,10 +495,17 @@ __device__ __forceinline__ void tiled_body(const Q6TiledArgs &a, const StagePoin
             cur = nxt;
             if (item + 1 < items_per_block) TILE::load(nxt, cur_p + (item + 1) * item_step, lane);
             else if (has_next) TILE::load(nxt, nxt_p, lane);
-            const uint2 *bf = bfrag + (kpi + item * a.kp) * 512 + lane * (TILE::PAIRED ? 2 : 1);
-            TILE::template mma<NTERMS, NT, TILE::PAIRED ? 8 : 256>(cur, [&](int nt, int pair, int plane) {
-                return reinterpret_cast<const uint8_t *>(bf + nt * tile_stride + plane * nfrag * 32 + pair * 64);
-            }, tot);
+            if constexpr (TILE::PAIRED) {
+                const uint4 *bf = reinterpret_cast<const uint4 *>(bfrag) + (kpi + item * a.kp) * 256 + lane;
+                TILE::template mma<NTERMS, NT, 8>(cur, [&](int nt, int pair, int plane) {
+                    return reinterpret_cast<const uint8_t *>(bf + nt * (tile_stride >> 1) + plane * nfrag * 16 + pair * 32);
+                }, tot);
+            } else {
+                const uint2 *bf = bfrag + (kpi + item * a.kp) * 512 + lane;
+                TILE::template mma<NTERMS, NT, 256>(cur, [&](int nt, int pair, int plane) {
+                    return reinterpret_cast<const uint8_t *>(bf + nt * tile_stride + plane * nfrag * 32 + pair * 64);
+                }, tot);
+            }
         }
 
         const int group = group0 + rgi;
