@@ -16,9 +16,10 @@
 // images, pairs of fragments, 16 bytes per lane) more than a multiple of 128 apart, so the tokens of one wavefront read
 // different banks.
 // The sums are those of the block-structured kernels with the same kp, bit for bit.
-// Bound by instruction issue (256 tokens, 512 experts: 0.63-0.68 of the slots, ALU pipe 0.54, DRAM 0.53 / 0.40): positions
-// in the run of row groups are kept by steps instead of divisions, and the copies are predicated, not branched around
-// (8-layer step of 64 tokens 1962 -> 1902 us, 16-token layer 133 -> 128).
+// Bound by instruction issue (256 tokens, 512 experts, gate/up and down: 0.67 of the slots, ALU pipe 0.61 / 0.58, DRAM 3.5 /
+// 3.3 TB/s; 428 and 679 instructions per 16 x 256 tile): positions in the run of row groups are kept by steps instead of
+// divisions, and the copies are predicated, not branched around (3 % of an 8-layer step of 64 tokens). Block-structured ->
+// streaming: 8-layer step of 64 tokens 2158 -> 2082 us, layer of 256 tokens 437 -> 378, of 16 tokens 143 -> 136.
 #pragma once
 
 #include "q6k_tiled.cuh"

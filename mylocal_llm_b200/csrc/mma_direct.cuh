@@ -15,7 +15,10 @@
 //   * the minima go through one more mma: A = the eight 6-bit mins, B = per-sub-block activation
 //     sums (FP16 high + remainder), giving sum(mn * sum_x);
 //   * y += d * acc - dmin * acc_min in FP32.
-// Every product is exact; roundings are the FP32 accumulations, as in the FP32-lane kernels.
+// Every product is exact; roundings are the FP32 accumulations, as in the FP32-lane kernels. (A masked nibble pair is an
+// FP16 subnormal as it stands and saves the permute and the FMA, but the tensor cores align products by the operands'
+// exponent fields: of a product with six leading zeros only what reaches 2^-19 of a step's largest is kept, 2^-25 of normal
+// ones. Against FP64 such Q4_K launches were up to 2.5 times further off.)
 //
 // Activations are prepared once per CTA (or per expert segment) exactly as in mma_gemv.cuh:
 // power-of-two scaling per token, FP16 high (+ remainder for FP32 inputs), stored as B fragments.
@@ -435,8 +438,8 @@ __device__ __forceinline__ void chunk_values(const RawChunk<NTERMS> &r, bool f16
 // The same preparation, the same bits, for many chunks per thread (dense launches of several tokens). What bounds it is
 // the latency of the reads - every CTA reads all of x from L2 - so BATCH chunks are requested before the first is looked
 // at, and the second pass starts with the batch that the first left in registers; above, the conversion behind every load
-// waits for it. Launches of 8 tokens: Q4_K [8192 x 2048] 11.7 -> 8.7 us, Q8_0 [2048 x 8192] 27.7 -> 14.6 us; 16 tokens,
-// Q8_0 [2048 x 2048] 14.6 -> 8.8 us. Up to MD_FEW_CHUNKS chunks per thread the short code above is the faster one: these copies of a chunk's
+// waits for it. Launches of 8 tokens: Q4_K [8192 x 2048] 12.7 -> 9.8 us, Q8_0 [2048 x 8192] 28.9 -> 15.1 us; 16
+// tokens, Q8_0 [2048 x 2048] 14.6 -> 8.8 us. Up to MD_FEW_CHUNKS chunks per thread the short code above is the faster one: these copies of a chunk's
 // code cost about 1 us of instruction fetch in a launch that uses one or two of them.
 // SUMS: this kernel's order, and the activation sums of the sub-blocks; else the natural order of q6k_tiled.cuh, PAIRED or
 // not.
