@@ -228,17 +228,26 @@ static bool plan_down(int fmt, int n, int k, int max_segments, GroupedArgs &a, s
 //     2048 x 1024: 45 segments 0.85; wider rows leave two tiles per warp and lose (64 of 1024 x 1536: 1.07-1.15).
 //   Q8_0 (tiles a third larger, less to decode) with one super-block per row 0.92-1.06, with two above 256 segments
 //     0.96-1.04: left to the block-structured kernel; 512 of 2048 x 512: 198 segments 0.83, 128 of 2048 x 768: 0.70-0.99.
+// B200Q_GROUPED_STREAM=1 / 0: wherever a plan fits / never (tests, A/B measurements), read at every call.
+static int stream_override() {
+    const char *v = std::getenv("B200Q_GROUPED_STREAM");
+    return v && (v[0] == '0' || v[0] == '1') ? v[0] - '0' : -1;
+}
 int grouped_gate_up_kp(int fmt, int n, int k, int x_dtype, int max_segments) {
     GroupedArgs a{};
     size_t smem = 0;
-    if (max_segments <= 112 || static_cast<long long>(max_segments) * (n / 16) * (k / 256) < 162LL * sm_count()) return 0;
+    const int forced = stream_override();
+    if (forced == 0) return 0;
+    if (forced < 0 && (max_segments <= 112 || static_cast<long long>(max_segments) * (n / 16) * (k / 256) < 162LL * sm_count())) return 0;
     return plan_gate_up(fmt, n, k, x_dtype, max_segments, a, smem) ? a.kp : 0;
 }
 int grouped_down_kp(int fmt, int n, int k, int max_segments) {
     GroupedArgs a{};
     size_t smem = 0;
-    if (max_segments <= 40 || k > 1024) return 0;
-    if (fmt == B200Q_Q8_0_TILED && (k < 512 || (k == 512 && max_segments > 256))) return 0;
+    const int forced = stream_override();
+    if (forced == 0) return 0;
+    if (forced < 0 && (max_segments <= 40 || k > 1024)) return 0;
+    if (forced < 0 && fmt == B200Q_Q8_0_TILED && (k < 512 || (k == 512 && max_segments > 256))) return 0;
     return plan_down(fmt, n, k, max_segments, a, smem) ? a.kp : 0;
 }
 

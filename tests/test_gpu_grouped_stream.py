@@ -29,6 +29,7 @@ def both(monkeypatch, run):
 @pytest.mark.parametrize("d,f", [(256, 16), (2048, 48), (768, 512), (2304, 256)])
 def test_same_bits_as_the_block_kernels(cuda, monkeypatch, tokens, e, k, d, f):
     torch = cuda
+    monkeypatch.setenv("B200Q_GROUPED_STREAM", "1")                     # also where the block-structured kernels are faster
     gen = torch.Generator(device="cuda")
     gen.manual_seed(tokens + d)
     scores = torch.rand((tokens, e), device="cuda", generator=gen)
@@ -73,3 +74,28 @@ def test_images_are_made_for_the_launches_that_read_them(cuda, tokens, e, k, d, 
     finally:
         _lib.call = real
     assert (calls.count("b200q_moe_token_images"), calls.count("b200q_moe_hidden_images")) == (gate_up, down)
+
+
+def test_infinities_and_nan_are_those_of_the_block_kernels(cuda, monkeypatch):
+    """Rows with an infinity, a NaN, only zeros or the type's largest magnitude, in the images and in what is computed."""
+    torch = cuda
+    tokens, e, k, d, f = 64, 96, 6, 2048, 512                           # 144 segments: both launches stream
+    ids = torch.rand((tokens, e), device="cuda").topk(k, dim=1).indices.contiguous()
+    plan = moe_ops.moe_plan(ids, e)
+    assert _lib.load().b200q_moe_gate_up_streams(_lib.FORMAT_ID["Q4_K_TILED"], f, d, 2, plan.max_segments)
+    assert _lib.load().b200q_moe_down_streams(_lib.FORMAT_ID["Q6_K_TILED"], d, f, plan.max_segments)
+
+    def odd(rows, width, dtype):
+        x = torch.randn((rows, width), device="cuda").to(dtype)
+        x[3, 5], x[9, 7], x[11], x[20, 1], x[33, 0] = float("inf"), float("nan"), 0, torch.finfo(dtype).max, -float("inf")
+        return x
+
+    (gate, stride), (up, _) = bank(torch, "Q4_K", e, f, d, 1), bank(torch, "Q4_K", e, f, d, 2)
+    x = odd(tokens, d, torch.bfloat16)
+    a, b = both(monkeypatch, lambda: moe_ops.moe_gate_up(x, plan, gate, up, "Q4_K_TILED", "Q4_K_TILED", f, d, stride, stride))
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num(), b.nan_to_num()) and torch.isnan(a).any()
+    down, stride = bank(torch, "Q6_K", e, d, f, 3)
+    hidden, route = odd(tokens * k, f, torch.float32), torch.rand((tokens, k), device="cuda")
+    a, b = both(monkeypatch, lambda: moe_ops.moe_down(hidden, route, plan, down, "Q6_K_TILED", d, f, stride))
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num(), b.nan_to_num()) and torch.isnan(a).any()
+    assert torch.isfinite(a[50:]).all()

@@ -61,3 +61,30 @@ def test_unsupported_forms_are_refused(cuda):
     for args in ((8, 3, 64, 100, 200, 2, 2), (8, 2, 128, 100, 200, 2, 2), (8, 2, 64, 100, 200, 1, 1), (8, 2, 64, 100, 99, 2, 2),
                  (8, 2, 64, 100, 1025, 2, 2)):
         assert _lib.load().b200q_prefill_attention_supported(*args) == 0
+
+
+@pytest.mark.parametrize("t,bad", [(70, 40), (300, 0), (600, 599)])
+def test_a_row_of_nan_reaches_the_rows_that_see_it(cuda, t, bad):
+    """... and the other sequence keeps its bits; so does every row block that ends before it."""
+    torch = cuda
+    batch, heads, dh = 2, 4, 64
+    angle = torch.arange(t, device="cuda")[:, None] * (10000.0 ** (-2.0 * torch.arange(dh // 2, device="cuda") / dh))
+    cos, sin = torch.cos(angle), torch.sin(angle)
+    qkv = torch.randn((batch * t, 3 * heads * dh), device="cuda")
+    ptr = lambda x: ctypes.c_void_p(x.data_ptr())
+
+    def run():
+        kc, vc = (torch.zeros((batch, heads, t, dh), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        out = torch.empty((batch, t, heads * dh), dtype=torch.bfloat16, device="cuda")
+        q, k, v = qkv.split(heads * dh, dim=1)
+        _lib.call("b200q_prefill_attention", ptr(q), ptr(k), ptr(v), qkv.stride(0), qkv.stride(0), qkv.stride(0), ptr(cos),
+                  ptr(sin), t, batch, t, heads, heads, dh, t, ptr(kc), ptr(vc), 2, float(dh ** -0.5), ptr(out), 2,
+                  _lib.current_stream())
+        return out
+
+    clean = run()
+    qkv[bad] = float("nan")
+    out = run()
+    assert torch.isnan(out[0, bad:]).all() and torch.equal(out[1], clean[1]) and torch.isfinite(clean).all()
+    before = bad // 64 * 64                              # (row blocks of 32 or 64)
+    assert torch.equal(out[0, :before], clean[0, :before])
