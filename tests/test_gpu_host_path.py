@@ -327,4 +327,4 @@ def test_other_threads_run_while_a_launch_waits(cuda, what):
     thread.join()
     torch.cuda.synchronize()
     assert waited > 0.4, "the queue did not fill"
-    assert max(gaps) < 0.2, max(gaps)
+    assert max(gaps) < waited / 2, (max(gaps), waited)          # (one call waits nearly all of it)
